@@ -9,8 +9,8 @@
 //    model's (half-)integer exponents taken as products and square roots instead of pow().  The
 //    age -> redshift / distance interpolations use per-interval slopes computed once per block
 //    (a multiply instead of a divide per lookup; results differ from the reference's divide by an ulp).
-//  * hgb_dbn_gw: differential binary number for Hard_GW (sam_cyutils.pyx:788-899); one thread per
-//    grid point.
+//  * hgb_dbn_gw: differential binary number for Hard_GW (sam_cyutils.pyx:788-899); one block per
+//    (mtot, mrat) cell.
 // FP64 throughout (the hardening integral and the lookback-time -> redshift inversion are the
 // FP64 islands of the path).  Built with -fmad=false so operation order and rounding follow the
 // reference loops; the remaining differences are the last-ulp behaviour of pow/log10.
@@ -592,43 +592,103 @@ __global__ void k_dbn_2pwl_eval_f32(CyConst cc, Dbn2plArgs a, const double *__re
 // differential binary number, Hard_GW
 // ------------------------------------------------------------------------------------------------
 
-__global__ void k_dbn_gw(CyConst cc, const double *__restrict__ fobs, int NF, const double *__restrict__ nden,
-                         const double *__restrict__ mtot, int nm, const double *__restrict__ mrat, int nq, int nz,
-                         const double *__restrict__ redz_prime, const double *__restrict__ zgrid,
-                         const double *__restrict__ dgrid, int NI, double *__restrict__ redz_final,
-                         double *__restrict__ diff_num) {
-    long row = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (row >= (long)nm * nq * nz) return;
-    int jj = (int)((row / nz) % nq);
-    int ii = (int)(row / ((long)nz * nq));
-    double *rf = redz_final + row * NF;
-    double *dn = diff_num + row * NF;
-    for (int f = 0; f < NF; f++) {
-        rf[f] = -1.0;
-        dn[f] = 0.0;
+// One block per (mtot, mrat) cell.  For GW-driven hardening the residence time is a product of powers,
+//   tres = (2/3) sepa / |da/dt| = (2/3) ksepa^4 mt^(4/3) (1 + mr)^2 / (|c_dadt| mt^3 mr) (f (1 + z))^(-8/3),
+// so an element is A(cell, z) B(f) with B = f^(-8/3) taken once per block and A once per grid point:
+// one FP64 product per element in place of two pow() and six divisions (on this GPU an FP64 warp
+// instruction holds its pipe for 64 cycles, so those set the time).  Targets are the block's fastest
+// index, so the two (M, Q, Z, F) outputs are written in contiguous runs; with one thread per grid
+// point walking its targets every store of a warp touched 32 lines.  61 x 47 x 53 points, 37 targets:
+// 5059 us with one thread per point, 121 us so (FP64 of the per-point terms).
+// The reference stops at the first target above the ISCO frequency, so target f is empty when any
+// f' <= f lies above it: the running maximum of the targets decides (products by 1 + z > 0 keep the
+// order).  B and the cell's constant carry 2^-80 and 2^80, which keeps A within a few decades of the
+// result.  f^(2/3) and mt^(1/3) are pow() of the rounded exponents, as in the reference: a cube root is
+// nearer to the real power but 4e-15 from the reference's value once it is raised to the fourth.
+constexpr int GW_ROWS = 256;    // redshifts staged at a time, one per thread
+constexpr int GW_FREQS = 512;   // targets staged at a time
+constexpr double GW_SCALE = 0x1.0p80, GW_SCALE_INV = 0x1.0p-80;
+
+__global__ void __launch_bounds__(GW_ROWS) k_dbn_gw(CyConst cc, const double *__restrict__ fobs, int NF,
+                                                    const double *__restrict__ nden, const double *__restrict__ mtot,
+                                                    const double *__restrict__ mrat, int nq, int nz,
+                                                    const double *__restrict__ redz_prime,
+                                                    const double *__restrict__ zgrid, const double *__restrict__ dgrid,
+                                                    int NI, double *__restrict__ redz_final,
+                                                    double *__restrict__ diff_num) {
+    __shared__ double fb[GW_FREQS], ftop[GW_FREQS];   // B and the running maximum of the targets
+    __shared__ double s_amp[GW_ROWS], s_z[GW_ROWS];
+    __shared__ int s_cut[GW_ROWS];                    // first empty target of the staged ones
+    __shared__ double s_k, s_isco;
+    const int t = threadIdx.x, cell = blockIdx.x;
+    if (t == 32) {
+        const double mt = mtot[cell / nq], mr = mrat[cell % nq];
+        const double ks2 = cc.ksepa * cc.ksepa, opq = 1.0 + mr;
+        const double m13 = pow(mt, 1.0 / 3.0), m23 = m13 * m13;
+        s_k = (2.0 / 3.0) * (ks2 * ks2) * (opq * opq) / (-cc.c_dadt * mr) * (m23 * m23 / mt / mt / mt) * GW_SCALE;
+        s_isco = cc.kfreq * sqrt(mt) / pow(3.0 * HGB_CY_SCHW * mt, 1.5);
     }
-    double rzp = redz_prime[row];
-    if (rzp <= 0.0) return;
-    double mt = mtot[ii], mr = mrat[jj];
-    double rad_isco = 3.0 * HGB_CY_SCHW * mt;
-    double frst_orb_isco = cc.kfreq * sqrt(mt) / pow(rad_isco, 1.5);
-    int zi = hgb::bracket_decreasing_from0(NI, rzp, zgrid);
-    if (zi > NI - 2) zi = NI - 2;
-    double dcom = hgb::interp_between(rzp, zgrid[zi], zgrid[zi + 1], dgrid[zi], dgrid[zi + 1]);
-    double nd = nden[row];
-    for (int f = 0; f < NF; f++) {
-        rf[f] = rzp;
-        double target_frst_orb = fobs[f] * (1.0 + rzp);
-        if (target_frst_orb > frst_orb_isco) {
-            for (int fp = f + 1; fp < NF; fp++) rf[fp] = rzp;
-            break;
+    double top = -INFINITY;   // (thread 0) largest target so far
+    for (int f0 = 0; f0 < NF; f0 += GW_FREQS) {
+        const int nfb = min(GW_FREQS, NF - f0);
+        __syncthreads();   // the previous targets are done with
+        for (int f = t; f < nfb; f += GW_ROWS) {
+            const double p = pow(fobs[f0 + f], 2.0 / 3.0), p2 = p * p;
+            fb[f] = GW_SCALE_INV / (p2 * p2);
         }
-        double sp = cc.ksepa * pow(mt, 1.0 / 3.0) / pow(target_frst_orb, 2.0 / 3.0);
-        double dadt = hgb::hard_gw(cc.c_dadt, mt, mr, sp);
-        double tres = -(2.0 / 3.0) * sp / dadt;
-        double dcm = dcom / HGB_CY_MPC;
-        double cosmo_fact = cc.fourpi * (1.0 + rzp) * (dcm * dcm);
-        dn[f] = nd * tres * cosmo_fact;
+        if (t == 0) {
+            for (int f = 0; f < nfb; f++) {
+                const double x = fobs[f0 + f];
+                top = x > top ? x : top;
+                ftop[f] = top;
+            }
+        }
+        __syncthreads();
+        const double kc = s_k, isco = s_isco;
+        for (int z0 = 0; z0 < nz; z0 += GW_ROWS) {
+            const int nzb = min(GW_ROWS, nz - z0);
+            const long row0 = (long)cell * nz + z0;
+            if (z0 > 0) __syncthreads();   // the previous rows are written
+            if (t < nzb) {
+                const double rzp = redz_prime[row0 + t];
+                double amp = 0.0;
+                int cut = 0;
+                if (!(rzp <= 0.0)) {
+                    int zi = hgb::bracket_decreasing_from0(NI, rzp, zgrid);
+                    if (zi > NI - 2) zi = NI - 2;
+                    const double dcom = hgb::interp_between(rzp, zgrid[zi], zgrid[zi + 1], dgrid[zi], dgrid[zi + 1]);
+                    const double dcm = dcom / HGB_CY_MPC, zp1 = 1.0 + rzp;
+                    const double cosmo_fact = cc.fourpi * zp1 * (dcm * dcm);
+                    // (1 + z)^(-8/3) = cbrt(1 + z) / (1 + z)^3
+                    amp = nden[row0 + t] * cosmo_fact * (kc * cbrt(zp1) / (zp1 * zp1 * zp1));
+                    int hi = nfb;   // first f with ftop[f] (1 + z) > isco
+                    while (cut < hi) {
+                        const int mid = (cut + hi) >> 1;
+                        if (ftop[mid] * zp1 > isco) hi = mid;
+                        else cut = mid + 1;
+                    }
+                }
+                s_amp[t] = amp;
+                s_z[t] = rzp <= 0.0 ? -1.0 : rzp;
+                s_cut[t] = cut;
+            }
+            __syncthreads();
+            double *rf = redz_final + row0 * NF + f0;
+            double *dn = diff_num + row0 * NF + f0;
+            const int dz = GW_ROWS / nfb, df = GW_ROWS - dz * nfb;
+            int z = t / nfb, f = t - z * nfb;
+            while (z < nzb) {
+                const long e = (long)z * NF + f;
+                rf[e] = s_z[z];
+                dn[e] = f < s_cut[z] ? s_amp[z] * fb[f] : 0.0;
+                z += dz;
+                f += df;
+                if (f >= nfb) {
+                    f -= nfb;
+                    z++;
+                }
+            }
+        }
     }
 }
 
@@ -932,10 +992,8 @@ int hgb_dbn_gw(const double *fobs_orb, int n_freq, const double *nden, const dou
     HGB_CHECK_ARG(fobs_orb && nden && mtot && mrat && redz_prime && cosmo && redz_final && diff_num);
     HGB_CHECK_ARG(n_freq > 0 && n_mtot > 0 && n_mrat > 0 && n_redz > 0);
     HGB_CHECK_ARG(cosmo->grid_size >= 2 && cosmo->grid_z && cosmo->grid_dcom);
-    long n = (long)n_mtot * n_mrat * n_redz;
-    int threads = 128;
-    k_dbn_gw<<<(unsigned)hgb::ceil_div(n, threads), threads, 0, (cudaStream_t)stream>>>(
-        hgb::cy_const(), fobs_orb, n_freq, nden, mtot, n_mtot, mrat, n_mrat, n_redz, redz_prime, cosmo->grid_z,
+    k_dbn_gw<<<(unsigned)((long)n_mtot * n_mrat), GW_ROWS, 0, (cudaStream_t)stream>>>(
+        hgb::cy_const(), fobs_orb, n_freq, nden, mtot, mrat, n_mrat, n_redz, redz_prime, cosmo->grid_z,
         cosmo->grid_dcom, cosmo->grid_size, redz_final, diff_num);
     return hgb::check_launch();
 }
