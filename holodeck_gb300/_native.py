@@ -67,12 +67,13 @@ class HgbSamModel(ctypes.Structure):
 
 
 class HgbScatterSizes(ctypes.Structure):
-    _fields_ = [("n_pts", _i), ("n_tri", _i), ("n_nbr", _i), ("n_grid", _i), ("n_levels", _i)]
+    _fields_ = [("n_pts", _i), ("n_tri", _i), ("n_nbr", _i), ("n_grid", _i), ("n_levels", _i),
+                ("n_phases", _i), ("phase_width", _i)]
 
 
 _SCATTER_ARRAYS = ["pts", "tri", "tri_kappa", "vtx_qinv", "nbr_ptr", "nbr_idx", "nbr_w", "level_ptr", "level_vtx",
                    "grid_tri", "grid_bary", "grid_near", "grid_axis", "weights", "back_idx", "back_t", "back_w",
-                   "lv_nbr_ptr", "lv_nbr", "lv_nbr_w", "lv_qinv"]
+                   "ph_ptr", "ph_info", "ph_nbr", "ph_m"]
 
 
 class HgbScatterHostPlan(ctypes.Structure):
@@ -82,7 +83,7 @@ class HgbScatterHostPlan(ctypes.Structure):
 class HgbScatterPlan(ctypes.Structure):
     _fields_ = ([("n_mtot", _i), ("n_mrat", _i), ("n_grid", _i), ("n_tri", _i), ("n_levels", _i)] +
                 [(name, _p) for name in _SCATTER_ARRAYS if name != "grid_axis"] +
-                [("grad_tol", _d), ("grad_maxiter", _i)])
+                [("grad_tol", _d), ("grad_maxiter", _i), ("n_phases", _i), ("phase_width", _i)])
 
 
 class HgbLoudestSample(ctypes.Structure):
@@ -90,6 +91,7 @@ class HgbLoudestSample(ctypes.Structure):
                 ("hc2ss", _p), ("hc2bg", _p), ("workspace", _p), ("workspace_bytes", _sz), ("d_status", _p)]
 
 
+SCATTER_DEG = 8          # HGB_SCATTER_DEG
 MLP_MAX_LAYERS = 8       # HGB_MLP_MAX_LAYERS
 MLP_SPLIT_ROWS = 128     # HGB_MLP_SPLIT_ROWS
 MLP_FUSED_MAX_BATCH = 16 # HGB_MLP_FUSED_MAX_BATCH
@@ -215,7 +217,7 @@ def check(rc, what):
 #: kernels each entry point launches (the radix argsort: a key gather, then a count, a scan and a
 #: scatter per 8 key bits); used to report the launch count of a timed region
 KERNELS_PER_CALL = {
-    "hgb_static_density": 1, "hgb_zero_stalled": 1, "hgb_add_scatter_to_masses": 5,
+    "hgb_static_density": 1, "hgb_zero_stalled": 1, "hgb_add_scatter_to_masses": 4,
     "hgb_find_2pwl_hardening_norm": 1, "hgb_sqrt_inplace": 1, "hgb_dbn_2pwl": 2, "hgb_dbn_2pwl_phase": 1, "hgb_dbn_2pwl_phase_f32": 1, "hgb_dbn_gw": 1,
     "hgb_integrate_3dx1d": 1, "hgb_char_strain_sq": 1, "hgb_number_and_strain": 1, "hgb_number_and_strain_f32": 1, "hgb_argsort_f0_desc": 25, "hgb_argsort_f0_desc_static": 25,
     "hgb_loudest_hc_from_sorted": 7, "hgb_loudest_hc_from_sorted_ex": 7, "hgb_sam_poisson_gwb": 3, "hgb_param_grids": 1, "hgb_model_details": 9,

@@ -3,18 +3,20 @@
 //   1. k_gradients: per-point gradients of the slice's density by the minimum-norm-network method
 //      (Nielson 1983; the gradient estimate behind scipy's CloughTocher2DInterpolator): Gauss-Seidel
 //      sweeps in point order, each point's 2x2 normal system solved with its precomputed inverse,
-//      until the largest relative change of a sweep falls below `grad_tol`.  One block per slice;
-//      the points of one wavefront level update concurrently and read exactly the neighbour values a
-//      sequential sweep would read, so the iterates equal the sequential ones.  k_gradients_lv keeps
-//      the slice in shared memory when it fits (grids up to ~9000 points).
+//      until the largest relative change of a sweep falls below `grad_tol`.  One block per slice.
+//      k_gradients_ph keeps several sweeps in flight on the plan's phases; k_gradients takes a plan
+//      without phases, one wavefront level at a time (a level's points update concurrently and read
+//      exactly the neighbour values that a sequential sweep would read).
 //   2. k_clough_tocher: the C1 piecewise-cubic Clough-Tocher interpolant (centroid split) at every
 //      node of the regular (log m1, log m2) grid; NaN outside the hull; NaN or negative values are
 //      replaced by the value of the nearest point.
 //   3. k_back_dot: the Gaussian redistribution W^T (W^T G) as the reference computes it (see
 //      hgb_add_scatter_to_masses) followed by the bilinear interpolation back to the points, fused
 //      into one dot product per (point, slice) with the plan's per-point row of (W W).
-// FP64 throughout; built with -fmad=false (k_gradients_lv fuses its multiply-adds explicitly).
+// FP64 throughout; built with -fmad=false (where multiply-adds are fused, explicitly).
 #include <math.h>
+
+#include <algorithm>
 
 #include "hgb_common.cuh"
 
@@ -78,183 +80,208 @@ __global__ void k_gradients(hgb_scatter_plan P, const double *__restrict__ dens,
     if (!converged && threadIdx.x == 0) hgb::flag(d_status, HGB_STATUS_GRADIENT_NOT_CONVERGED);
 }
 
-// The same solve with the slice's values and gradients in shared memory, indexed by level-order
-// position (a level's points are contiguous), for grids whose state fits on one SM.  GB300's FP64
-// units belong to the four SM sub-partitions and charge each warp instruction in full however few
-// lanes are active, so the block has four warps, one per sub-partition, and the per-level work is
-// spread so that no sub-partition carries much more than a quarter of it:
-//   * a level's points (about 20 at 91x81) share the lanes of every warp; warp w sums the terms of
-//     edges o, o+4, o+8, ... of its point with o = (w + 2) mod 4, so an interior point's six edges
-//     put two terms on warps 2 and 3 and one on warps 0 and 1;
-//   * warps 0 and 1 add the four partial sums and solve the x and the y component of the point's
-//     2x2 system respectively;
-//   * warp 2 evaluates the convergence test of the previous 32 points (their changes and magnitudes,
-//     double-buffered in shared memory) while warps 0 and 1 update the current ones.
-// The static data of the next level (each warp's first LV_REG edges of its point, the rows of the
-// inverse normal matrix that warps 0 and 1 use) is loaded into registers while the current level
-// computes.  Per point the terms and the test are those of k_gradients, with two differences of
-// rounding: the neighbour sum is grouped as four interleaved partial sums, and the multiply-adds are
-// fused (explicit __fma_rn, the file being built with -fmad=false).  An edge term
-//   c = 6 (f_j - f_i) - 2 (g_jx w0 + g_jy w1),  sx += c w2,  sy += c w3
-// takes 6 FP64 instructions instead of 11: the plan stores -2 w0 and -2 w1 (an exact scaling), so
-//   t = fma(g_jy, -2 w1, g_jx (-2 w0)),  c = fma(6, f_j - f_i, t),  sx = fma(c, w2, sx),  sy = fma(c, w3, sy),
-// and the 2x2 solve takes 2 instead of 3.  The FP64 pipe bounds this kernel, so the instruction
-// count is its time; each fused operation skips one rounding (an ulp of the term).
-constexpr int LV_WARPS = 4;
-constexpr int LV_REG = 3;   // edges o, o+4, o+8 per warp: interior points have 6 neighbours
+// The same solve with several sweeps in flight.  A sweep's levels are a chain (441 levels of about 17
+// points at 91 x 81), and one level at a time leaves the SM waiting: GB300's FP64 units charge a warp
+// instruction 64 cycles however few of its lanes are live, so a level of 17 points costs what 32 cost,
+// on one sub-partition.  A point of sweep k + 1 needs its higher-indexed neighbours' sweep k only, and
+// no neighbour lies more than D levels away, so sweep k + 1 may follow D + 1 = n_phases levels behind
+// sweep k (81 levels at 91 x 81, set by the hull's fan points: five to six sweeps in flight).  The plan
+// groups the points by level modulo n_phases; a pass over the phases advances every point by one
+// sweep, one barrier per phase, in place:
+//   * a lower-indexed neighbour (at most D levels before) has made the same sweep and not the next;
+//   * a higher-indexed one (at most D levels after) has made the previous sweep and not this one;
+//   * two neighbours never share a phase.
+// The values that a point reads, and so the iterates, are those of sweeps one after another.
+// Every update is also kept by sweep (`hist`, a ring of the sweeps in flight), since a sweep is known
+// to have converged only when its last level is done and the next sweeps have begun by then; the
+// converged sweep is taken from there.
+// The update itself is linear in the neighbours' gradients, g_i = c_i + sum_j M_ij g_j: c_i (the
+// slice's values, k_scatter_rhs) is taken once per solve and M_ij (geometry) comes with the plan, so a
+// neighbour costs 4 fused multiply-adds instead of 6 and the 2x2 solve is gone.  Rounding differs
+// from k_gradients by regrouping only.
+// Two lanes per point, one per component: 16 points per warp.  A point with more than HGB_SCATTER_DEG
+// neighbours (the hull's fans, up to 82) takes a warp: 16 lane pairs share its neighbours.  The static
+// entries of a warp's points in the next phase are loaded while the current phase computes.
+// FP64 bounds a phase: 90 points of about 6 neighbours are 6 warps of 13 to 15 FP64 instructions on
+// four sub-partitions, 1900 of its 2400 cycles.  91 x 81 points, 101 slices: 4283 us one level at a
+// time, 1896 us with sweeps in flight (and 69 us for c); 181 x 161, 201 slices, where the slice exceeds
+// shared memory and its gradients stay in L2: 78.5 and 18.1 ms.
+constexpr int PH_WARPS = 8;    // most warps of a block: two prefetched sets of entries need 200 registers
+constexpr int PH_RING = 16;    // sweeps whose test is open (at most HGB_SCATTER_STAGES + 1)
+constexpr int PH_DEG = HGB_SCATTER_DEG;
 
-__device__ __forceinline__ int lv_edge_offset(int warp) { return (warp + 2) & (LV_WARPS - 1); }
+// c_i = Q_i^-1 sum_j 6 (f_j - f_i) w23_ij, by position; also the slice's values, (Z, points)
+__global__ void __launch_bounds__(256) k_scatter_rhs(hgb_scatter_plan P, const double *__restrict__ dens, int nz,
+                                                     double *__restrict__ vals, double2 *__restrict__ cvec) {
+    const int n = P.n_mtot * P.n_mrat;
+    const int p = blockIdx.x * 8 + threadIdx.y, z = blockIdx.y * 32 + threadIdx.x;
+    if (p >= n || z >= nz) return;
+    const int i = P.ph_info[4 * p];
+    const double fi = dens[(long)i * nz + z];
+    double sx = 0.0, sy = 0.0;
+    for (int e = P.nbr_ptr[i]; e < P.nbr_ptr[i + 1]; e++) {
+        const double c = 6.0 * (dens[(long)P.nbr_idx[e] * nz + z] - fi);
+        sx = __fma_rn(c, P.nbr_w[4 * e + 2], sx);
+        sy = __fma_rn(c, P.nbr_w[4 * e + 3], sy);
+    }
+    const double *q = P.vtx_qinv + 4 * i;
+    vals[(long)z * n + i] = fi;
+    cvec[(long)z * n + p] = make_double2(__fma_rn(q[1], sy, q[0] * sx), __fma_rn(q[3], sy, q[2] * sx));
+}
 
-struct LvPre {
-    int e0, e1;
-    int idx[LV_REG];
-    double2 w01[LV_REG], w23[LV_REG];
-    double2 q;   // warps 0 / 1: row 0 / 1 of the point's inverse normal matrix
+struct PhPre {   // a lane's point (16 per warp, two lanes each) and its row of M
+    int4 info;   // point, stage, neighbours (-1: no point), first entry
+    int nbr[PH_DEG];
+    double2 m[PH_DEG];
+    double c;
 };
 
-__device__ __forceinline__ void lv_load(const hgb_scatter_plan &P, const int *eptr, int p, bool active, int warp,
-                                        LvPre &x) {
-    x.e0 = active ? eptr[p] : 0;
-    x.e1 = active ? eptr[p + 1] : 0;
-#pragma unroll
-    for (int k = 0; k < LV_REG; k++) {
-        const int e = x.e0 + lv_edge_offset(warp) + LV_WARPS * k;
-        if (e < x.e1) {
-            x.idx[k] = __ldg(P.lv_nbr + e);
-            x.w01[k] = __ldg((const double2 *)(P.lv_nbr_w + 4 * (long)e));
-            x.w23[k] = __ldg((const double2 *)(P.lv_nbr_w + 4 * (long)e + 2));
-        }
-    }
-    if (active && warp < 2) x.q = __ldg((const double2 *)(P.lv_qinv + 4 * (long)p + 2 * warp));   // row `warp`
+// lane's point of chunk `base` of a phase (points with few neighbours): what ph_entries needs
+__device__ __forceinline__ int4 ph_point(const hgb_scatter_plan &P, const int4 ph, int base, int lane) {
+    const int q = base + (lane >> 1);
+    return q < ph.z ? __ldg((const int4 *)P.ph_info + ph.x + q) : make_int4(0, 0, -1, 0);
 }
 
-__global__ void __launch_bounds__(32 * LV_WARPS, 1) k_gradients_lv(hgb_scatter_plan P, const double *__restrict__ dens,
-                                                                  int nz, double *__restrict__ vals,
-                                                                  double *__restrict__ grads, int *d_status) {
-    extern __shared__ double sm[];
-    __shared__ double psx[LV_WARPS][32], psy[LV_WARPS][32];
-    __shared__ double chg[2][2][32], mag[2][2][32];   // [chunk parity][component][lane]: |change|, |new value|
-    __shared__ int s_over;
-    const int z = blockIdx.x, t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int n = P.n_mtot * P.n_mrat;
-    double *f = sm;                                  // [n]
-    double *g = f + n;                               // [n][2]
-    int *eptr = (int *)(g + 2 * n);                  // [n + 1]
-    int *lptr = eptr + n + 1;                        // [n_levels + 1]
-    for (int p = t; p < n; p += blockDim.x) {
-        const int i = P.level_vtx[p];
-        const double v = dens[(long)i * nz + z];
-        f[p] = v;
-        vals[(long)z * n + i] = v;
-        g[2 * p] = 0.0;
-        g[2 * p + 1] = 0.0;
-        eptr[p] = P.lv_nbr_ptr[p];
-    }
-    if (t == 0) eptr[n] = P.lv_nbr_ptr[n];
-    for (int l = t; l <= P.n_levels; l += blockDim.x) lptr[l] = P.level_ptr[l];
-    __syncthreads();
-    const int nlev = P.n_levels;
-    const double tol_lo = P.grad_tol * (1.0 - 1e-12);   // below this multiple of the scale: surely < tol
-    bool converged = false;
-    LvPre nxt;
-    lv_load(P, eptr, lptr[0] + lane, lane < lptr[1] - lptr[0], warp, nxt);
-    // exact test of one chunk's points from the buffered changes and magnitudes (warp 2)
-    auto test_chunk = [&](int b, bool over) {
-        const double change = fmax(chg[b][0][lane], chg[b][1][lane]);
-        const double scale = fmax(1.0, fmax(mag[b][0][lane], mag[b][1][lane]));
-        // relative change, divided out only where the comparison with the tolerance is close (the
-        // decision is that of change / scale < tol)
-        if (change >= tol_lo * scale) over = over || (change / scale >= P.grad_tol);
-        return over;
-    };
-    for (int it = 0; it < P.grad_maxiter; it++) {
-        bool over = false;   // (warp 2) some point changed by >= grad_tol (relative) in this sweep
-        int kc = 0;          // chunks updated so far in this sweep
-        for (int lev = 0; lev < nlev; lev++) {
-            const int p0 = lptr[lev], p1 = lptr[lev + 1];
-            const LvPre cur = nxt;
-            {   // the next level (the first level again after the last), loaded ahead
-                const int nl = (lev + 1 < nlev) ? lev + 1 : 0;
-                const int q0 = lptr[nl], q1 = lptr[nl + 1];
-                lv_load(P, eptr, q0 + lane, lane < q1 - q0, warp, nxt);
-            }
-            for (int c0 = p0; c0 < p1; c0 += 32) {   // 32 points at a time (one pass at 91x81)
-                const int p = c0 + lane;
-                const bool act = p < p1;
-                const bool pre = (c0 == p0);         // the prefetched chunk; wider levels load directly
-                double sx = 0.0, sy = 0.0;
-                if (act) {
-                    const double fi = f[p];
-                    const int e0 = pre ? cur.e0 : eptr[p], e1 = pre ? cur.e1 : eptr[p + 1];
-                    int e = e0 + lv_edge_offset(warp);
-                    if (pre) {
+__device__ __forceinline__ void ph_entries(const hgb_scatter_plan &P, const int4 ph, int base, int lane,
+                                           const double *cz, PhPre &x) {
+    if (x.info.z < 0) return;
+    x.c = __ldg(cz + 2 * (ph.x + base + (lane >> 1)) + (lane & 1));
 #pragma unroll
-                        for (int k = 0; k < LV_REG; k++) {
-                            if (e < e1) {
-                                const int j = cur.idx[k];
-                                const double tt = __fma_rn(g[2 * j + 1], cur.w01[k].y, g[2 * j] * cur.w01[k].x);
-                                const double cc = __fma_rn(6.0, f[j] - fi, tt);
-                                sx = __fma_rn(cc, cur.w23[k].x, sx);
-                                sy = __fma_rn(cc, cur.w23[k].y, sy);
-                            }
-                            e += LV_WARPS;
+    for (int e = 0; e < PH_DEG; e++) {
+        if (e < x.info.z) {
+            const long k = x.info.w + (long)e * ph.z;
+            x.nbr[e] = __ldg(P.ph_nbr + k);
+            x.m[e] = __ldg((const double2 *)(P.ph_m + 4 * k + 2 * (lane & 1)));
+        }
+    }
+}
+
+// whether a point's change (the pair of lanes hold its components) reaches tol relative to
+// max(1, |new value|).  Decided in FP32 unless within 1e-5 of the tolerance or out of FP32's range.
+__device__ __forceinline__ bool ph_over(double d, double v, double tol, float tolf) {
+    float cd = fabsf(hgb::f64_to_f32_rz(d)), sc = fabsf(hgb::f64_to_f32_rz(v));
+    cd = fmaxf(cd, __shfl_xor_sync(0xffffffffu, cd, 1));
+    sc = fmaxf(1.0f, fmaxf(sc, __shfl_xor_sync(0xffffffffu, sc, 1)));
+    const bool under = cd < tolf * 0.99999f * sc;
+    bool over = cd >= tolf * 1.00001f * sc && cd < 1e38f && sc < 1e38f;
+    if (__any_sync(0xffffffffu, !under && !over)) {
+        const double dd = __shfl_xor_sync(0xffffffffu, d, 1), vv = __shfl_xor_sync(0xffffffffu, v, 1);
+        if (!under && !over) {
+            const double change = fmax(fabs(d), fabs(dd));
+            over = change / fmax(1.0, fmax(fabs(v), fabs(vv))) >= tol;
+        }
+    }
+    return over;
+}
+
+template <bool SMEM>
+__global__ void __launch_bounds__(32 * PH_WARPS, 1) k_gradients_ph(hgb_scatter_plan P, int nz,
+                                                                  const double *__restrict__ cvec,
+                                                                  double *__restrict__ hist, double *grads,
+                                                                  int *d_status) {
+    extern __shared__ double2 sm2[];
+    __shared__ int s_over[PH_RING];
+    const int z = blockIdx.x, t = threadIdx.x, lane = t & 31, warp = t >> 5, nw = blockDim.x >> 5;
+    const int n = P.n_mtot * P.n_mrat;
+    const int nph = P.n_phases, last_phase = (P.n_levels - 1) % nph, last_stage = (P.n_levels - 1) / nph;
+    const int nring = last_stage + 1;   // a sweep's ring entry is rewritten once its last level is done
+    int4 *ptr = (int4 *)sm2;            // [nph] the phases
+    // gradients by position, advanced in place: in shared memory, or in this slice's part of `grads`
+    // (read and written by this block only, a barrier apart; rewritten by point at the end)
+    double *g = SMEM ? (double *)(sm2 + nph) : grads + 2L * z * n;
+    const double *cz = cvec + 2L * z * n;
+    const float tolf = (float)P.grad_tol;
+    for (int f = t; f < nph; f += blockDim.x) ptr[f] = __ldg((const int4 *)P.ph_ptr + f);
+    for (int p = t; p < n; p += blockDim.x) ((double2 *)g)[p] = make_double2(0.0, 0.0);
+    if (t < PH_RING) s_over[t] = 0;
+    __syncthreads();
+    // prefetch: a warp's points two phases ahead, their entries one phase ahead
+    const int base0 = 16 * warp;
+    PhPre nxt;
+    nxt.info = ph_point(P, ptr[0], base0, lane);
+    ph_entries(P, ptr[0], base0, lane, cz, nxt);
+    int f1 = nph > 1 ? 1 : 0;   // the next phase
+    int4 info1 = ph_point(P, ptr[f1], base0, lane);
+    bool converged = false;
+    int k_end = -1;
+    for (int T = 0; k_end < 0; T++) {
+        if (t == 0) s_over[(T + 1) & (PH_RING - 1)] = 0;   // sweep T + 1 starts after this pass
+        for (int phase = 0; phase < nph; phase++) {
+            const PhPre cur = nxt;
+            const int4 now = ptr[phase];
+            nxt.info = info1;
+            ph_entries(P, ptr[f1], base0, lane, cz, nxt);
+            f1 = f1 + 1 < nph ? f1 + 1 : 0;
+            info1 = ph_point(P, ptr[f1], base0, lane);
+            for (int base = base0; base < now.z; base += 16 * nw) {
+                PhPre x;
+                if (base == base0) {
+                    x = cur;
+                } else {
+                    x.info = ph_point(P, now, base, lane);
+                    ph_entries(P, now, base, lane, cz, x);
+                }
+                const int k = T - x.info.y;
+                const bool live = x.info.z >= 0 && k >= 0 && k < P.grad_maxiter;
+                double v = 0.0, d = 0.0;
+                if (live) {
+                    v = x.c;
+#pragma unroll
+                    for (int e = 0; e < PH_DEG; e++) {
+                        if (e < x.info.z) {
+                            const double2 gj = ((const double2 *)g)[x.nbr[e]];
+                            v = __fma_rn(x.m[e].x, gj.x, v);
+                            v = __fma_rn(x.m[e].y, gj.y, v);
                         }
                     }
-                    for (; e < e1; e += LV_WARPS) {
-                        const int j = __ldg(P.lv_nbr + e);
-                        const double2 w01 = __ldg((const double2 *)(P.lv_nbr_w + 4 * (long)e));
-                        const double2 w23 = __ldg((const double2 *)(P.lv_nbr_w + 4 * (long)e + 2));
-                        const double tt = __fma_rn(g[2 * j + 1], w01.y, g[2 * j] * w01.x);
-                        const double cc = __fma_rn(6.0, f[j] - fi, tt);
-                        sx = __fma_rn(cc, w23.x, sx);
-                        sy = __fma_rn(cc, w23.y, sy);
-                    }
+                    const int o = 2 * (now.x + base + (lane >> 1)) + (lane & 1);
+                    d = v - g[o];
+                    g[o] = v;
+                    hist[2L * n * ((long)z * nring + k % nring) + o] = v;
                 }
-                psx[warp][lane] = sx;
-                psy[warp][lane] = sy;
-                __syncthreads();
-                const int b = kc & 1;
-                if (warp < 2) {   // warp 0 solves the x component, warp 1 the y component
-                    double dv = 0.0, av = 0.0;
-                    if (act) {
-                        const double tx = ((psx[0][lane] + psx[1][lane]) + psx[2][lane]) + psx[3][lane];
-                        const double ty = ((psy[0][lane] + psy[1][lane]) + psy[2][lane]) + psy[3][lane];
-                        const double2 q = pre ? cur.q : __ldg((const double2 *)(P.lv_qinv + 4 * (long)p + 2 * warp));
-                        const double nv = __fma_rn(q.y, ty, q.x * tx);
-                        dv = fabs(nv - g[2 * p + warp]);
-                        av = fabs(nv);
-                        g[2 * p + warp] = nv;
-                    }
-                    chg[b][warp][lane] = dv;
-                    mag[b][warp][lane] = av;
-                } else if (warp == 2 && kc > 0) {
-                    over = test_chunk(b ^ 1, over);   // the previous chunk, while this one updates
+                if (ph_over(d, v, P.grad_tol, tolf)) s_over[k & (PH_RING - 1)] = 1;
+            }
+            // points with many neighbours, one warp each, from the last warp down
+            for (int q = now.z + (nw - 1 - warp); q < now.y; q += nw) {
+                const int p = now.x + q;
+                const int4 info = __ldg((const int4 *)P.ph_info + p);
+                const int k = T - info.y;
+                if (k < 0 || k >= P.grad_maxiter) continue;
+                double v = lane < 2 ? cz[2 * p + lane] : 0.0, d = 0.0;
+                for (int e = lane >> 1; e < info.z; e += 16) {
+                    const long kk = info.w + e;
+                    const double2 m = __ldg((const double2 *)(P.ph_m + 4 * kk + 2 * (lane & 1)));
+                    const double2 gj = ((const double2 *)g)[__ldg(P.ph_nbr + kk)];
+                    v = __fma_rn(m.x, gj.x, v);
+                    v = __fma_rn(m.y, gj.y, v);
                 }
-                __syncthreads();
-                kc++;
+#pragma unroll
+                for (int o = 16; o > 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                if (lane < 2) {
+                    d = v - g[2 * p + lane];
+                    g[2 * p + lane] = v;
+                    hist[2L * n * ((long)z * nring + k % nring) + 2 * p + lane] = v;
+                }
+                if (ph_over(d, v, P.grad_tol, tolf) && lane < 2) s_over[k & (PH_RING - 1)] = 1;
+            }
+            __syncthreads();
+            if (phase == last_phase && T >= last_stage) {   // sweep T - last_stage is complete
+                const int k = T - last_stage;
+                converged = s_over[k & (PH_RING - 1)] == 0;
+                if (converged || k + 1 >= P.grad_maxiter) {
+                    k_end = k;
+                    break;
+                }
             }
         }
-        if (warp == 2) {
-            if (kc > 0) over = test_chunk((kc - 1) & 1, over);   // the sweep's last chunk
-            const bool any = __any_sync(0xffffffffu, over);
-            if (lane == 0) s_over = any ? 1 : 0;
-        }
-        __syncthreads();
-        converged = (s_over == 0);
-        __syncthreads();
-        if (converged) break;
     }
     if (!converged && t == 0) hgb::flag(d_status, HGB_STATUS_GRADIENT_NOT_CONVERGED);
-    for (int p = t; p < n; p += blockDim.x) {
-        const int i = P.level_vtx[p];
-        grads[2L * z * n + 2 * i] = g[2 * p];
-        grads[2L * z * n + 2 * i + 1] = g[2 * p + 1];
-    }
+    const double2 *h = (const double2 *)(hist + 2L * n * ((long)z * nring + k_end % nring));
+    for (int p = t; p < n; p += blockDim.x) ((double2 *)(grads + 2L * z * n))[P.ph_info[4 * p]] = h[p];
 }
 
-size_t gradients_lv_smem(const hgb_scatter_plan &P) {
-    const size_t n = (size_t)P.n_mtot * P.n_mrat;
-    return sizeof(double) * 3 * n + sizeof(int) * (n + 1) + sizeof(int) * (P.n_levels + 1);
+size_t gradients_smem(const hgb_scatter_plan &P, bool grads) {
+    return sizeof(double2) * ((size_t)P.n_phases + (grads ? (size_t)P.n_mtot * P.n_mrat : 0));
 }
 
 // ---- 2. Clough-Tocher value at barycentric (l0, l1, l2) of triangle r
@@ -358,8 +385,9 @@ extern "C" {
 size_t hgb_scatter_workspace_bytes(int n_mtot, int n_mrat, int n_redz, int n_grid) {
     if (n_mtot < 2 || n_mrat < 2 || n_redz < 1 || n_grid < 2) return 0;
     size_t n = (size_t)n_mtot * n_mrat, NN = (size_t)n_grid * n_grid;
-    return align256(sizeof(double) * n * n_redz) + align256(sizeof(double) * 2 * n * n_redz) +
-           align256(sizeof(double) * NN * n_redz);
+    const size_t last = std::max(NN, 2 * HGB_SCATTER_STAGES * n);   // the regular grid; the sweeps in flight
+    return align256(sizeof(double) * n * n_redz) + 2 * align256(sizeof(double) * 2 * n * n_redz) +
+           align256(sizeof(double) * last * n_redz);
 }
 
 int hgb_add_scatter_to_masses(const hgb_scatter_plan *plan, double *dens, int n_redz, void *workspace,
@@ -378,22 +406,36 @@ int hgb_add_scatter_to_masses(const hgb_scatter_plan *plan, double *dens, int n_
     w += align256(sizeof(double) * n * n_redz);
     double *grads = (double *)w;
     w += align256(sizeof(double) * 2 * n * n_redz);
+    double *cvec = (double *)w;
+    w += align256(sizeof(double) * 2 * n * n_redz);
     double *gridA = (double *)w;
+    double *hist = gridA;   // the sweeps in flight are done with before the grid is written
     cudaStream_t st = (cudaStream_t)stream;
 
-    const size_t lv_smem = gradients_lv_smem(P);
-    int dev = 0, smem_optin = 0;
+    int rc, dev = 0, smem_optin = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    if (P.lv_nbr_ptr && P.lv_nbr && P.lv_nbr_w && P.lv_qinv && lv_smem + 8192 <= (size_t)smem_optin) {
-        const int rc = hgb::ensure_dyn_smem((const void *)k_gradients_lv, lv_smem);
-        if (rc) return rc;
-        k_gradients_lv<<<n_redz, 32 * LV_WARPS, lv_smem, st>>>(P, dens, n_redz, vals, grads, d_status);
+    // the phases where the plan has them and their table fits one SM; the gradients beside it where
+    // they fit too (grids up to about 14000 points)
+    if (P.ph_ptr && P.ph_info && P.ph_nbr && P.ph_m && P.n_phases >= 1 && P.phase_width >= 1 &&
+        gradients_smem(P, false) + 1024 <= (size_t)smem_optin) {
+        HGB_CHECK_ARG((P.n_levels - 1) / P.n_phases < HGB_SCATTER_STAGES);
+        k_scatter_rhs<<<dim3((unsigned)hgb::ceil_div((long)n, 8), (unsigned)hgb::ceil_div(n_redz, 32)), dim3(32, 8), 0,
+                        st>>>(P, dens, n_redz, vals, (double2 *)cvec);
+        if ((rc = hgb::check_launch())) return rc;
+        // a warp per 16 points of the widest phase and one for a fan point, whole sub-partitions
+        int nw = (int)hgb::ceil_div(P.phase_width, 16) + 1;
+        nw = std::min(PH_WARPS, (nw + 3) / 4 * 4);
+        const bool in_smem = gradients_smem(P, true) + 1024 <= (size_t)smem_optin;
+        const size_t smem = gradients_smem(P, in_smem);
+        const void *fn = in_smem ? (const void *)k_gradients_ph<true> : (const void *)k_gradients_ph<false>;
+        if ((rc = hgb::ensure_dyn_smem(fn, smem))) return rc;
+        if (in_smem) k_gradients_ph<true><<<n_redz, 32 * nw, smem, st>>>(P, n_redz, cvec, hist, grads, d_status);
+        else k_gradients_ph<false><<<n_redz, 32 * nw, smem, st>>>(P, n_redz, cvec, hist, grads, d_status);
     } else {
         k_gradients<<<n_redz, 256, 0, st>>>(P, dens, n_redz, vals, grads, d_status);
     }
-    int rc = hgb::check_launch();
-    if (rc) return rc;
+    if ((rc = hgb::check_launch())) return rc;
     dim3 gct((unsigned)hgb::ceil_div((long)NN, 256), (unsigned)n_redz);
     k_clough_tocher<<<gct, 256, 0, st>>>(P, vals, grads, gridA);
     if ((rc = hgb::check_launch())) return rc;

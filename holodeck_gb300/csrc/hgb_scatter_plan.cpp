@@ -15,7 +15,7 @@
 //     2x2 normal matrix of the minimum-norm-network gradient update (Nielson 1983), and the
 //     Gauss-Seidel wavefront levels: level(i) = 1 + max level of the lower-indexed neighbours, so
 //     one level's points update concurrently while reading exactly the values a sequential sweep in
-//     point order would read;
+//     point order would read, and the phases in which several sweeps run at once;
 //   * per node of the regular (log m1, log m2) grid: containing triangle and barycentric
 //     coordinates (or -1 outside the hull) and the nearest point (greedy descent on the Delaunay
 //     graph, exact for any query point);
@@ -275,6 +275,8 @@ int hgb_scatter_plan_bounds(int n_mtot, int n_mrat, int refine, hgb_scatter_size
     out->n_nbr = 6 * n;
     out->n_grid = refine * n_mtot;
     out->n_levels = n;
+    out->n_phases = n;
+    out->phase_width = n;
     return HGB_OK;
 }
 
@@ -424,21 +426,70 @@ int hgb_scatter_plan_build(const double *mtot, int n_mtot, const double *mrat, i
         for (int l = 0; l <= nlev; l++) plan->level_ptr[l] = count[l];
         std::vector<int> fill(count.begin(), count.end() - 1);
         for (int i = 0; i < n; i++) plan->level_vtx[fill[level[i]]++] = i;
-        // level-order copies: a level's points are contiguous, neighbours keep their order
-        std::vector<int> pos_of(n);
-        for (int p = 0; p < n; p++) pos_of[plan->level_vtx[p]] = p;
-        int e = 0;
-        for (int p = 0; p < n; p++) {
-            const int i = plan->level_vtx[p];
-            plan->lv_nbr_ptr[p] = e;
-            for (int q = plan->nbr_ptr[i]; q < plan->nbr_ptr[i + 1]; q++, e++) {
-                plan->lv_nbr[e] = pos_of[plan->nbr_idx[q]];
-                // -2 w0, -2 w1, w2, w3: the level-order solve folds the factor -2 into its weights
-                for (int c = 0; c < 4; c++) plan->lv_nbr_w[4 * e + c] = (c < 2 ? -2.0 : 1.0) * plan->nbr_w[4 * q + c];
-            }
-            for (int c = 0; c < 4; c++) plan->lv_qinv[4 * p + c] = plan->vtx_qinv[4 * i + c];
+    }
+    // phases of the pipelined sweeps: more of them than any two neighbours' levels are apart, and
+    // enough that at most HGB_SCATTER_STAGES sweeps are in flight
+    int nph = (nlev + HGB_SCATTER_STAGES - 1) / HGB_SCATTER_STAGES, width = 0;
+    for (int i = 0; i < n; i++)
+        for (int j : nb[i]) nph = std::max(nph, level[i] - level[j] + 1);
+    {
+        std::vector<int> few(nph, 0), many(nph, 0), pos_of(n);
+        auto is_few = [&](int i) { return (int)nb[i].size() <= HGB_SCATTER_DEG; };
+        for (int i = 0; i < n; i++) (is_few(i) ? few : many)[level[i] % nph]++;
+        std::vector<int> fill_few(nph), fill_many(nph), first(nph);
+        int pos = 0, entry = 0;
+        for (int f = 0; f < nph; f++) {
+            int32_t *pp = plan->ph_ptr + 4 * f;
+            pp[0] = pos;
+            pp[1] = few[f] + many[f];
+            pp[2] = few[f];
+            pp[3] = 0;
+            fill_few[f] = pos;
+            fill_many[f] = pos + few[f];
+            first[f] = entry;
+            pos += pp[1];
+            entry += HGB_SCATTER_DEG * few[f];
+            width = std::max(width, pp[1]);
         }
-        plan->lv_nbr_ptr[n] = e;
+        // within a phase the points with most neighbours first: a warp's 16 points then have nearly the
+        // same number, and it runs as long as its longest
+        std::vector<int> by_deg(plan->level_vtx, plan->level_vtx + n);
+        std::stable_sort(by_deg.begin(), by_deg.end(),
+                         [&](int x, int y) { return nb[x].size() > nb[y].size(); });
+        for (int i : by_deg) {
+            const int f = level[i] % nph;
+            const int p = is_few(i) ? fill_few[f]++ : fill_many[f]++;
+            pos_of[i] = p;
+            int32_t *info = plan->ph_info + 4 * p;
+            info[0] = i;
+            info[1] = level[i] / nph;
+            info[2] = (int)nb[i].size();
+            if (is_few(i)) {
+                info[3] = first[f] + (p - plan->ph_ptr[4 * f]);
+            } else {
+                info[3] = entry;
+                entry += (int)nb[i].size();
+            }
+        }
+        for (int k = 0; k < entry; k++) plan->ph_nbr[k] = 0;
+        for (int p = 0; p < n; p++) {
+            const int32_t *info = plan->ph_info + 4 * p;
+            const int i = info[0], f = level[i] % nph;
+            const int stride = is_few(i) ? few[f] : 1;
+            const double *q = plan->vtx_qinv + 4 * i;
+            for (int e = 0; e < info[2]; e++) {
+                const long k = info[3] + (long)e * stride;
+                const int src = plan->nbr_ptr[i] + e;
+                const double *w = plan->nbr_w + 4 * src;
+                // g_i = Q^-1 sum_j (6 (f_j - f_i) - 2 (g_j . w01)) w23: M_ij = -2 (Q^-1 w23) w01^T
+                const double ux = -2.0 * (q[0] * w[2] + q[1] * w[3]), uy = -2.0 * (q[2] * w[2] + q[3] * w[3]);
+                plan->ph_nbr[k] = pos_of[plan->nbr_idx[src]];
+                plan->ph_m[4 * k + 0] = ux * w[0];
+                plan->ph_m[4 * k + 1] = ux * w[1];
+                plan->ph_m[4 * k + 2] = uy * w[0];
+                plan->ph_m[4 * k + 3] = uy * w[1];
+            }
+        }
     }
 
     // ---- regular (log m1, log m2) grid (sam.py:1349-1357)
@@ -603,6 +654,8 @@ int hgb_scatter_plan_build(const double *mtot, int n_mtot, const double *mrat, i
     sizes->n_nbr = nnz;
     sizes->n_grid = N;
     sizes->n_levels = nlev;
+    sizes->n_phases = nph;
+    sizes->phase_width = width;
     return HGB_OK;
 }
 

@@ -24,8 +24,8 @@ GRAD_MAXITER = 400     # CloughTocher2DInterpolator default sweep limit
 _DTYPES = dict(pts=np.float64, tri=np.int32, tri_kappa=np.float64, vtx_qinv=np.float64, nbr_ptr=np.int32,
                nbr_idx=np.int32, nbr_w=np.float64, level_ptr=np.int32, level_vtx=np.int32, grid_tri=np.int32,
                grid_bary=np.float64, grid_near=np.int32, grid_axis=np.float64, weights=np.float64,
-               back_idx=np.int32, back_t=np.float64, back_w=np.float64, lv_nbr_ptr=np.int32, lv_nbr=np.int32,
-               lv_nbr_w=np.float64, lv_qinv=np.float64)
+               back_idx=np.int32, back_t=np.float64, back_w=np.float64, ph_ptr=np.int32, ph_info=np.int32,
+               ph_nbr=np.int32, ph_m=np.float64)
 
 _PLANS = collections.OrderedDict()   # least recently used first
 _PLAN_CACHE_MAX = 8                   # plans kept per process (a 91 x 81 plan holds about 60 MB)
@@ -44,7 +44,8 @@ def host_plan(mtot, mrat, scatter, refine=4):
                   nbr_idx=(nnbr,), nbr_w=(nnbr, 4), level_ptr=(nlev + 1,), level_vtx=(npts,),
                   grid_tri=(ngrid * ngrid,), grid_bary=(ngrid * ngrid, 3), grid_near=(ngrid * ngrid,),
                   grid_axis=(ngrid,), weights=(ngrid, ngrid), back_idx=(npts, 2), back_t=(npts, 2),
-                  back_w=(npts, 2, ngrid), lv_nbr_ptr=(npts + 1,), lv_nbr=(nnbr,), lv_nbr_w=(nnbr, 4), lv_qinv=(npts, 4))
+                  back_w=(npts, 2, ngrid), ph_ptr=(npts, 4), ph_info=(npts, 4),
+                  ph_nbr=(N.SCATTER_DEG * npts + nnbr,), ph_m=(N.SCATTER_DEG * npts + nnbr, 4))
     arrs = {kk: np.zeros(shapes[kk], dtype=_DTYPES[kk]) for kk in N._SCATTER_ARRAYS}
     hp = N.HgbScatterHostPlan(**{kk: arrs[kk].ctypes.data_as(ctypes.c_void_p) for kk in N._SCATTER_ARRAYS})
     sz = N.HgbScatterSizes()
@@ -55,8 +56,7 @@ def host_plan(mtot, mrat, scatter, refine=4):
     arrs["tri_kappa"] = arrs["tri_kappa"][:sz.n_tri]
     arrs["nbr_idx"] = arrs["nbr_idx"][:sz.n_nbr]
     arrs["nbr_w"] = arrs["nbr_w"][:sz.n_nbr]
-    arrs["lv_nbr"] = arrs["lv_nbr"][:sz.n_nbr]
-    arrs["lv_nbr_w"] = arrs["lv_nbr_w"][:sz.n_nbr]
+    arrs["ph_ptr"] = arrs["ph_ptr"][:sz.n_phases]
     arrs["level_ptr"] = arrs["level_ptr"][:sz.n_levels + 1]
     return arrs, sz
 
@@ -77,6 +77,8 @@ class DevicePlan:
         s.n_grid = sz.n_grid
         s.n_tri = sz.n_tri
         s.n_levels = sz.n_levels
+        s.n_phases = sz.n_phases
+        s.phase_width = sz.phase_width
         for kk in N._SCATTER_ARRAYS:
             if kk != "grid_axis":
                 setattr(s, kk, N.ptr(self.dev[kk]))

@@ -129,6 +129,8 @@ typedef struct {
     int n_nbr;      /* directed point-neighbour entries */
     int n_grid;     /* refine*M nodes per axis */
     int n_levels;   /* Gauss-Seidel wavefront levels */
+    int n_phases;   /* phases of the pipelined sweeps (hgb_scatter_plan) */
+    int phase_width;   /* most points of one phase */
 } hgb_scatter_sizes;
 
 typedef struct {    /* host arrays, sized by hgb_scatter_plan_bounds */
@@ -149,11 +151,17 @@ typedef struct {    /* host arrays, sized by hgb_scatter_plan_bounds */
     int32_t *back_idx;  /* [n_pts][2] lower grid cell */
     double *back_t;     /* [n_pts][2] fractional offsets */
     double *back_w;     /* [n_pts][2][n_grid] (1-ty) bw and ty bw, bw = (1-tx) (W W)[:, a] + tx (W W)[:, a+1] */
-    /* the neighbourhoods again, indexed by level-order position p (point level_vtx[p]) */
-    int32_t *lv_nbr_ptr; /* [n_pts+1] */
-    int32_t *lv_nbr;    /* [n_nbr] neighbour positions, in the order of nbr_idx */
-    double *lv_nbr_w;   /* [n_nbr][4]: -2 w0, -2 w1, w2, w3 of nbr_w, in level order */
-    double *lv_qinv;    /* [n_pts][4] */
+    /* the gradient solve's pipelined sweeps.  Phase of a point: its level modulo n_phases, where
+     * n_phases exceeds the level distance of any two neighbours; stage: its level over n_phases.
+     * While a point of stage j makes its sweep k, one of stage j + 1 makes its sweep k - 1, so a
+     * pass over the phases advances every point once and reads exactly the values that sweeps one
+     * after another would read.  Points are numbered by position p, phase by phase. */
+    int32_t *ph_ptr;    /* [n_phases][4] first position, points, of these with at most HGB_SCATTER_DEG
+                         * neighbours (they come first), unused */
+    int32_t *ph_info;   /* [n_pts][4] point, stage, neighbours, first entry */
+    int32_t *ph_nbr;    /* [HGB_SCATTER_DEG n_pts + n_nbr] neighbours' positions; entry e of a point with few neighbours is
+                         * first + e times those points of its phase, otherwise first + e */
+    double *ph_m;       /* the same entries, [4]: M with g_i = c_i + sum_j M_ij g_j, row-major */
 } hgb_scatter_host_plan;
 
 typedef struct {    /* the same arrays on the device */
@@ -174,14 +182,17 @@ typedef struct {    /* the same arrays on the device */
     const int32_t *back_idx;
     const double *back_t;
     const double *back_w;
-    const int32_t *lv_nbr_ptr;
-    const int32_t *lv_nbr;
-    const double *lv_nbr_w;
-    const double *lv_qinv;
+    const int32_t *ph_ptr;
+    const int32_t *ph_info;
+    const int32_t *ph_nbr;
+    const double *ph_m;
     double grad_tol;    /* 1e-6 in the reference */
     int grad_maxiter;   /* 400 in the reference */
+    int n_phases, phase_width;   /* 0 (or a NULL ph_ array): sweeps one after another */
 } hgb_scatter_plan;
 
+#define HGB_SCATTER_DEG 8      /* a point with more neighbours is summed by a whole warp */
+#define HGB_SCATTER_STAGES 8   /* most sweeps in flight */
 /* Upper bounds of the plan array sizes (n_grid is exact). */
 int hgb_scatter_plan_bounds(int n_mtot, int n_mrat, int refine, hgb_scatter_sizes *out);
 /* Build the geometry on the host; mtot / mrat are HOST arrays; writes the actual sizes. */
