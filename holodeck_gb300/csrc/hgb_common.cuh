@@ -166,6 +166,29 @@ __device__ __forceinline__ double f32_to_f64_scaled(float v, int k) {
 // the bit pattern of -1.0, the "no target reached" sentinel of redz_final
 constexpr long long F64_MINUS_ONE_BITS = (long long)0xBFF0000000000000ull;
 
+// 1 / y and 1 / sqrt(y) in FP64 from the hardware's estimate r (relative error a few 2^-21 of the value
+// with y's low word cleared): with e = 1 - y r, 1 / y = r (1 + e + e^2 + ...), and with e = 1 - y r^2,
+// 1 / sqrt(y) = r (1 + e / 2 + 3 e^2 / 8 + ...).  The series cut after e^2 leaves less than 2^-57, so
+// the result carries one or two roundings.  Three and five FP64 operations in place of the eight to
+// twelve of a correctly rounded quotient or root, on a GPU whose FP64 pipe sets these kernels' time.
+// y positive and within 2^+-900 (no zero, subnormal, infinity or NaN: the caller sees to it).
+__device__ __forceinline__ double fast_rcp(double y) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(y));
+    const double e = __fma_rn(-y, r, 1.0);
+    return __fma_rn(r, __fma_rn(e, e, e), r);
+}
+__device__ __forceinline__ double fast_rsqrt(double y) {
+    double r;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(y));
+    const double e = __fma_rn(-y * r, r, 1.0);
+    return __fma_rn(r * e, __fma_rn(0.375, e, 0.5), r);
+}
+// whether a positive y lies within 2^+-900, from its exponent bits
+__device__ __forceinline__ bool fast_range(double y) {
+    return ((unsigned)__double2hiint(y) >> 20) - 123u < 1800u;
+}
+
 // Kahan-compensated FP32 accumulator
 struct Kahan32 {
     float s = 0.0f, c = 0.0f;

@@ -692,177 +692,183 @@ __global__ void __launch_bounds__(GW_ROWS) k_dbn_gw(CyConst cc, const double *__
     }
 }
 
-// The same root, one warp per cell and eight cells per block.  A lane holds the constants of nodes
-// s = lane + 32 k in registers: the hardening shape, the GW rate and the trapezoid coefficient
-// c[s] = 2 (sepa[s+1] - sepa[s]).  Each Brent round sums the lifetime c[s] / (v[s] + v[s+1]) with
-// one partial per lane and an xor-butterfly reduction.  Every lane ends with the same total
-// (addition is commutative), so the warp's Brent state stays uniform and the warps never wait for
-// one another.  The evaluation sequence is that of warp_brent; only the grouping of the step sum
-// differs from the reference's step order (a relative change of the lifetime near 1e-16, far
-// below the 1e-3 root tolerance, which the root follows unless a Brent comparison falls within
-// that margin: the normalisation is checked against the reference at 1e-10 in log10).
-constexpr int NB_CELLS = 8;    // 256 threads: half an SM's registers, so other stages' blocks fit beside
-constexpr int NB_NODES = 10;   // nodes per lane: nsteps + 1 <= 320
+// The same root with CPW cells per warp, 32 / CPW lanes each.  The lifetime's trapezoid sum is
+//   T(norm) = sum_s 1 / (norm alpha_s + beta_s),  alpha_s = (shape_s + shape_s+1) / (2 dx_s) and
+//   beta_s = (gw_s + gw_s+1) / (2 dx_s)  (rates counted positive, dx_s the step's width),
+// so a Brent round costs a step one multiply-add, a reciprocal (fast_rcp) and an addition: 5 FP64
+// operations, where v_s = norm shape_s + gw_s, their sum, the quotient and the addition took 14.  A lane
+// keeps the alpha and beta of a run of consecutive steps in registers.  Each cell's lanes share its Brent
+// state (an xor-butterfly leaves the same total in all of them); the root finding itself, one exp10 and
+// some fifty uniform FP64 operations a round, is shared by the warp's CPW cells, neighbours in the grid
+// that need about the same number of rounds.  The log10 separations are init - s dx, one rounding each.
+// (Separations as products of a few shared powers of ten would save another tenth of the time, and two
+// roundings that come out cubed: the norm's error doubles, 4e-17 to 9e-17, so each is its own exp10.)
+// The sum's grouping moves the lifetime by about 1e-16 relative, far below the root tolerance of 1e-3,
+// which the root follows unless a Brent comparison falls within that margin (checked against the
+// reference at 1e-10 in log10).  FP64 bounds it.  91 x 81 cells: 2767 us with one cell per warp and a
+// quotient per node and round, NORM_4 us with four (NORM_1 and NORM_2 with one and two); 30 x 30 cells:
+// 441 us before, NORMS_1 with one, NORMS_4 with four.
+constexpr int NB_STEPS = 320;   // steps the kernel holds in registers
 
-__global__ void __launch_bounds__(NB_CELLS * 32, 2) k_hardening_norm_blk(CyConst cc, NormArgs a,
-                                                                       const double *__restrict__ mtot,
-                                                                       const double *__restrict__ mrat, int n,
-                                                                       double *__restrict__ norm_log10,
-                                                                       double *__restrict__ norm, int *d_status) {
-    extern __shared__ double smem[];   // [NB_CELLS][S + 1]: each warp's log10 separations
-    const int S = a.nsteps;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int cell = blockIdx.x * NB_CELLS + warp;
-    if (cell >= n) return;   // the whole warp: no block-wide barrier follows
-    double *row = smem + (size_t)warp * (S + 1);
-    const double mt = mtot[cell], mr = mrat[cell];
-    const double mt3 = pow(mt, 3.0), mr12 = pow(1.0 + mr, 2.0);
-    // log10 separation nodes by repeated subtraction (sam_cyutils.pyx:367-383)
-    if (lane == 0) {
-        const double risco_log10 = log10(3.0 * HGB_CY_SCHW * mt);
-        const double dx = (a.sepa_init_log10 - risco_log10) / S;
-        double sl = a.sepa_init_log10;
-        row[0] = sl;
-        for (int s = 1; s <= S; s++) {
-            sl -= dx;
-            row[s] = sl;
-        }
-    }
-    __syncwarp();
-    // per node: the hardening shape (1 + x)^(gi - go) / x^(gi - 1) and the GW rate, which do not
-    // depend on the normalisation, so each Brent round costs one product and one sum per node
-    double rr[NB_NODES], gw[NB_NODES], sp[NB_NODES], cf[NB_NODES];
-#pragma unroll
-    for (int k = 0; k < NB_NODES; k++) {
-        const int s = lane + 32 * k;
-        rr[k] = 1.0;
-        gw[k] = sp[k] = 0.0;
-        if (s <= S) {
-            const double x = pow(10.0, row[s]);
-            const double xx = x / a.rchar;
-            rr[k] = pow_ratio_planned(1.0 + xx, -a.go + a.gi, a.p_outer, xx, a.gi - 1.0, a.p_inner);
-            gw[k] = cc.c_dadt * mt3 * mr / (x * x * x) / mr12;
-            sp[k] = x;
-        }
-    }
-    // c[s] = 2 (sepa[s+1] - sepa[s]) for s < S, 0 beyond
-#pragma unroll
-    for (int k = 0; k < NB_NODES; k++) {
-        double nxt = __shfl_down_sync(0xffffffffu, sp[k], 1);
-        const double wrap = __shfl_sync(0xffffffffu, (k + 1 < NB_NODES) ? sp[k + 1] : 0.0, 0);
-        if (lane == 31) nxt = wrap;
-        const int s = lane + 32 * k;
-        cf[k] = (s < S) ? 2.0 * (nxt - sp[k]) : 0.0;
-    }
 
-    // Brent's method as in warp_brent, one evaluation per round
-    double xa = NORM_LOG10_LO, xb = NORM_LOG10_HI, xc = 0.0, fa = 0.0, fb = 0.0, fc = 0.0, d = 0.0, e = 0.0;
-    int stage = 0, it = 0, nit = 0;
-    double root = 0.0;
-    for (int round = 0; round < BRENT_MAXITER + 2; round++) {
-        const double xe = (stage == 0) ? xa : xb;
-        const double nrm = pow(10.0, xe);
-        double v[NB_NODES];
-#pragma unroll
-        for (int k = 0; k < NB_NODES; k++) {
-            double dl = -nrm * rr[k];
-            dl += gw[k];
-            v[k] = dl;
-        }
-        double part = 0.0;
-#pragma unroll
-        for (int k = 0; k < NB_NODES; k++) {
-            double vn = __shfl_down_sync(0xffffffffu, v[k], 1);
-            const double wrap = __shfl_sync(0xffffffffu, (k + 1 < NB_NODES) ? v[k + 1] : 0.0, 0);
-            if (lane == 31) vn = wrap;
-            const int s = lane + 32 * k;
-            if (s < S) part += cf[k] / (v[k] + vn);
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-        const double fv = part - a.target_time;
-        if (stage == 0) {
-            fa = fv;
-            stage = 1;
-            continue;
-        }
-        fb = fv;
-        if (stage == 1) {
-            stage = 2;
-            if (fa * fb > 0.0) {
-                root = 0.0;
-                break;
-            }
-            if (fa == 0.0) {
-                root = xa;
-                break;
-            }
-            if (fb == 0.0) {
-                root = xb;
-                break;
-            }
-            xc = xa;
-            fc = fa;
-            d = xb - xa;
-            e = d;
-            it = 0;
-        } else {
-            it++;
-            if (it >= BRENT_MAXITER) {
-                root = xb;
-                nit = BRENT_MAXITER + 1;
-                break;
-            }
-        }
-        nit = it + 1;
-        if (fb * fc > 0.0) {
-            xc = xa;
-            fc = fa;
-            d = xb - xa;
-            e = d;
-        }
-        if (fabs(fc) < fabs(fb)) {
-            xa = xb; xb = xc; xc = xa;
-            fa = fb; fb = fc; fc = fa;
-        }
-        const double tol = 0.5 * (BRENT_XTOL + BRENT_RTOL * fabs(xb));
-        const double m = 0.5 * (xc - xb);
-        if (fb == 0.0 || fabs(m) < tol) {
-            root = xb;
-            break;
-        }
-        if (fabs(e) > tol && fabs(fb) < fabs(fa)) {
-            double sst;
-            if (xa == xc) {
-                sst = -fb * (xb - xa) / (fb - fa);
-            } else {
-                const double da = (fa - fb) / (xa - xb);
-                const double dc = (fc - fb) / (xc - xb);
-                sst = -fb * (fc * dc - fa * da) / (dc * da * (fc - fa));
-            }
-            if (2.0 * fabs(sst) < fmin(fabs(e), 3.0 * fabs(m) - tol)) {
-                e = d;
-                d = sst;
-            } else {
-                d = m;
-                e = m;
-            }
-        } else {
-            d = m;
-            e = m;
-        }
-        xa = xb;
-        fa = fb;
-        xb = xb + ((fabs(d) > tol) ? d : ((m > 0.0) ? tol : -tol));
-    }
-    if (lane == 0) {
-        norm_log10[cell] = root;
-        if (norm) norm[cell] = pow(10.0, root);
-        if (nit > BRENT_MAXITER) hgb::flag(d_status, HGB_STATUS_ITERATION_LIMIT);
-    }
+// y^p of the hardening shape's outer factor, y = 1 + x: a planned negative (half-)integer power from one
+// reciprocal square root, any other exponent as pow_planned
+__device__ __forceinline__ double shape_outer(double y, double p, PowPlan plan) {
+    if (plan.kind == 0 || !plan.neg || !hgb::fast_range(y)) return pow_planned(y, p, plan);
+    const double r = hgb::fast_rsqrt(y), r2 = r * r;
+    double v = plan.kind == 2 ? r : 1.0;
+    for (int i = 0; i < plan.n; i++) v *= r2;
+    return v;
 }
 
-size_t norm_blk_smem(int nsteps) { return sizeof(double) * (size_t)NB_CELLS * ((size_t)nsteps + 1); }
+template <int CPW>
+__global__ void __launch_bounds__(32) k_hardening_norm_sub(CyConst cc, NormArgs a, const double *__restrict__ mtot,
+                                                           const double *__restrict__ mrat, int n,
+                                                           double *__restrict__ norm_log10,
+                                                           double *__restrict__ norm, int *d_status) {
+    constexpr int LPC = 32 / CPW, NL = NB_STEPS / LPC;   // lanes per cell, steps per lane
+    const int S = a.nsteps;
+    const int sub = threadIdx.x % LPC;
+    const int own = blockIdx.x * CPW + threadIdx.x / LPC;
+    const int cell = min(own, n - 1);   // a last, partly filled warp repeats its last cell
+    const double mt = mtot[cell], mr = mrat[cell];
+    const double opq = 1.0 + mr;
+    const double gw_k = -cc.c_dadt * (mt * mt * mt) * mr / (opq * opq);
+    const double dx = (a.sepa_init_log10 - log10(3.0 * HGB_CY_SCHW * mt)) / S;
+    const double inv_rchar = 1.0 / a.rchar;
+    double al[NL], be[NL];
+    {
+        const double pin = 1.0 - a.gi;
+        double x0 = 0.0, r0 = 0.0, g0 = 0.0;   // the previous node: separation, hardening shape, GW rate
+        double sd = (double)(sub * NL);
+#pragma unroll
+        for (int k = 0; k <= NL; k++) {
+            const int s = sub * NL + k;
+            const double x1 = exp10(__fma_rn(-sd, dx, a.sepa_init_log10));
+            sd += 1.0;
+            const double xx = x1 * inv_rchar;
+            const double r1 = shape_outer(1.0 + xx, -a.go + a.gi, a.p_outer) *
+                              pow_planned(xx, pin, PowPlan{a.p_inner.kind, a.p_inner.n, !a.p_inner.neg});
+            const double x3 = x1 * x1 * x1;
+            const double g1 = hgb::fast_range(x3) ? gw_k * hgb::fast_rcp(x3) : gw_k / x3;
+            if (k > 0) {
+                const double w = x0 - x1;
+                const double c = 0.5 * (hgb::fast_range(w) ? hgb::fast_rcp(w) : 1.0 / w);
+                // steps beyond the last add 1e-60 s
+                al[k - 1] = s <= S ? (r0 + r1) * c : 0.0;
+                be[k - 1] = s <= S ? (g0 + g1) * c : 1e60;
+            }
+            x0 = x1;
+            r0 = r1;
+            g0 = g1;
+        }
+    }
+
+    // Brent's method as in warp_brent, one evaluation per round; the warp goes on until its last cell is
+    // done (its lanes exchange partial sums, so none leaves early)
+    double xa = NORM_LOG10_LO, xb = NORM_LOG10_HI, xc = 0.0, fa = 0.0, fb = 0.0, fc = 0.0, d = 0.0, e = 0.0;
+    double root = 0.0;
+    bool done = false, limit = false;
+    for (int round = 0; round < BRENT_MAXITER + 2; round++) {
+        const double nrm = exp10(round == 0 ? xa : xb);
+        double part = 0.0;
+#pragma unroll
+        for (int k = 0; k + 1 < NL; k += 4) {
+            // four steps share a reciprocal (two, at the end of an odd half): 15 FP64 operations, not 20
+            const double y0 = __fma_rn(nrm, al[k], be[k]), y1 = __fma_rn(nrm, al[k + 1], be[k + 1]);
+            double num = y0 + y1, den = y0 * y1;
+            if (k + 3 < NL) {
+                const double y2 = __fma_rn(nrm, al[k + 2], be[k + 2]), y3 = __fma_rn(nrm, al[k + 3], be[k + 3]);
+                const double d2 = y2 * y3;
+                num = __fma_rn(num, d2, (y2 + y3) * den);
+                den *= d2;
+            }
+            if (hgb::fast_range(den)) {
+                part = __fma_rn(num, hgb::fast_rcp(den), part);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+                    if (k + i < NL) part += 1.0 / __fma_rn(nrm, al[k + i], be[k + i]);
+            }
+        }
+#pragma unroll
+        for (int o = LPC / 2; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+        const double fv = part - a.target_time;
+        if (round == 0) {
+            fa = fv;
+            continue;
+        }
+        if (!done) {
+            fb = fv;
+            if (round == 1) {
+                if (fa * fb > 0.0) {
+                    done = true;   // no root between the ends: 0
+                } else if (fa == 0.0) {
+                    root = xa;
+                    done = true;
+                } else if (fb == 0.0) {
+                    root = xb;
+                    done = true;
+                }
+                xc = xa;
+                fc = fa;
+                d = xb - xa;
+                e = d;
+            } else if (round > BRENT_MAXITER) {
+                root = xb;
+                limit = done = true;
+            }
+        }
+        if (!done) {
+            if (fb * fc > 0.0) {
+                xc = xa;
+                fc = fa;
+                d = xb - xa;
+                e = d;
+            }
+            if (fabs(fc) < fabs(fb)) {
+                xa = xb; xb = xc; xc = xa;
+                fa = fb; fb = fc; fc = fa;
+            }
+            const double tol = 0.5 * (BRENT_XTOL + BRENT_RTOL * fabs(xb));
+            const double m = 0.5 * (xc - xb);
+            if (fb == 0.0 || fabs(m) < tol) {
+                root = xb;
+                done = true;
+            } else {
+                if (fabs(e) > tol && fabs(fb) < fabs(fa)) {
+                    double sst;
+                    if (xa == xc) {
+                        sst = -fb * (xb - xa) / (fb - fa);
+                    } else {
+                        const double da = (fa - fb) / (xa - xb);
+                        const double dc = (fc - fb) / (xc - xb);
+                        sst = -fb * (fc * dc - fa * da) / (dc * da * (fc - fa));
+                    }
+                    if (2.0 * fabs(sst) < fmin(fabs(e), 3.0 * fabs(m) - tol)) {
+                        e = d;
+                        d = sst;
+                    } else {
+                        d = m;
+                        e = m;
+                    }
+                } else {
+                    d = m;
+                    e = m;
+                }
+                xa = xb;
+                fa = fb;
+                xb = xb + ((fabs(d) > tol) ? d : ((m > 0.0) ? tol : -tol));
+            }
+        }
+        if (__all_sync(0xffffffffu, done)) break;
+    }
+    if (sub == 0 && own < n) {
+        norm_log10[own] = root;
+        if (norm) norm[own] = pow(10.0, root);
+        if (limit) hgb::flag(d_status, HGB_STATUS_ITERATION_LIMIT);
+    }
+}
 
 size_t norm_smem_per_warp(int nsteps) { return (size_t)5 * (nsteps + 1) * sizeof(double); }
 
@@ -886,11 +892,16 @@ int hgb_find_2pwl_hardening_norm(double target_time, const double *mtot, const d
     if (rc) return rc;
     NormArgs a{target_time, log10(sepa_init), rchar, gamma_inner, gamma_outer, nsteps,
                pow_plan(-gamma_outer + gamma_inner), pow_plan(gamma_inner - 1.0)};
-    if (nsteps + 1 <= 32 * NB_NODES) {
-        const size_t bsmem = norm_blk_smem(nsteps);
-        if ((rc = hgb::ensure_dyn_smem((const void *)k_hardening_norm_blk, bsmem))) return rc;
-        k_hardening_norm_blk<<<(unsigned)hgb::ceil_div(n, NB_CELLS), NB_CELLS * 32, bsmem, (cudaStream_t)stream>>>(
-            hgb::cy_const(), a, mtot, mrat, n, norm_log10, norm, d_status);
+    if (nsteps <= NB_STEPS) {
+        cudaStream_t st = (cudaStream_t)stream;
+        // four cells a warp do least work, but below about one warp per sub-partition two are faster:
+        // 30 x 30 cells 246 and 153 us, 60 x 60 cells 496 and 558 us
+        if (n >= 4 * 4 * hgb::sm_count())
+            k_hardening_norm_sub<4><<<(unsigned)hgb::ceil_div(n, 4), 32, 0, st>>>(hgb::cy_const(), a, mtot, mrat, n,
+                                                                                  norm_log10, norm, d_status);
+        else
+            k_hardening_norm_sub<2><<<(unsigned)hgb::ceil_div(n, 2), 32, 0, st>>>(hgb::cy_const(), a, mtot, mrat, n,
+                                                                                  norm_log10, norm, d_status);
         return hgb::check_launch();
     }
     unsigned blocks = (unsigned)hgb::ceil_div(n, wpb);
