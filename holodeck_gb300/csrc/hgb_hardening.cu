@@ -695,8 +695,9 @@ __global__ void __launch_bounds__(GW_ROWS) k_dbn_gw(CyConst cc, const double *__
 // The same root with CPW cells per warp, 32 / CPW lanes each.  The lifetime's trapezoid sum is
 //   T(norm) = sum_s 1 / (norm alpha_s + beta_s),  alpha_s = (shape_s + shape_s+1) / (2 dx_s) and
 //   beta_s = (gw_s + gw_s+1) / (2 dx_s)  (rates counted positive, dx_s the step's width),
-// so a Brent round costs a step one multiply-add, a reciprocal (fast_rcp) and an addition: 5 FP64
-// operations, where v_s = norm shape_s + gw_s, their sum, the quotient and the addition took 14.  A lane
+// so a Brent round costs a step one multiply-add, a share of a reciprocal (fast_rcp, four steps over one
+// denominator) and an addition: 3.75 FP64 operations, where v_s = norm shape_s + gw_s, their sum, the
+// quotient and the addition took 14.  A lane
 // keeps the alpha and beta of a run of consecutive steps in registers.  Each cell's lanes share its Brent
 // state (an xor-butterfly leaves the same total in all of them); the root finding itself, one exp10 and
 // some fifty uniform FP64 operations a round, is shared by the warp's CPW cells, neighbours in the grid
@@ -705,9 +706,9 @@ __global__ void __launch_bounds__(GW_ROWS) k_dbn_gw(CyConst cc, const double *__
 // roundings that come out cubed: the norm's error doubles, 4e-17 to 9e-17, so each is its own exp10.)
 // The sum's grouping moves the lifetime by about 1e-16 relative, far below the root tolerance of 1e-3,
 // which the root follows unless a Brent comparison falls within that margin (checked against the
-// reference at 1e-10 in log10).  FP64 bounds it.  91 x 81 cells: 2767 us with one cell per warp and a
-// quotient per node and round, NORM_4 us with four (NORM_1 and NORM_2 with one and two); 30 x 30 cells:
-// 441 us before, NORMS_1 with one, NORMS_4 with four.
+// reference at 1e-10 in log10).  FP64 bounds it.  91 x 81 cells: 2822 us with one cell per warp and a
+// quotient per node and round, 841 us with four (896 and 1081 with two and one); general exponents
+// (two pow() a node) 3626 and 1769 us.
 constexpr int NB_STEPS = 320;   // steps the kernel holds in registers
 
 
