@@ -411,6 +411,328 @@ __global__ void __launch_bounds__(512) k_dbn_2pwl(CyConst cc, Dbn2plArgs a, int 
     }
 }
 
+// y^p of the hardening shape's outer factor, y = 1 + x: a planned negative (half-)integer power from one
+// reciprocal square root, any other exponent as pow_planned
+__device__ __forceinline__ double shape_outer(double y, double p, PowPlan plan) {
+    if (plan.kind == 0 || !plan.neg || !hgb::fast_range(y)) return pow_planned(y, p, plan);
+    const double r = hgb::fast_rsqrt(y), r2 = r * r;
+    double v = plan.kind == 2 ? r : 1.0;
+    for (int i = 0; i < plan.n; i++) v *= r2;
+    return v;
+}
+
+// The walk for ascending targets: which step brackets a target is decided in FP32, and only the bracket
+// found is evaluated in FP64.
+// One block takes a run of mrat cells of one mtot.  What depends on mtot alone (separations, rest
+// frequencies, the steps' shape and GW sums alpha and beta, see k_hardening_norm_sub) is built once per
+// block, and the cells' step times 1 / (norm alpha + gw_k beta) and their running sums.  Then, for a few
+// cells at a time:
+//   A  one thread per (cell, redshift) row walks its nodes in FP32 (time, redshift, observed frequency:
+//      relative error a few 1e-7 against steps of some percent) and notes for each target the step and
+//      the age-table interval it starts in;
+//   B  the row's (redshift, target) elements, spread over all threads with the target fastest, test the
+//      noted step in FP64 and move by one where FP32 chose a neighbour.  The tests at a node are
+//      ft (1 + z) >= frst from its right and <= frst from its left with the same values, so every target
+//      between the first node and the last belongs to a step.  Of the time in the bracket,
+//        t_l + (t_r - t_l) (ft - f_l) / (f_r - f_l),  f = frst / (1 + z),
+//      both frequencies' quotients and the interpolation's are one reciprocal: twenty FP64 operations.
+// FP64 bounds both forms, but the walk in FP64 spent some 25 operations a step on 80 steps a row,
+// comparisons among them, with lanes idle where their neighbours walk longer, and wrote its outputs
+// eight bytes to a line.  91 x 81 x 101 points, 40 targets: 3130 us before, 1002 us now (FP64 pipe 75% busy); 30^3 points
+// with 20: 443 and 147 us.
+constexpr int WK_THREADS = 256;
+constexpr unsigned WK_NONE = 0xFFFFFFFFu, WK_NAN = 0xFFFFFFFEu;
+
+struct WalkShape {
+    int cb;       // cells walked together
+    int qc;       // mrat cells per block
+    int rows;     // rows of one pass (cb cells' rows go in passes of this many)
+    size_t smem;
+};
+
+// The log10 separations of the reference's loop (S subtractions of dx, each rounded) without the chain of
+// S dependent operations: while the values stay in one binade, with last place u, every rounded step is
+// the same multiple of u (dx rounded to it; only a dx half way between two would alternate), so the
+// nodes of a binade are first - j d exactly.  Writes the segments' first values, steps and first nodes and
+// returns their number; what does not fit the scheme (values at or below 1, a tie) goes to `node`, one
+// after another, as the last, empty segment's place.
+constexpr int WK_SEGS = 8;
+
+__device__ int log_nodes(double init, double dx, int S, double *first, double *step, int *seg, double *node) {
+    double sl = init;
+    int s = 0, k = 0;
+    while (s <= S && k < WK_SEGS - 1 && sl > 1.0 && dx > 0.0) {
+        const double low = __hiloint2double(__double2hiint(sl) & 0x7FF00000, 0);   // the binade's lower end
+        const double d = sl - (sl - dx);
+        if (!(sl - dx >= low) || 2.0 * fabs(dx - d) >= low * 0x1.0p-52) {   // one step leaves it, or a tie
+            seg[k] = s;
+            first[k] = sl;
+            step[k++] = 0.0;
+            sl -= dx;
+            s++;
+            continue;
+        }
+        int j = (int)fmin((sl - low) / d, (double)(S - s));   // steps that stay
+        while (j > 0 && sl - (double)j * d < low) j--;
+        while (j < S - s && sl - (double)(j + 1) * d >= low) j++;
+        seg[k] = s;
+        first[k] = sl;
+        step[k++] = d;
+        s += j + 1;
+        sl = (sl - (double)j * d) - dx;   // the step out of the binade rounds by the next one's last place
+    }
+    seg[k] = min(s, S + 1);
+    for (; s <= S; s++) {
+        node[s] = sl;
+        sl -= dx;
+    }
+    return k;
+}
+
+__host__ __device__ inline int wk_stride(int nf) { return nf | 1; }   // an odd row length keeps the lanes' rows in different banks
+
+__global__ void __launch_bounds__(WK_THREADS, 3) k_dbn_2pwl_walk(
+    CyConst cc, Dbn2plArgs a, WalkShape ws, const double *__restrict__ fobs, const double *__restrict__ hard_norm,
+    const double *__restrict__ mtot, const double *__restrict__ mrat, const double *__restrict__ redz,
+    const double *__restrict__ gmt_time, const double *__restrict__ zgrid_g, const double *__restrict__ agrid_g,
+    double *__restrict__ redz_final, double *__restrict__ diff_num) {
+    extern __shared__ double smem[];
+    const int S = a.num_steps, NI = a.n_interp, NF = a.n_freq, NZ = a.n_redz;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    double *zg = smem, *ag = zg + NI, *sz = ag + NI;   // age table and dz/dt of its intervals
+    double *ft = sz + NI;                              // [NF]
+    double *rage = ft + NF;                            // [NZ] age at the starting redshift
+    double *frst = rage + NZ, *al = frst + S + 1, *be = al + S + 1;   // [S + 1] nodes, [S] steps
+    double *base = be + S + 1;                         // [rows] merger time
+    double *tn = base + ws.rows;                       // [qc][S + 1] time of a cell's nodes from the first
+    float *zgf = (float *)(tn + (size_t)ws.qc * (S + 1)), *agf = zgf + NI, *szf = agf + NI, *ftf = szf + NI;
+    float *frf = ftf + NF;
+    unsigned *code = (unsigned *)(frf + S + 1);   // [rows][wk_stride(NF)] step | interval << 16
+    __shared__ int s_first;
+    const int nqb = (a.n_mrat + ws.qc - 1) / ws.qc;
+    const int ii = blockIdx.x / nqb, q0 = (blockIdx.x % nqb) * ws.qc, q1 = min(q0 + ws.qc, a.n_mrat);
+    const double mt = mtot[ii];
+
+    for (int i = t; i < NI; i += WK_THREADS) {
+        zg[i] = zgrid_g[i];
+        ag[i] = agrid_g[i];
+    }
+    for (int f = t; f < NF; f += WK_THREADS) {
+        ft[f] = fobs[f];
+        ftf[f] = (float)fobs[f];
+    }
+    // nodes: separation, and in the steps' arrays for now the hardening shape and 1 / separation^3
+    double *sepa = tn;   // the first cell's times come later
+    __shared__ double s_sl[WK_SEGS], s_d[WK_SEGS];
+    __shared__ int s_seg[WK_SEGS + 1], s_nseg;
+    if (t == 0) s_nseg = log_nodes(a.sepa_init_log10, (a.sepa_init_log10 - log10(3.0 * HGB_CY_SCHW * mt)) / S, S, s_sl, s_d, s_seg, sepa);
+    __syncthreads();
+    for (int k = 0; k < s_nseg; k++)
+        for (int s = s_seg[k] + t; s < s_seg[k + 1]; s += WK_THREADS) sepa[s] = __fma_rn(-(double)(s - s_seg[k]), s_d[k], s_sl[k]);
+    __syncthreads();
+    {
+        const double inv_rchar = 1.0 / a.rchar, kf = cc.kfreq * sqrt(mt), pin = 1.0 - a.gi;
+        for (int s = t; s <= S; s += WK_THREADS) {
+            const double sp = exp10(sepa[s]);
+            const double r = hgb::fast_range(sp) ? hgb::fast_rsqrt(sp) : 1.0 / sqrt(sp);
+            const double xx = sp * inv_rchar, r2 = r * r;
+            sepa[s] = sp;
+            frst[s] = kf * (r2 * r);
+            frf[s] = (float)frst[s];
+            al[s] = shape_outer(1.0 + xx, -a.go + a.gi, a.p_outer) *
+                    pow_planned(xx, pin, PowPlan{a.p_inner.kind, a.p_inner.n, !a.p_inner.neg});
+            be[s] = r2 * r2 * r2;
+        }
+    }
+    __syncthreads();
+    for (int i = t; i < NI; i += WK_THREADS) {
+        if (i < NI - 1) {
+            sz[i] = (zg[i + 1] - zg[i]) / (ag[i + 1] - ag[i]);
+            szf[i] = (float)sz[i];
+        }
+        zgf[i] = (float)zg[i];
+        agf[i] = (float)ag[i];
+    }
+    for (int k = t; k < NZ; k += WK_THREADS) {   // sam_cyutils.pyx:563-573
+        const double zk = redz[k];
+        int zi = hgb::bracket_decreasing_from0(NI, zk, zg);
+        if (zi > NI - 2) zi = NI - 2;
+        rage[k] = hgb::interp_between(zk, zg[zi], zg[zi + 1], ag[zi], ag[zi + 1]);
+    }
+    if (t == 0) {   // first step whose right edge reaches the lowest target (z >= 0: observed <= rest frame)
+        int lo = 0, hi = S;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (frst[mid + 1] < ft[0]) lo = mid + 1;
+            else hi = mid;
+        }
+        s_first = lo;
+    }
+    for (int s0 = 0; s0 < S; s0 += WK_THREADS) {   // sums over a step's two nodes over twice its width
+        const int s = s0 + t;
+        double av = 0.0, bv = 0.0;
+        if (s < S) {
+            const double w = sepa[s] - sepa[s + 1];
+            const double c = 0.5 * (hgb::fast_range(w) ? hgb::fast_rcp(w) : 1.0 / w);
+            av = (al[s] + al[s + 1]) * c;
+            bv = (be[s] + be[s + 1]) * c;
+        }
+        __syncthreads();   // every node of this run is read, and node s0 + WK_THREADS is rewritten next
+        if (s < S) {
+            al[s] = av;
+            be[s] = bv;
+        }
+    }
+    __syncthreads();
+    const int first = s_first;
+    const float age_f = (float)ag[NI - 1] * 1.000001f;   // beyond it in FP32: beyond the table's end in FP64
+    const long long age_bits = __double_as_longlong(ag[NI - 1]);
+    const int stride = wk_stride(NF);
+
+    // node times of the block's cells: every step by its own thread, then one thread per cell adds them in
+    // step order.  The order matters: a target reached just before the present is at z ~ 1e-7, where one
+    // ulp of the time (64 s) is 1e-9 of the distance, so the sums round as the reference's do.
+    const int nq = q1 - q0;
+    for (int i = t; i < nq * S; i += WK_THREADS) {
+        const int c = i / S, s = i % S;
+        const double mr = mrat[q0 + c], opq = 1.0 + mr;
+        const double gw_k = -cc.c_dadt * (mt * mt * mt) * mr / (opq * opq);
+        const double y = __fma_rn(hard_norm[(long)ii * a.n_mrat + q0 + c], al[s], gw_k * be[s]);
+        tn[(size_t)c * (S + 1) + s + 1] = hgb::fast_range(y) ? hgb::fast_rcp(y) : 1.0 / y;
+    }
+    __syncthreads();
+    if (t < nq) {
+        double *tc = tn + (size_t)t * (S + 1);
+        double te = 0.0;
+        tc[0] = 0.0;
+#pragma unroll 8
+        for (int s = 1; s <= S; s++) {
+            te += tc[s];
+            tc[s] = te;
+        }
+    }
+
+    for (int qb = q0; qb < q1; qb += ws.cb) {
+        const int nc = min(ws.cb, q1 - qb);
+        const long cell0 = (long)ii * a.n_mrat + qb;
+        const double *tnb = tn + (size_t)(qb - q0) * (S + 1);
+        for (int row0 = 0; row0 < nc * NZ; row0 += ws.rows) {
+            const int nr = min(ws.rows, nc * NZ - row0);
+            __syncthreads();   // node times are complete; the previous pass is written
+            // ---- A
+            if (t < nr) {
+                const int c = (row0 + t) / NZ, kk = (row0 + t) % NZ;
+                const double b = gmt_time[(cell0 + c) * NZ + kk];
+                base[t] = b;
+                const float bf = hgb::f64_to_f32_rz(b + rage[kk]);
+                const double *tc = tnb + (size_t)c * (S + 1);
+                unsigned *cd = code + t * stride;
+                int f = 0;
+                unsigned rest = WK_NONE;
+                if (b != b) {
+                    rest = WK_NAN;   // every step brackets every target, with no time
+                } else {
+                    float tl = bf + hgb::f64_to_f32_rz(tc[first]);
+                    int il = 0, hi = NI - 2;   // interval of the first node
+                    while (il < hi) {
+                        const int mid = (il + hi) >> 1;
+                        if (agf[mid + 1] < tl) il = mid + 1;
+                        else hi = mid;
+                    }
+                    int n = first;
+                    for (; n < S && f < NF && tl <= age_f; n++) {
+                        const float tr = bf + hgb::f64_to_f32_rz(tc[n + 1]), fr = frf[n + 1];
+                        const int in = il;
+                        while (il < NI - 2 && agf[il + 1] < tr) il++;
+                        const float p = 1.0f + fmaxf(zgf[il] + (tr - agf[il]) * szf[il], 0.0f);
+                        while (f < NF && ftf[f] * p < fr) cd[f++] = (unsigned)n | ((unsigned)in << 16);
+                        tl = tr;
+                    }
+                    if (n == S && S > first) rest = (unsigned)(S - 1) | ((unsigned)il << 16);   // within FP32 of the last node
+                }
+                for (; f < NF; f++) cd[f] = rest;
+            }
+            __syncthreads();
+            // ---- B
+            double *rf = redz_final + (cell0 * NZ + row0) * NF;
+            double *dn = diff_num + (cell0 * NZ + row0) * NF;
+            const int dr = WK_THREADS / NF, df = WK_THREADS - dr * NF;
+            int r = t / NF, f = t - r * NF;
+            while (r < nr) {
+                const unsigned cd = code[r * stride + f];
+                double out_r = -1.0, out_t = 0.0;
+                if (cd == WK_NAN) {
+                    out_r = 0.0;
+                    out_t = base[r];
+                } else if (cd != WK_NONE) {
+                    int s = (int)(cd & 0xFFFFu), il = (int)(cd >> 16);
+                    const double *tc = tnb + (size_t)((row0 + r) / NZ) * (S + 1);
+                    const double gmt = base[r], ra = rage[(row0 + r) % NZ], target = ft[f];
+                    for (int go = 0; go <= S; go++) {   // at most one move in practice
+                        const double tl = tc[s] + gmt + ra, tr = tc[s + 1] + gmt + ra;
+                        if (__double_as_longlong(tl) > age_bits) break;
+                        while (il < NI - 2 && __double_as_longlong(ag[il + 1]) < __double_as_longlong(tl)) il++;
+                        while (il > 0 && __double_as_longlong(ag[il]) > __double_as_longlong(tl)) il--;
+                        const double zl = __fma_rn(tl - ag[il], sz[il], zg[il]);
+                        if (__double2hiint(zl) < 0) break;
+                        const double pl = 1.0 + zl, fl = frst[s];
+                        const double x = __fma_rn(target, pl, -fl);
+                        if (__double2hiint(x) < 0) {   // below the step
+                            if (s == first) break;
+                            s--;
+                            continue;
+                        }
+                        int ir = il;
+                        while (ir < NI - 2 && __double_as_longlong(ag[ir + 1]) < __double_as_longlong(tr)) ir++;
+                        double zr = __fma_rn(tr - ag[ir], sz[ir], zg[ir]);
+                        if (__double2hiint(zr) < 0) zr = 0.0;
+                        const double pr = 1.0 + zr, fr = frst[s + 1];
+                        const double y = __fma_rn(-target, pr, fr);
+                        if (__double2hiint(y) < 0) {   // above it
+                            if (s == S - 1) break;
+                            s++;
+                            continue;
+                        }
+                        const double den = __fma_rn(fr, pl, -(fl * pr)) * 0x1.0p40;   // frequencies of 1e-10 Hz and less
+                        const double num = (tr - tl) * (x * 0x1.0p40) * pr;
+                        const double tt = hgb::fast_range(den) ? __fma_rn(num, hgb::fast_rcp(den), tl) : tl + num / den;
+                        if (!(__double_as_longlong(tt) > age_bits)) {
+                            out_r = hgb::f32_to_f64_scaled((float)il, 0);   // the interval the evaluation starts from
+                            out_t = tt;
+                        }
+                        break;
+                    }
+                }
+                const long e = (long)r * NF + f;
+                rf[e] = out_r;
+                dn[e] = out_t;
+                r += dr;
+                f += df;
+                if (f >= NF) {
+                    f -= NF;
+                    r++;
+                }
+            }
+        }
+    }
+}
+
+// Cells and rows of a block, and its shared memory: cells walked together fill the threads with rows, and
+// a block takes up to eight of them where that leaves about eight blocks a multiprocessor.
+WalkShape walk_shape(const Dbn2plArgs &a) {
+    WalkShape w;
+    const long cells = (long)a.n_mtot * a.n_mrat;
+    w.qc = (int)std::max(1L, std::min(8L, std::min((long)a.n_mrat, hgb::ceil_div(cells, 8L * hgb::sm_count()))));
+    w.cb = std::max(1, std::min(w.qc, WK_THREADS / a.n_redz));
+    w.rows = std::min(WK_THREADS, w.cb * a.n_redz);
+    const size_t row_bytes = sizeof(unsigned) * wk_stride(a.n_freq);
+    w.rows = std::max(1, std::min<int>(w.rows, (int)(48 * 1024 / row_bytes)));
+    const size_t nodes = (size_t)a.num_steps + 1;
+    w.smem = sizeof(double) * (3 * (size_t)a.n_interp + a.n_freq + a.n_redz + 3 * nodes + w.rows + w.qc * nodes) +
+             sizeof(float) * (3 * (size_t)a.n_interp + a.n_freq + nodes) + row_bytes * w.rows;
+    return w;
+}
+
 // Phase 2 of the Fixed_Time_2PL_SAM number: every (redz, frequency) element of a (mtot, mrat) cell
 // whose target was bracketed (sam_cyutils.pyx:731-768).  One block per cell, so the cell's
 // constant powers are taken once and the elements run without divergence.
@@ -712,16 +1034,6 @@ __global__ void __launch_bounds__(GW_ROWS) k_dbn_gw(CyConst cc, const double *__
 constexpr int NB_STEPS = 320;   // steps the kernel holds in registers
 
 
-// y^p of the hardening shape's outer factor, y = 1 + x: a planned negative (half-)integer power from one
-// reciprocal square root, any other exponent as pow_planned
-__device__ __forceinline__ double shape_outer(double y, double p, PowPlan plan) {
-    if (plan.kind == 0 || !plan.neg || !hgb::fast_range(y)) return pow_planned(y, p, plan);
-    const double r = hgb::fast_rsqrt(y), r2 = r * r;
-    double v = plan.kind == 2 ? r : 1.0;
-    for (int i = 0; i < plan.n; i++) v *= r2;
-    return v;
-}
-
 template <int CPW>
 __global__ void __launch_bounds__(32) k_hardening_norm_sub(CyConst cc, NormArgs a, const double *__restrict__ mtot,
                                                            const double *__restrict__ mrat, int n,
@@ -928,25 +1240,39 @@ int hgb_dbn_2pwl_phase(const double *fobs_orb, int n_freq, int fobs_sorted, doub
                  pow_plan(gamma_inner - 1.0)};
     unsigned blocks = (unsigned)((long)n_mtot * n_mrat);
     if (phase & 1) {
-        // cells per block: fill up to 512 rows (cpb x n_redz), within a shared-memory budget
-        const size_t base = sizeof(double) * ((size_t)4 * cosmo->grid_size + n_freq);
-        const size_t per_cell = sizeof(double) * (3 * (size_t)(num_steps + 1) + 2 * (size_t)num_steps);
-        HGB_CHECK_ARG(base + per_cell <= 200 * 1024);
-        int cpb = 512 / n_redz;
-        cpb = std::min<long>(cpb, (long)((160 * 1024 - std::min<size_t>(base, 160 * 1024)) / per_cell));
-        cpb = std::max(1, std::min(cpb, WALK_MAX_CELLS));
-        const size_t smem = base + per_cell * cpb;
-        int src = hgb::ensure_dyn_smem((const void *)k_dbn_2pwl, smem);
-        if (src) return src;
-        int threads = (int)hgb::ceil_div((long)cpb * n_redz, 32) * 32;
-        if (threads > 512) threads = 512;
-        const unsigned wblocks = (unsigned)hgb::ceil_div((long)n_mtot * n_mrat, cpb);
-        k_dbn_2pwl<<<wblocks, threads, smem, (cudaStream_t)stream>>>(hgb::cy_const(), a, cpb, fobs_orb, hard_norm, nden,
-                                                                    mtot, mrat, redz, gmt_time, cosmo->grid_z,
-                                                                    cosmo->grid_age, cosmo->grid_dcom, redz_final,
-                                                                    diff_num);
-        int rc = hgb::check_launch();
-        if (rc) return rc;
+        const WalkShape ws = walk_shape(a);
+        // ascending targets, step and interval numbers that fit the walk's 16-bit notes, and tables that
+        // fit one SM; any other call takes the FP64 walk
+        if (fobs_sorted && num_steps < 0xFFFF && cosmo->grid_size < 0xFFFF && ws.smem <= 200 * 1024) {
+            const int wrc = hgb::ensure_dyn_smem((const void *)k_dbn_2pwl_walk, ws.smem);
+            if (wrc) return wrc;
+            const unsigned wb = (unsigned)((long)n_mtot * hgb::ceil_div(n_mrat, ws.qc));
+            k_dbn_2pwl_walk<<<wb, WK_THREADS, ws.smem, (cudaStream_t)stream>>>(
+                hgb::cy_const(), a, ws, fobs_orb, hard_norm, mtot, mrat, redz, gmt_time, cosmo->grid_z,
+                cosmo->grid_age, redz_final, diff_num);
+            const int rc = hgb::check_launch();
+            if (rc) return rc;
+        } else {
+            // cells per block: fill up to 512 rows (cpb x n_redz), within a shared-memory budget
+            const size_t base = sizeof(double) * ((size_t)4 * cosmo->grid_size + n_freq);
+            const size_t per_cell = sizeof(double) * (3 * (size_t)(num_steps + 1) + 2 * (size_t)num_steps);
+            HGB_CHECK_ARG(base + per_cell <= 200 * 1024);
+            int cpb = 512 / n_redz;
+            cpb = std::min<long>(cpb, (long)((160 * 1024 - std::min<size_t>(base, 160 * 1024)) / per_cell));
+            cpb = std::max(1, std::min(cpb, WALK_MAX_CELLS));
+            const size_t smem = base + per_cell * cpb;
+            int src = hgb::ensure_dyn_smem((const void *)k_dbn_2pwl, smem);
+            if (src) return src;
+            int threads = (int)hgb::ceil_div((long)cpb * n_redz, 32) * 32;
+            if (threads > 512) threads = 512;
+            const unsigned wblocks = (unsigned)hgb::ceil_div((long)n_mtot * n_mrat, cpb);
+            k_dbn_2pwl<<<wblocks, threads, smem, (cudaStream_t)stream>>>(hgb::cy_const(), a, cpb, fobs_orb, hard_norm, nden,
+                                                                        mtot, mrat, redz, gmt_time, cosmo->grid_z,
+                                                                        cosmo->grid_age, cosmo->grid_dcom, redz_final,
+                                                                        diff_num);
+            int rc = hgb::check_launch();
+            if (rc) return rc;
+        }
     }
     if (phase & 2) {
         size_t smem2 = sizeof(double) * ((size_t)5 * cosmo->grid_size + n_freq);
