@@ -81,6 +81,13 @@ def comoving_distance_table(cosmo, n=_DC_TABLE_N):
     return val, der
 
 
+def distance_cubics(val, der, n=_DC_TABLE_N):
+    """Coefficients (n, 4), lowest power first, of each interval's Hermite cubic in t = u n - k."""
+    m0, m1, d = der[:-1] / n, der[1:] / n, np.diff(val)
+    c3 = (m0 + m1) - 2.0 * d
+    return np.stack([val[:-1], m0, d - m0 - c3, c3], axis=1)
+
+
 def distance_ratio_table(cosmo, val, der, n=_DC_TABLE_N):
     """The FP32 entry points' distance table: g(u) = D_C(u) / (D_H (1 - u)) and dg/du on u = k/n, from
     the FP64 values and derivatives of :func:`comoving_distance_table`.  At u = 1 (z = 0) g is the
@@ -109,6 +116,7 @@ class DeviceCosmology:
         val, der = comoving_distance_table(cosmo)
         self.dc_val = as_device(val, dev)
         self.dc_der = as_device(der, dev)
+        self.dc_cub = as_device(distance_cubics(val, der), dev)
         gv, gd = distance_ratio_table(cosmo, val, der)
         t = torch()
         self.dcg_val = as_device(gv, dev, dtype=t.float32)
@@ -131,6 +139,7 @@ class DeviceCosmology:
         s.dc_n = _DC_TABLE_N
         s.dcg_val = N.ptr(self.dcg_val)
         s.dcg_der = N.ptr(self.dcg_der)
+        s.dc_cub = N.ptr(self.dc_cub)
         self.struct = s
         # cached and used from every stream: the uploads are complete before the cache hands it out
         t.cuda.current_stream(device(dev)).synchronize()

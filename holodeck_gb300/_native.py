@@ -55,6 +55,7 @@ class HgbCosmo(ctypes.Structure):
         ("age_limit", _d), ("hubble_distance", _d),
         ("grid_z", _p), ("grid_age", _p), ("grid_dcom", _p), ("grid_size", _i),
         ("dc_val", _p), ("dc_der", _p), ("dc_n", _i), ("dcg_val", _p), ("dcg_der", _p),
+        ("dc_cub", _p),
     ]
 
 

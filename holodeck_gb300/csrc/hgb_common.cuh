@@ -149,6 +149,15 @@ __device__ __forceinline__ float f64_to_f32_rz(double x) {
     return __uint_as_float(sign | ((unsigned)e << 23) | ((hi & 0xFFFFFu) << 3) | (lo >> 29));
 }
 
+// x rounded to the nearest float, ties to even, for a positive x in the range of normal floats: the
+// hardware conversion's result without the FP64 pipe
+__device__ __forceinline__ float f64_to_f32_rn_normal(double x) {
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const unsigned f = ((hi - (896u << 20)) << 3) | (lo >> 29);           // truncated; 896 = 1023 - 127
+    const unsigned rest = lo & 0x1FFFFFFFu;                               // what is cut off, in units of 2^-29
+    return __uint_as_float(f + (rest > 0x10000000u - (f & 1u) ? 1u : 0u));   // a carry runs into the exponent
+}
+
 // v * 2^k as a double, exactly, for a float v that is zero, normal, inf or NaN (a subnormal v gives
 // a signed zero); |k| must keep the result inside the double range.
 __device__ __forceinline__ double f32_to_f64_scaled(float v, int k) {

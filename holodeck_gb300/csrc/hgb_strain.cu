@@ -1,12 +1,11 @@
 // Cell integration and per-bin strain on the (M-1, Q-1, Z-1, F) bin grid (kernel k_cells):
 //  * NUMBER: integrate_differential_number_3dx1d (holodeck/sams/sam_cyutils.pyx:115-216)
 //  * STRAIN: char_strain_sq_from_bin_edges_redz (holodeck/gravwaves.py:694-724)
-//  * both in one pass for gwb() (sam.py:930-935): each vertex of dnum and redz_final is read from
-//    L1/L2 by the eight bins that share it, and number / h2fdf are written once.
-// One block per (mtot, mrat) cell; its threads walk the (redz, frequency) elements with the
-// frequency fastest, so the eight vertex loads of a warp are contiguous runs along the frequency
-// axis.  Built with -fmad=false: the eight-vertex sum and the midpoints round like the Cython/numpy
-// code; the strain product is regrouped (see cell_strain), which moves it by a few ulp.
+//  * both in one pass for gwb() (sam.py:930-935): each vertex of dnum and redz_final is read by the four
+//    (mtot, mrat) cells that share it, and number / h2fdf are written once.
+// One block per (mtot, mrat) cell, the frequency fastest over its threads.  Built with -fmad=false: the
+// eight-vertex sum and the midpoints round like the Cython/numpy code; the strain product is regrouped
+// (see bin_strain), which moves it by a few ulp.
 #include <math.h>
 
 #include "hgb_common.cuh"
@@ -21,104 +20,141 @@ __device__ __forceinline__ long vtx(const BinGeom &g, int m, int q, int z, int f
     return (((long)m * g.nq + q) * g.nz + z) * g.nf + f;
 }
 
-// sam_cyutils.pyx:199-214
-__device__ __forceinline__ double cell_number(const BinGeom &g, const double *dnum, int m, int q, int z, int f,
-                                              const double *log10_mtot, const double *mrat, const double *redz,
-                                              const double *dln_freq) {
-    double dm = log10_mtot[m + 1] - log10_mtot[m];
-    double dmdq = dm * (mrat[q + 1] - mrat[q]);
-    double dmdqdz = dmdq * (redz[z + 1] - redz[z]);
-    double temp = 0.0;
-#pragma unroll
-    for (int ii = 0; ii < 2; ii++)
-#pragma unroll
-        for (int jj = 0; jj < 2; jj++)
-#pragma unroll
-            for (int kk = 0; kk < 2; kk++) temp += dnum[vtx(g, m + ii, q + jj, z + kk, f)];
-    return temp * dmdqdz * dln_freq[f] / 8.0;
-}
-
 struct StrainArgs {
     double gw_src_const;
     const double *dc_val, *dc_der;
-    int dc_n;
-    double dc_h;   // 1 / dc_n
+    const double2 *dc_cub;   // [dc_n][2] cubic coefficients (may be null)
+    int dc_n, dc_log2;       // dc_log2: log2 of a power of two dc_n up to 2^20, -1 otherwise
+    double dc_h;             // 1 / dc_n
 };
 
-// gravwaves.py:694-724 rearranged: hs = K mc (2 mc fr)^(2/3) / dc with fr = fc (1 + zbar) is evaluated
-// as [K mc (2 mc)^(2/3)] [fc^(2/3)] [(1 + zbar)^(2/3)] / dc, the first factor once per (mtot, mrat)
-// cell and the second once per frequency, so each (bin, frequency) costs one inverse cube root (an
-// FP32 estimate and one FP64 Newton step) and the comoving-distance lookup.  The redshift midpoints are taken along mtot, then mrat, then redz.
-__device__ __forceinline__ double cell_strain(const BinGeom &g, const double *rz, int m, int q, int z, int f,
-                                              double amp_mq, double amp_f, double fc_df, const StrainArgs &s,
-                                              int *d_status) {
-    double r[2][2][2];
-#pragma unroll
-    for (int ii = 0; ii < 2; ii++)
-#pragma unroll
-        for (int jj = 0; jj < 2; jj++)
-#pragma unroll
-            for (int kk = 0; kk < 2; kk++) {
-                double v = rz[vtx(g, m + ii, q + jj, z + kk, f)];
-                if (v < 0.0 && v != -1.0) hgb::flag(d_status, HGB_STATUS_INVALID_REDSHIFT);
-                r[ii][jj][kk] = v;
-            }
-    double a00 = 0.5 * (r[1][0][0] + r[0][0][0]);
-    double a01 = 0.5 * (r[1][0][1] + r[0][0][1]);
-    double a10 = 0.5 * (r[1][1][0] + r[0][1][0]);
-    double a11 = 0.5 * (r[1][1][1] + r[0][1][1]);
-    double b0 = 0.5 * (a10 + a00);
-    double b1 = 0.5 * (a11 + a01);
-    double zb = 0.5 * (b1 + b0);
-    if (!(zb > 0.0)) return 0.0;   // +inf comoving distance: zero strain
-    double dc = hgb::comoving_distance_fast(s.dc_val, s.dc_der, s.dc_n, s.dc_h, zb);
-    double zp1 = 1.0 + zb;
-    // (1 + z)^(2/3) = (1 + z) r with r = (1 + z)^(-1/3): FP32 start, one Newton step for the inverse
-    // cube root, r (4 - y r^3) / 3, in FP64 (relative error about 1e-14; 1 + z lies in (1, 12));
-    // 1 / dc likewise, q (2 - dc q) from an FP32 reciprocal
-    const double r0 = (double)rcbrtf((float)zp1);
-    const double r1 = r0 * (4.0 - zp1 * (r0 * r0 * r0)) * (1.0 / 3.0);
-    const double q0 = (double)__frcp_rn((float)dc);
-    const double q1 = q0 * (2.0 - dc * q0);
-    double hs = amp_mq * amp_f * (zp1 * r1) * q1;
+StrainArgs strain_args(double k, const hgb_cosmo *c) {
+    StrainArgs s{k, c->dc_val, c->dc_der, (const double2 *)c->dc_cub, c->dc_n, -1, 1.0 / c->dc_n};
+    if ((c->dc_n & (c->dc_n - 1)) == 0 && c->dc_n <= (1 << 20)) {
+        s.dc_log2 = 0;
+        while ((1 << s.dc_log2) < c->dc_n) s.dc_log2++;
+    }
+    return s;
+}
+
+// Comoving distance at y = 1 + z > 1.  u = y^(-1/2) is an FP32 estimate with one FP64 Newton step, as in
+// comoving_distance_fast and with its bits (near z = 0 the distance is the small 1 - u, so another
+// rounding there would show); the interval comes from u's bits, its cubic from the table.
+__device__ __forceinline__ double distance_at(const StrainArgs &s, double y) {
+    const float u0f = rsqrtf(hgb::f64_to_f32_rn_normal(y));
+    const double u0 = hgb::f32_to_f64_scaled(u0f, 0), half = hgb::f32_to_f64_scaled(u0f, -1);
+    const double u = half * (3.0 - y * (u0 * u0));
+    // k = floor(u 2^L), at most 2^L - 1, from the bits of u in (0, 1 + 1e-14)
+    const unsigned hi = (unsigned)__double2hiint(u);
+    const int sh = 1023 - (int)(hi >> 20) - s.dc_log2;   // u 2^L = 1.m 2^-sh
+    int k = sh > 0 ? 0 : (int)(((hi & 0xFFFFFu) | 0x100000u) >> (20 + sh));
+    k = min(k, s.dc_n - 1);
+    const double t = __fma_rn(u, (double)s.dc_n, -hgb::f32_to_f64_scaled((float)k, 0));   // exact product
+    const double2 c01 = __ldg(s.dc_cub + 2 * k), c23 = __ldg(s.dc_cub + 2 * k + 1);
+    return __fma_rn(__fma_rn(__fma_rn(c23.y, t, c23.x), t, c01.y), t, c01.x);
+}
+
+// gravwaves.py:694-724 on a bin with midpoint redshift z > 0, y = 1 + z, rearranged:
+// hs = K mc (2 mc fr)^(2/3) / dc with fr = fc y is [K mc (2 mc)^(2/3) fc^(2/3)] y^(2/3) / dc, the first
+// factor (amp) once per (mtot, mrat) cell and frequency.  y^(2/3) = y y^(-1/3), an FP32 cube root with one
+// third-order step.
+__device__ __forceinline__ double bin_strain(const StrainArgs &s, double z, double y, double amp, double fc_df) {
+    const bool table = s.dc_cub && s.dc_log2 >= 0 && __double2hiint(y) < (1023 + 100) << 20;   // an infinite z: as before
+    const double dc = table ? distance_at(s, y) : hgb::comoving_distance_fast(s.dc_val, s.dc_der, s.dc_n, s.dc_h, z);
+    const double r0 = hgb::f32_to_f64_scaled(rcbrtf(hgb::f64_to_f32_rz(y)), 0);
+    const double yr = y * r0;
+    const double e = __fma_rn(-yr, r0 * r0, 1.0);   // 1 - y r0^3, a few 1e-7
+    const double y23 = __fma_rn(yr * e, __fma_rn(2.0 / 9.0, e, 1.0 / 3.0), yr);
+    const double inv = hgb::fast_range(dc) ? hgb::fast_rcp(dc) : 1.0 / dc;
+    const double hs = amp * y23 * inv;
     return (hs * hs) * fc_df;
 }
 
-// One block per (mtot, mrat) bin cell; threads stride over its (redz, frequency) elements.
+// One block per (mtot, mrat) bin cell.  A thread keeps one frequency (the threads' fastest index, so a
+// warp's loads and stores are contiguous) and walks a run of redshifts, taking each vertex plane's values
+// from memory once:
+//   * the eight-vertex sum of the number keeps the reference's order, bit for bit;
+//   * the strain's midpoints are taken along mtot, then mrat, then redz; halving is exact, so the sums
+//     of a plane serve both of its bins and 1 + zb is one multiply-add.
+// The sentinel and sign tests read the values' bits: an FP64 comparison holds the pipe as long as a
+// product.  9 and 26 FP64 operations an element where 16 and some 55 were, and FP64 bounds it.
+// 67 x 59 x 83 edges, 37 frequencies: number 305 us before, 263 us now, strain 1593 and 504 us;
+// both together (gwb), 41 x 31 x 37, 20 frequencies: 148 and 72 us.
+constexpr int CELL_THREADS = 256;
+
 template <bool NUMBER, bool STRAIN>
-__global__ void k_cells(BinGeom g, StrainArgs s, const double *__restrict__ mtot, const double *__restrict__ log10_mtot,
+__global__ void __launch_bounds__(CELL_THREADS) k_cells(BinGeom g, StrainArgs s, const double *__restrict__ mtot, const double *__restrict__ log10_mtot,
                         const double *__restrict__ mrat, const double *__restrict__ redz,
                         const double *__restrict__ fedges, const double *__restrict__ dln_freq,
                         const double *__restrict__ dnum, const double *__restrict__ redz_final,
                         double *__restrict__ number, double *__restrict__ h2fdf, int *d_status) {
-    extern __shared__ double sm[];
-    double *amp_f = sm;              // [nf] fc^(2/3)
-    double *fc_df = sm + g.nf;       // [nf] fc / df
-    __shared__ double amp_mq;
     const int cell = blockIdx.x;
     const int m = cell / (g.nq - 1), q = cell % (g.nq - 1);
+    const int fb = min(g.nf, CELL_THREADS);        // frequencies side by side
+    const int runs = CELL_THREADS / fb;            // redshift runs side by side
+    const int nzb = g.nz - 1, zlen = (nzb + runs - 1) / runs;
+    const int run = threadIdx.x / fb, z0 = run * zlen, z1 = min(z0 + zlen, nzb);
+    __shared__ double amp_mq;
     if (STRAIN) {
-        for (int f = threadIdx.x; f < g.nf; f += blockDim.x) {
-            double fc = 0.5 * (fedges[f + 1] + fedges[f]);
-            double df = fedges[f + 1] - fedges[f];
-            amp_f[f] = pow(fc, 2.0 / 3.0);
-            fc_df[f] = fc / df;
-        }
         if (threadIdx.x == 0) {
-            double mt = 0.5 * (mtot[m + 1] + mtot[m]);
-            double mr = 0.5 * (mrat[q + 1] + mrat[q]);
-            double mc = mt * pow(mr, 3.0 / 5.0) / pow(1.0 + mr, 6.0 / 5.0);
-            amp_mq = s.gw_src_const * mc * pow(2.0 * mc, 2.0 / 3.0);
+            // K mc (2 mc)^(2/3) with mc^(5/3) = mt^(5/3) mr / (1 + mr)^2
+            const double mt = 0.5 * (mtot[m + 1] + mtot[m]);
+            const double mr = 0.5 * (mrat[q + 1] + mrat[q]);
+            const double c = cbrt(mt), opq = 1.0 + mr;
+            amp_mq = s.gw_src_const * 1.5874010519681994748 * (mt * (c * c) * mr / (opq * opq));   // 2^(2/3)
         }
         __syncthreads();
     }
-    const int nzf = (g.nz - 1) * g.nf;
-    const long out0 = (long)cell * nzf;
-    for (int e = threadIdx.x; e < nzf; e += blockDim.x) {
-        int z = e / g.nf, f = e % g.nf;
-        if (NUMBER) number[out0 + e] = cell_number(g, dnum, m, q, z, f, log10_mtot, mrat, redz, dln_freq);
-        if (STRAIN) h2fdf[out0 + e] = cell_strain(g, redz_final, m, q, z, f, amp_mq, amp_f[f], fc_df[f], s, d_status);
+    if (run >= runs) return;
+    double dmdq = 0.0;
+    if (NUMBER) dmdq = (log10_mtot[m + 1] - log10_mtot[m]) * (mrat[q + 1] - mrat[q]);
+    const long plane = (long)g.nq * g.nz * g.nf, row = (long)g.nz * g.nf;   // steps along mtot, mrat
+    bool bad = false;
+    for (int f = threadIdx.x - run * fb; f < g.nf; f += fb) {
+        double amp = 0.0, fc_df = 0.0, dlnf8 = 0.0;
+        if (STRAIN) {
+            const double fc = 0.5 * (fedges[f + 1] + fedges[f]);
+            const double c = cbrt(fc);
+            amp = amp_mq * (c * c);
+            fc_df = fc / (fedges[f + 1] - fedges[f]);
+        }
+        if (NUMBER) dlnf8 = dln_freq[f] * 0.125;
+        double n00 = 0.0, n01 = 0.0, n10 = 0.0, n11 = 0.0, below = 0.0;   // the lower plane's values, its redshift sum
+        for (int z = z0; z <= z1 && z0 < z1; z++) {
+            const long v = vtx(g, m, q, z, f);
+            const long out = ((long)cell * nzb + (z - 1)) * g.nf + f;
+            const bool bin = z > z0;   // vertex z closes bin z - 1
+            if (NUMBER) {
+                const double u00 = dnum[v], u01 = dnum[v + row], u10 = dnum[v + plane], u11 = dnum[v + plane + row];
+                if (bin) {   // sam_cyutils.pyx:199-214; the division by 8 is exact wherever it is taken
+                    const double sum = ((((((n00 + u00) + n01) + u01) + n10) + u10) + n11) + u11;
+                    const double vol = dmdq * (redz[z] - redz[z - 1]);
+                    number[out] = sum * vol * dlnf8;
+                }
+                n00 = u00; n01 = u01; n10 = u10; n11 = u11;
+            }
+            if (STRAIN) {
+                const double r00 = redz_final[v], r01 = redz_final[v + row];
+                const double r10 = redz_final[v + plane], r11 = redz_final[v + plane + row];
+                const long long b4[4] = {__double_as_longlong(r00), __double_as_longlong(r01),
+                                         __double_as_longlong(r10), __double_as_longlong(r11)};
+#pragma unroll
+                for (int c = 0; c < 4; c++)   // below 0 and not -1 (and no -0, no NaN)
+                    bad |= b4[c] < 0 && b4[c] != hgb::F64_MINUS_ONE_BITS && b4[c] != (long long)0x8000000000000000ull &&
+                           (unsigned long long)b4[c] <= 0xFFF0000000000000ull;
+                const double above = (r11 + r01) + (r10 + r00);
+                if (bin) {
+                    const double sum = above + below;   // 8 zb
+                    const long long bits = __double_as_longlong(sum);
+                    // zb <= 0 or NaN: infinite comoving distance, zero strain
+                    h2fdf[out] = (bits > 0 && bits <= 0x7FF0000000000000ll)
+                                     ? bin_strain(s, 0.125 * sum, __fma_rn(0.125, sum, 1.0), amp, fc_df) : 0.0;
+                }
+                below = above;
+            }
+        }
     }
+    if (STRAIN && bad) hgb::flag(d_status, HGB_STATUS_INVALID_REDSHIFT);
 }
 
 // ---- FP32 production mode of k_cells<true, true>
@@ -266,7 +302,7 @@ __global__ void k_cells_f32(BinGeom g, StrainArgs32 s, double amp_scale, const d
 }
 
 // single_sources.py:117-143 on one (bin, frequency): the redshift midpoints (same order as
-// cell_strain), -1 where not positive; comoving distance (+inf there); Kepler separation at the
+// k_cells), -1 where not positive; comoving distance (+inf there); Kepler separation at the
 // rest-frame orbital frequency; angular separation.  IEEE semantics give the reference's inf / NaN
 // for the -1 bins.  Also records the largest finite magnitude of each grid (as a frexp exponent)
 // over the bins with nonzero strain.
@@ -333,7 +369,7 @@ int hgb_param_grids(const double *mt_cent, int n_mtot, int n_mrat, int n_redz, c
     HGB_CHECK_ARG(n_mtot >= 2 && n_mrat >= 2 && n_redz >= 2 && n_freq >= 1);
     HGB_CHECK_ARG(cosmo->dc_val && cosmo->dc_der && cosmo->dc_n >= 2);
     BinGeom g{n_mtot, n_mrat, n_redz, n_freq};
-    StrainArgs s{0.0, cosmo->dc_val, cosmo->dc_der, cosmo->dc_n, 1.0 / cosmo->dc_n};
+    const StrainArgs s = strain_args(0.0, cosmo);
     cudaStream_t st = (cudaStream_t)stream;
     if (scale_log2) {
         cudaError_t err = cudaMemsetAsync(scale_log2, 0x80, 4 * sizeof(int), st);   // very negative
@@ -354,9 +390,9 @@ int hgb_integrate_3dx1d(const double *log10_mtot, int n_mtot, const double *mrat
     HGB_CHECK_ARG(log10_mtot && mrat && redz && dln_freq && dnum && number);
     HGB_CHECK_ARG(n_mtot >= 2 && n_mrat >= 2 && n_redz >= 2 && n_freq >= 1);
     BinGeom g{n_mtot, n_mrat, n_redz, n_freq};
-    StrainArgs s{0.0, nullptr, nullptr, 0, 0.0};
+    const StrainArgs s{0.0, nullptr, nullptr, nullptr, 0, -1, 0.0};
     unsigned cells = (unsigned)((n_mtot - 1) * (n_mrat - 1));
-    k_cells<true, false><<<cells, 256, 0, (cudaStream_t)stream>>>(g, s, nullptr, log10_mtot, mrat, redz, nullptr,
+    k_cells<true, false><<<cells, CELL_THREADS, 0, (cudaStream_t)stream>>>(g, s, nullptr, log10_mtot, mrat, redz, nullptr,
                                                                   dln_freq, dnum, nullptr, number, nullptr, nullptr);
     return hgb::check_launch();
 }
@@ -368,11 +404,9 @@ int hgb_char_strain_sq(const double *mtot, int n_mtot, const double *mrat, int n
     HGB_CHECK_ARG(n_mtot >= 2 && n_mrat >= 2 && n_redz >= 2 && n_freq >= 1);
     HGB_CHECK_ARG(cosmo->dc_val && cosmo->dc_der && cosmo->dc_n >= 2);
     BinGeom g{n_mtot, n_mrat, n_redz, n_freq};
-    StrainArgs s{gw_src_const, cosmo->dc_val, cosmo->dc_der, cosmo->dc_n, 1.0 / cosmo->dc_n};
+    const StrainArgs s = strain_args(gw_src_const, cosmo);
     unsigned cells = (unsigned)((n_mtot - 1) * (n_mrat - 1));
-    size_t smem = sizeof(double) * 2 * n_freq;
-    HGB_CHECK_ARG(smem <= 48 * 1024);
-    k_cells<false, true><<<cells, 256, smem, (cudaStream_t)stream>>>(g, s, mtot, nullptr, mrat, nullptr, fobs_orb_edges,
+    k_cells<false, true><<<cells, CELL_THREADS, 0, (cudaStream_t)stream>>>(g, s, mtot, nullptr, mrat, nullptr, fobs_orb_edges,
                                                                      nullptr, nullptr, redz_final, nullptr, h2fdf,
                                                                      d_status);
     return hgb::check_launch();
@@ -408,11 +442,9 @@ int hgb_number_and_strain(const double *mtot, const double *log10_mtot, int n_mt
     HGB_CHECK_ARG(n_mtot >= 2 && n_mrat >= 2 && n_redz >= 2 && n_freq >= 1);
     HGB_CHECK_ARG(cosmo->dc_val && cosmo->dc_der && cosmo->dc_n >= 2);
     BinGeom g{n_mtot, n_mrat, n_redz, n_freq};
-    StrainArgs s{gw_src_const, cosmo->dc_val, cosmo->dc_der, cosmo->dc_n, 1.0 / cosmo->dc_n};
+    const StrainArgs s = strain_args(gw_src_const, cosmo);
     unsigned cells = (unsigned)((n_mtot - 1) * (n_mrat - 1));
-    size_t smem = sizeof(double) * 2 * n_freq;
-    HGB_CHECK_ARG(smem <= 48 * 1024);
-    k_cells<true, true><<<cells, 256, smem, (cudaStream_t)stream>>>(g, s, mtot, log10_mtot, mrat, redz, fobs_orb_edges,
+    k_cells<true, true><<<cells, CELL_THREADS, 0, (cudaStream_t)stream>>>(g, s, mtot, log10_mtot, mrat, redz, fobs_orb_edges,
                                                                     dln_freq, dnum, redz_final, number, h2fdf, d_status);
     return hgb::check_launch();
 }

@@ -73,6 +73,9 @@ typedef struct {
      * g (dimensionless) and dg/du on the same nodes u = k / dc_n, cubic Hermite between them */
     const float *dcg_val;   /* [dc_n + 1] */
     const float *dcg_der;   /* [dc_n + 1] */
+    /* the Hermite cubics of dc_val / dc_der as polynomials in t = u dc_n - k, lowest power first (16-byte
+     * aligned; may be NULL: formed from dc_val / dc_der where they are used) */
+    const double *dc_cub;   /* [dc_n][4] */
 } hgb_cosmo;
 
 /* Galaxy / black-hole population model (holodeck/sams/components.py, host_relations.py). */
