@@ -9,7 +9,7 @@
 // accumulated in fp32.
 //
 // All three contractions (forward Y = X W^T, input gradient dX = dZ W, weight gradient
-// dW = dZ^T X) run on the tensor cores the same way: a CTA of 128 threads owns a 128-row output tile
+// dW = dZ^T X) run on the tensor cores the same way: a CTA of 256 threads owns a 128-row output tile
 // of NT columns in tensor memory (tcgen05.alloc, fp32 accumulators), stages the operands in shared
 // memory in the canonical no-swizzle K-major layout (8 x 16-byte core matrices), one elected thread
 // issues tcgen05.mma (kind::f16, bf16 x bf16 -> fp32, M = 128, K = 16 per instruction) and commits
@@ -19,10 +19,10 @@
 //     accelerator (cp.async.bulk.tensor, one box of 8 columns per K-group) against an mbarrier;
 //     the whole reduction axis (<= 256) at once, output columns split 64 per CTA, so a layer is one
 //     copy / MMA / read-back round trip on (row tiles x column tiles x members) CTAs.
-//   * Input and weight gradients (k_mlp_gemm<DxOp / DwOp>): one operand is read transposed (a column
-//     gather of a row-major buffer), so the threads stage both operands through registers; the input
-//     gradient stages the whole reduction axis with columns split 64 per CTA, the weight gradient
-//     keeps all columns in one CTA and reduces one 128-row batch split per CTA.
+//   * Input and weight gradients (k_mlp_bwd, one launch per layer for both): operands that lie
+//     transposed in memory are staged through registers by 8 x 8 blocks; the input gradient stages the
+//     whole reduction axis with columns split 64 per CTA, the weight gradient reduces one 128-row batch
+//     split per CTA, also 64 columns wide.
 // Every wait is bounded: on expiry the kernel flags HGB_STATUS_ITERATION_LIMIT, frees its tensor
 // memory and returns.
 //
@@ -50,7 +50,7 @@ typedef __nv_bfloat16 bf16;
 
 constexpr int TM = 128;            // output rows per CTA (tcgen05 M)
 constexpr int NMAX = 256;          // widest layer (tcgen05 N limit for M = 128)
-constexpr int THREADS = 128;
+constexpr int LAYER_THREADS = 256;         // eight warps stage a layer's tile and share its epilogue
 constexpr int SMEM_DYN = 100 * 1024;       // holds both staged slices; caps residency at two CTAs per SM
 constexpr uint64_t WAIT_NS = 1000000000ull;   // a wait for the tensor core gives up after 1 s
 constexpr int WIDTH = 256;                 // row stride (elements) of the hidden activation buffers
@@ -157,6 +157,15 @@ union Pack8 {
     bf16 h[8];
 };
 
+// eight consecutive values, in one access where the buffer allows it
+__device__ __forceinline__ uint4 load8(const bf16 *p, bool aligned) {
+    if (aligned) return *(const uint4 *)p;
+    Pack8 v;
+#pragma unroll
+    for (int i = 0; i < 8; i++) v.h[i] = p[i];
+    return v.u;
+}
+
 // ---- epilogues of the three contractions and the gradients' operand loaders -------------------------
 // A loader: 8 consecutive reduction entries of output row r; B loader: the same for output column n.
 // Both return zeros outside the operands.
@@ -211,39 +220,43 @@ struct FwdOp {   // epilogue of the forward: Y[b][n] = act(acc + bias[n]) (opera
 
 struct DxOp {   // dZprev[b][k] = (sum_n dZ[b][n] W[n][k]) * silu'(Zprev[b][k])
     static constexpr int KC = 256, NT = 64;
-    static constexpr bool COL_TILED = true;
     const bf16 *dz;    // [b][WIDTH], reduction over its first N columns
     long dz_es;
     const bf16 *w;     // [N][K]
     long w_es;
+    bool w_aligned;    // every member's weights start on 16 bytes
     const float *pre;  // Zprev [b][WIDTH]
     long pre_es;
     bf16 *dzp;         // dZprev [b][WIDTH]
     long dzp_es;
     int K, N, batch;
 
-    __device__ int red() const { return N; }
-    __host__ __device__ int ncols() const { return K; }
     __device__ uint4 load_a(int e, int row, int n) const {
         if (row >= batch || n >= N) return make_uint4(0, 0, 0, 0);
         return *(const uint4 *)(dz + e * dz_es + (long)row * WIDTH + n);
     }
-    __device__ uint4 load_b(int e, int k, int n) const {
-        Pack8 p;
-        const bf16 *wp = w + e * w_es + k;
-#pragma unroll
-        for (int j = 0; j < 8; j++)
-            p.h[j] = (k < K && n + j < N) ? wp[(long)(n + j) * K] : __float2bfloat16_rn(0.0f);
-        return p.u;
+    // row n + j of W, columns k .. k + 7: block (k, n) of the transposed operand
+    __device__ uint4 row_b(int e, int k, int n, int j) const {
+        if (k >= K || n + j >= N) return make_uint4(0, 0, 0, 0);
+        return load8(w + e * w_es + (long)(n + j) * K + k, w_aligned);
     }
     __device__ void store(int e, int row, int k0, const float (&v)[16]) const {
         if (row >= batch || k0 >= K) return;
-        const float *zp = pre + e * pre_es + (long)row * WIDTH + k0;
+        const float4 *zp = (const float4 *)(pre + e * pre_es + (long)row * WIDTH + k0);
+        float z[16];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const float4 q = zp[i];
+            z[4 * i] = q.x;
+            z[4 * i + 1] = q.y;
+            z[4 * i + 2] = q.z;
+            z[4 * i + 3] = q.w;
+        }
         Pack8 p0, p1;
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            p0.h[i] = __float2bfloat16_rn(v[i] * silu_grad(zp[i]));
-            p1.h[i] = __float2bfloat16_rn(v[i + 8] * silu_grad(zp[i + 8]));
+            p0.h[i] = __float2bfloat16_rn(v[i] * silu_grad(z[i]));
+            p1.h[i] = __float2bfloat16_rn(v[i + 8] * silu_grad(z[i + 8]));
         }
         uint4 *d = (uint4 *)(dzp + e * dzp_es + (long)row * WIDTH + k0);
         d[0] = p0.u;
@@ -252,43 +265,29 @@ struct DxOp {   // dZprev[b][k] = (sum_n dZ[b][n] W[n][k]) * silu'(Zprev[b][k])
 };
 
 struct DwOp {   // part[s][n][k] = sum over this split's rows b of dZ[b][n] X[b][k]
-    static constexpr int KC = HGB_MLP_SPLIT_ROWS, NT = NMAX;
-    static constexpr bool COL_TILED = false;   // blockIdx.y is the batch split
+    static constexpr int KC = HGB_MLP_SPLIT_ROWS, NT = 64;
     const bf16 *dz;    // [b][WIDTH]
     long dz_es;
     const bf16 *x;     // layer input [b][ldx]
     long x_es;
     int ldx;
+    bool x_aligned;    // every row starts on 16 bytes (widths are multiples of 16)
     float *part;       // [E][S][N][K]
-    int K, N, batch, rows_per_split, nsplit;
+    int K, N, batch, nsplit;
 
-    __device__ int red() const { return rows_per_split; }
-    __host__ __device__ int ncols() const { return K; }
-    __device__ uint4 load_a(int e, int n, int r) const {   // r: row offset inside the split
-        Pack8 p;
-        const int b0 = blockIdx.y * rows_per_split + r;
-        const bf16 *d = dz + e * dz_es + n;
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const int b = b0 + j;
-            p.h[j] = (n < N && r + j < rows_per_split && b < batch) ? d[(long)b * WIDTH] : __float2bfloat16_rn(0.0f);
-        }
-        return p.u;
+    __device__ uint4 row_a(int e, int split, int n, int r, int j) const {   // r: row offset inside the split
+        const int b = split * HGB_MLP_SPLIT_ROWS + r + j;
+        if (n >= N || b >= batch) return make_uint4(0, 0, 0, 0);
+        return *(const uint4 *)(dz + e * dz_es + (long)b * WIDTH + n);
     }
-    __device__ uint4 load_b(int e, int k, int r) const {
-        Pack8 p;
-        const int b0 = blockIdx.y * rows_per_split + r;
-        const bf16 *xp = x + e * x_es + k;
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const int b = b0 + j;
-            p.h[j] = (k < K && r + j < rows_per_split && b < batch) ? xp[(long)b * ldx] : __float2bfloat16_rn(0.0f);
-        }
-        return p.u;
+    __device__ uint4 row_b(int e, int split, int k, int r, int j) const {
+        const int b = split * HGB_MLP_SPLIT_ROWS + r + j;
+        if (k >= K || b >= batch) return make_uint4(0, 0, 0, 0);
+        return load8(x + e * x_es + (long)b * ldx + k, x_aligned);
     }
-    __device__ void store(int e, int n, int k0, const float (&v)[16]) const {
+    __device__ void store(int e, int split, int n, int k0, const float (&v)[16]) const {
         if (n >= N || k0 >= K) return;
-        float4 *d = (float4 *)(part + (((long)e * nsplit + blockIdx.y) * N + n) * K + k0);
+        float4 *d = (float4 *)(part + (((long)e * nsplit + split) * N + n) * K + k0);
 #pragma unroll
         for (int i = 0; i < 4; i++) d[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
     }
@@ -297,25 +296,58 @@ struct DwOp {   // part[s][n][k] = sum over this split's rows b of dZ[b][n] X[b]
 template <int N>
 __host__ __device__ constexpr int tmem_cols() { return N <= 32 ? 32 : N <= 64 ? 64 : N <= 128 ? 128 : 256; }
 
-// One 128 x NT output tile (blockIdx.x: row tile, blockIdx.y: column tile or batch split,
-// blockIdx.z: ensemble member).
-template <class Op>
-__global__ void __launch_bounds__(THREADS) k_mlp_gemm(Op op, int *status) {
-    constexpr int KC = Op::KC, NT = Op::NT, COLS = tmem_cols<NT>();
-    constexpr int SMEM_A = TM * KC * 2;
-    static_assert(SMEM_A + NT * KC * 2 <= SMEM_DYN, "staged slices must fit the dynamic shared memory");
-    static_assert(KC % 16 == 0 && NT % 16 == 0 && NT <= NMAX, "tile shape");
+// Transposes an 8 x 8 block of bf16, rows in r[0..7], in registers: the pairs and quads move by naming,
+// the halves by byte permutes.
+__device__ __forceinline__ void transpose8(const uint4 (&r)[8], uint4 (&t)[8]) {
+    uint32_t o[8][4];
+#pragma unroll
+    for (int c = 0; c < 4; c++) {   // columns 2 c and 2 c + 1
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const uint32_t lo = (&r[2 * j].x)[c], hi = (&r[2 * j + 1].x)[c];
+            o[2 * c][j] = __byte_perm(lo, hi, 0x5410);
+            o[2 * c + 1][j] = __byte_perm(lo, hi, 0x7632);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; i++) t[i] = make_uint4(o[i][0], o[i][1], o[i][2], o[i][3]);
+}
+
+// the core matrices of rows x .. x + 7, reduction entries r .. r + 7, from eight rows of the row-major
+// buffer that has x fastest: row(j) holds reduction entry r + j
+template <int KC, class Row>
+__device__ __forceinline__ void stage_transposed(uint8_t *s, int x, int r, const Row &row) {
+    uint4 in[8], t[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) in[j] = row(j);
+    transpose8(in, t);
+#pragma unroll
+    for (int i = 0; i < 8; i++) *(uint4 *)(s + slice_off<KC>(x + i, r)) = t[i];
+}
+
+// One layer of the backward pass in one launch: the blocks of the input gradient (128 batch rows x 64
+// columns each, first: the next layer waits for them) and those of the weight gradient (128 outputs x
+// 64 inputs of one 128-row batch split).  Both read dZ of the layer and depend on nothing else of each
+// other's.  Operands that lie transposed in memory are staged by 8 x 8 blocks, eight 16-byte loads a
+// thread and a register transpose (gathering them two bytes at a time took most of the time): at batch
+// 512 and 4 members of 256 x 256, 24 + 23 us a layer for the two gradients in launches of their own and
+// with four warps a block,
+// 13 us for both.
+struct BwdLayer {
+    DxOp dx;
+    DwOp dw;
+    int dx_rows, dx_cols;              // tiles of the input gradient (0 for the first layer)
+    int dw_rows, dw_cols, nsplit;      // tiles and batch splits of the weight gradient
+};
+
+__global__ void __launch_bounds__(LAYER_THREADS) k_mlp_bwd(const __grid_constant__ BwdLayer L, int *status) {
+    constexpr int NT = 64, COLS = tmem_cols<NT>();
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t mbar;
     __shared__ uint32_t tmem_slot;
-    uint8_t *sa = smem;
-    uint8_t *sb = smem + SMEM_A;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int e = blockIdx.z;
-    const int row0 = blockIdx.x * TM;
-    const int col0 = Op::COL_TILED ? (int)blockIdx.y * NT : 0;
-    const int ncols = min(NT, op.ncols() - col0), red = op.red();
-    const int npad = (ncols + 15) & ~15;
+    const int e = blockIdx.y, n_dx = L.dx_rows * L.dx_cols;
+    const bool is_dx = (int)blockIdx.x < n_dx;
     const uint32_t mb = smem_u32(&mbar);
 
     if (warp == 0) tmem_alloc(smem_u32(&tmem_slot), COLS);
@@ -324,51 +356,69 @@ __global__ void __launch_bounds__(THREADS) k_mlp_gemm(Op op, int *status) {
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
-    const uint32_t idesc = idesc_bf16(TM, npad);
 
-    bool ok = true;
-    uint32_t parity = 0;
-    const int nslices = (red + KC - 1) / KC;
-    for (int c = 0; c < nslices; c++) {
-        const int k0 = c * KC;
-        const int kact = min(KC, ((red - k0) + 15) & ~15);   // staged (and multiplied) part of the slice
-        for (int v = threadIdx.x; v < TM * (kact / 8); v += THREADS) {
-            const int r = v % TM, kg = v / TM;
-            *(uint4 *)(sa + slice_off<KC>(r, kg * 8)) = op.load_a(e, row0 + r, k0 + kg * 8);
+    int row0, col0, split = 0, npad, red;
+    uint8_t *sa = smem, *sb;
+    if (is_dx) {
+        row0 = ((int)blockIdx.x / L.dx_cols) * TM;
+        col0 = ((int)blockIdx.x % L.dx_cols) * NT;
+        npad = min(NT, L.dx.K - col0);      // widths are multiples of 16
+        red = L.dx.N;
+        sb = smem + TM * DxOp::KC * 2;
+        const int kg = red / 8;
+#pragma unroll 8
+        for (int v = threadIdx.x; v < TM * kg; v += LAYER_THREADS) {
+            const int r = v % TM, g = v / TM;
+            *(uint4 *)(sa + slice_off<DxOp::KC>(r, g * 8)) = L.dx.load_a(e, row0 + r, g * 8);
         }
-        for (int v = threadIdx.x; v < npad * (kact / 8); v += THREADS) {
-            const int n = v % npad, kg = v / npad;
-            *(uint4 *)(sb + slice_off<KC>(n, kg * 8)) = op.load_b(e, col0 + n, k0 + kg * 8);
+        for (int v = threadIdx.x; v < (npad / 8) * kg; v += LAYER_THREADS) {
+            const int x = (v % (npad / 8)) * 8, n = (v / (npad / 8)) * 8;
+            stage_transposed<DxOp::KC>(sb, x, n, [&](int j) { return L.dx.row_b(e, col0 + x, n, j); });
         }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            tc_fence_after();
-            for (int s = 0; s < kact / 16; s++)
-                mma_bf16(tmem, smem_desc(smem_u32(sa) + 256 * s, 128, 16 * KC),
-                         smem_desc(smem_u32(sb) + 256 * s, 128, 16 * KC), idesc, (c > 0 || s > 0) ? 1u : 0u);
-            mma_commit(mb);
+    } else {
+        int i = (int)blockIdx.x - n_dx;
+        split = i % L.nsplit;
+        i /= L.nsplit;
+        row0 = (i / L.dw_cols) * TM;
+        col0 = (i % L.dw_cols) * NT;
+        npad = min(NT, L.dw.K - col0);
+        red = HGB_MLP_SPLIT_ROWS;           // rows beyond the batch are zeros
+        sb = smem + TM * DwOp::KC * 2;
+        constexpr int KG = HGB_MLP_SPLIT_ROWS / 8;
+        for (int v = threadIdx.x; v < (TM / 8) * KG; v += LAYER_THREADS) {
+            const int x = (v % (TM / 8)) * 8, r = (v / (TM / 8)) * 8;
+            stage_transposed<DwOp::KC>(sa, x, r, [&](int j) { return L.dw.row_a(e, split, row0 + x, r, j); });
         }
-        // every thread waits: the next slice overwrites shared memory, the epilogue reads TMEM
-        const bool done = mbar_wait(mb, parity);
-        parity ^= 1u;
-        if (!__syncthreads_and(done)) {
-            ok = false;
-            break;
+        for (int v = threadIdx.x; v < (npad / 8) * KG; v += LAYER_THREADS) {
+            const int x = (v % (npad / 8)) * 8, r = (v / (npad / 8)) * 8;
+            stage_transposed<DwOp::KC>(sb, x, r, [&](int j) { return L.dw.row_b(e, split, col0 + x, r, j); });
         }
     }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        tc_fence_after();
+        const uint32_t idesc = idesc_bf16(TM, npad);
+        const uint32_t sbo = 16 * (is_dx ? DxOp::KC : DwOp::KC);
+        for (int s = 0; s < red / 16; s++)
+            mma_bf16(tmem, smem_desc(smem_u32(sa) + 256 * s, 128, sbo), smem_desc(smem_u32(sb) + 256 * s, 128, sbo),
+                     idesc, s > 0 ? 1u : 0u);
+        mma_commit(mb);
+    }
+    const bool ok = __syncthreads_and(mbar_wait(mb, 0));
     tc_fence_after();
     if (ok) {
-        const int m = warp * 32 + lane;
-        const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
-        for (int n0 = 0; n0 < npad; n0 += 16) {
+        const int m = (warp & 3) * 32 + lane;   // a warp reads the TMEM lanes of its place among four
+        const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+        for (int n0 = (warp >> 2) * 16; n0 < npad; n0 += 32) {
             float v[16];
             tmem_ld16(lane_addr + (uint32_t)n0, v);
-            op.store(e, row0 + m, col0 + n0, v);
+            if (is_dx) L.dx.store(e, row0 + m, col0 + n0, v);
+            else L.dw.store(e, split, row0 + m, col0 + n0, v);
         }
     } else {
         if (threadIdx.x == 0) hgb::flag(status, HGB_STATUS_ITERATION_LIMIT);
-        mbar_wait(mb, parity ^ 1u);   // give the tensor core a last bounded chance to finish
+        mbar_wait(mb, 0);   // give the tensor core a last bounded chance to finish
     }
     tc_fence_before();
     __syncthreads();
@@ -400,7 +450,7 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map
 
 // blockIdx.x: 128-row tile, blockIdx.y: 64-column tile, blockIdx.z: member.  xmap: [members or 1][rows][K]
 // activations (x_member != 0 when each member has its own), wmap: [members][N][K] weights.
-__global__ void __launch_bounds__(THREADS) k_mlp_fwd_tma(const __grid_constant__ CUtensorMap xmap,
+__global__ void __launch_bounds__(LAYER_THREADS) k_mlp_fwd_tma(const __grid_constant__ CUtensorMap xmap,
                                                          const __grid_constant__ CUtensorMap wmap, FwdOp op,
                                                          int x_member, int *status) {
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -421,9 +471,10 @@ __global__ void __launch_bounds__(THREADS) k_mlp_fwd_tma(const __grid_constant__
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
-    if (threadIdx.x == 0) {
-        mbar_expect_tx(mb, (uint32_t)groups * (TM + FWD_NT) * 16);
-        for (int g = 0; g < groups; g++) {
+    if (warp == 0) {   // a lane per K-group: one thread's 64 boxes, one after another, set the pace before
+        if (lane == 0) mbar_expect_tx(mb, (uint32_t)groups * (TM + FWD_NT) * 16);
+        __syncwarp();
+        for (int g = lane; g < groups; g += 32) {
             tma_load_3d(smem_u32(sa + g * TM * 16), &xmap, g * 8, row0, x_member ? e : 0, mb);
             tma_load_3d(smem_u32(sb + g * FWD_NT * 16), &wmap, g * 8, col0, e, mb);
         }
@@ -444,9 +495,9 @@ __global__ void __launch_bounds__(THREADS) k_mlp_fwd_tma(const __grid_constant__
     }
     tc_fence_after();
     if (ok) {
-        const int m = warp * 32 + lane;
-        const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
-        for (int n0 = 0; n0 < ncols; n0 += 16) {
+        const int m = (warp & 3) * 32 + lane;   // a warp reads the TMEM lanes of its place among four
+        const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+        for (int n0 = (warp >> 2) * 16; n0 < ncols; n0 += 32) {
             float v[16];
             tmem_ld16(lane_addr + (uint32_t)n0, v);
             op.store(e, row0 + m, col0 + n0, v);
@@ -516,7 +567,7 @@ int launch_fwd_tma(const FwdOp &op, long x_member_stride_elems, int members, int
                         (uint64_t)op.w_es * 2, 8, FWD_NT);
     if (rc) return rc;
     dim3 grid((unsigned)hgb::ceil_div(op.batch, TM), (unsigned)hgb::ceil_div(op.N, FWD_NT), (unsigned)members);
-    k_mlp_fwd_tma<<<grid, THREADS, SMEM_DYN, st>>>(xmap, wmap, op, x_member, status);
+    k_mlp_fwd_tma<<<grid, LAYER_THREADS, SMEM_DYN, st>>>(xmap, wmap, op, x_member, status);
     return hgb::check_launch();
 }
 
@@ -548,26 +599,33 @@ NetView view_of(const hgb_mlp *net) {
     return v;
 }
 
-// loss[e] = mean (out - target)^2; dZ of the last layer = d loss / d out (bf16), one block per member
-__global__ void k_mse(int batch, int nout, const float *__restrict__ out, const float *__restrict__ target,
-                      long t_es, bf16 *__restrict__ dz, long dz_es, float *__restrict__ loss) {
-    const int e = blockIdx.x;
+// dZ of the last layer = d loss / d out (bf16) of loss[e] = mean (out - target)^2, and this block's part
+// of the loss's sum (added up in block order by k_grad_reduce).  One block per member took 162 us of a
+// 512-row step; over MSE_BLOCKS blocks a member it is 7 us.
+constexpr int MSE_BLOCKS = 32;
+
+__global__ void __launch_bounds__(256) k_mse(int batch, int nout, const float *__restrict__ out, const float *__restrict__ target,
+                      long t_es, bf16 *__restrict__ dz, long dz_es, float *__restrict__ part) {
+    const int e = blockIdx.y;
     const float scale = 2.0f / ((float)batch * (float)nout);
+    const long total = (long)batch * nout;
     float acc = 0.0f;
-    for (long i = threadIdx.x; i < (long)batch * nout; i += blockDim.x) {
+    for (long i = (long)blockIdx.x * 256 + threadIdx.x; i < total; i += 256L * MSE_BLOCKS) {
         const long b = i / nout, n = i % nout;
-        const float d = out[e * (long)batch * nout + i] - target[e * t_es + i];
+        const float d = out[e * total + i] - target[e * t_es + i];
         acc += d * d;
         dz[e * dz_es + b * WIDTH + n] = __float2bfloat16_rn(scale * d);
     }
-    __shared__ float red[256];
-    red[threadIdx.x] = acc;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    __shared__ float red[8];
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
     __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-        __syncthreads();
+    if (threadIdx.x == 0) {
+        float v = red[0];
+        for (int w = 1; w < 8; w++) v += red[w];
+        part[e * MSE_BLOCKS + blockIdx.x] = v;
     }
-    if (threadIdx.x == 0 && loss) loss[e] = red[0] / ((float)batch * (float)nout);
 }
 
 struct GradArgs {
@@ -577,28 +635,58 @@ struct GradArgs {
     const bf16 *dz[HGB_MLP_MAX_LAYERS];      // [E][B][WIDTH]
     long dz_es;
     float *grad;                             // [E][n_p]
+    const float *loss_part;                  // [E][MSE_BLOCKS]
+    float *loss;                             // [E] or null
+    int w_blocks, bias_tiles;                // blocks of the weights; 32-output tiles of one member's biases
 };
 
-// weight gradients: the split partials summed in split order; bias gradients: dZ summed over the batch
-__global__ void k_grad_reduce(GradArgs a) {
-    const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (long)a.v.E * a.v.n_p) return;
-    const int e = (int)(idx / a.v.n_p);
-    const long p = idx % a.v.n_p;
-    int l = 0;
-    while (l + 1 < a.v.L && p >= a.v.p_off[l + 1]) l++;
-    const int K = a.v.K[l], N = a.v.N[l];
-    float g = 0.0f;
-    if (p < a.v.b_off[l]) {
-        const long wi = p - a.v.p_off[l];
-        const float *pp = a.part[l] + (long)e * a.nsplit * N * K + wi;
-        for (int s = 0; s < a.nsplit; s++) g += pp[(long)s * N * K];
-    } else {
-        const int n = (int)(p - a.v.b_off[l]);
-        const bf16 *d = a.dz[l] + e * a.dz_es + n;
-        for (int b = 0; b < a.batch; b++) g += __bfloat162float(d[(long)b * WIDTH]);
+// weight gradients: the split partials summed in split order, one thread each (blocks of the first
+// `w_blocks`, the rest of the grid being: one block per member, layer and 32 outputs, whose eight warps
+// sum dZ over an eighth of the batch each for the bias gradients; then one block for the losses).  A
+// single thread per bias walked the whole batch: 23 us, 12 us now.
+__global__ void __launch_bounds__(256) k_grad_reduce(GradArgs a) {
+    const int t = threadIdx.x;
+    if ((int)blockIdx.x < a.w_blocks) {
+        const long idx = (long)blockIdx.x * 256 + t;
+        if (idx >= (long)a.v.E * a.v.n_p) return;
+        const int e = (int)(idx / a.v.n_p);
+        const long p = idx % a.v.n_p;
+        int l = 0;
+        while (l + 1 < a.v.L && p >= a.v.p_off[l + 1]) l++;
+        if (p >= a.v.b_off[l]) return;
+        const long nk = (long)a.v.K[l] * a.v.N[l];
+        const float *pp = a.part[l] + (long)e * a.nsplit * nk + (p - a.v.p_off[l]);
+        float g = 0.0f;
+        for (int s = 0; s < a.nsplit; s++) g += pp[(long)s * nk];
+        a.grad[idx] = g;
+        return;
     }
-    a.grad[idx] = g;
+    __shared__ float red[8][32];
+    int i = (int)blockIdx.x - a.w_blocks;
+    if (i == a.v.E * a.bias_tiles) {
+        for (int e = t; a.loss && e < a.v.E; e += 256) {
+            float v = 0.0f;
+            for (int k = 0; k < MSE_BLOCKS; k++) v += a.loss_part[e * MSE_BLOCKS + k];
+            a.loss[e] = v / ((float)a.batch * (float)a.v.N[a.v.L - 1]);
+        }
+        return;
+    }
+    const int e = i / a.bias_tiles;
+    i %= a.bias_tiles;
+    int l = 0;
+    while (i >= (a.v.N[l] + 31) / 32) i -= (a.v.N[l++] + 31) / 32;
+    const int n = 32 * i + (t & 31), warp = t >> 5;
+    float g = 0.0f;
+    if (n < a.v.N[l]) {
+        const bf16 *d = a.dz[l] + e * a.dz_es + n;
+        for (int b = warp; b < a.batch; b += 8) g += __bfloat162float(d[(long)b * WIDTH]);
+    }
+    red[warp][t & 31] = g;
+    __syncthreads();
+    if (warp == 0 && n < a.v.N[l]) {
+        for (int w = 1; w < 8; w++) g += red[w][t];
+        a.grad[(long)e * a.v.n_p + a.v.b_off[l] + n] = g;
+    }
 }
 
 // decoupled AdamW on the fp32 master parameters; weights (not biases) decay; bf16 weight copies written
@@ -644,20 +732,18 @@ int check_net(const hgb_mlp *net) {
     return 1;
 }
 
-template <class Op>
-int launch_gemm(const Op &op, int row_tiles, int members, int *status, cudaStream_t st, int splits = 1) {
-    static std::atomic<bool> attr_set{false};   // idempotent; set before the first launch of each instantiation
+int launch_bwd(const BwdLayer &L, int members, int *status, cudaStream_t st) {
+    static std::atomic<bool> attr_set{false};   // idempotent; set before the first launch
     if (!attr_set.load(std::memory_order_acquire)) {
-        cudaError_t err = cudaFuncSetAttribute(k_mlp_gemm<Op>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_DYN);
+        cudaError_t err = cudaFuncSetAttribute(k_mlp_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_DYN);
         if (err != cudaSuccess) {
             hgb::set_cuda_error(err);
             return HGB_ERR_CUDA;
         }
         attr_set.store(true, std::memory_order_release);
     }
-    const int ytiles = Op::COL_TILED ? (int)hgb::ceil_div(op.ncols(), Op::NT) : splits;
-    dim3 grid((unsigned)row_tiles, (unsigned)ytiles, (unsigned)members);
-    k_mlp_gemm<Op><<<grid, THREADS, SMEM_DYN, st>>>(op, status);
+    const unsigned blocks = (unsigned)((long)L.dx_rows * L.dx_cols + (long)L.dw_rows * L.dw_cols * L.nsplit);
+    k_mlp_bwd<<<dim3(blocks, (unsigned)members), LAYER_THREADS, SMEM_DYN, st>>>(L, status);
     return hgb::check_launch();
 }
 
@@ -948,7 +1034,7 @@ size_t hgb_mlp_backward_workspace_bytes(const hgb_mlp *net, int batch) {
     const int nsplit = (int)hgb::ceil_div(batch, HGB_MLP_SPLIT_ROWS);
     size_t bytes = sizeof(uint16_t) * (size_t)v.L * v.E * batch * WIDTH;   // dZ per layer
     for (int l = 0; l < v.L; l++) bytes += sizeof(float) * (size_t)v.E * nsplit * v.N[l] * v.K[l];
-    return bytes;
+    return bytes + sizeof(float) * (size_t)v.E * MSE_BLOCKS;
 }
 
 int hgb_mlp_backward(const hgb_mlp *net, const uint16_t *x, long x_member_stride, int batch, const uint16_t *act,
@@ -978,40 +1064,52 @@ int hgb_mlp_backward(const hgb_mlp *net, const uint16_t *x, long x_member_stride
         }
     }
     const int last = v.L - 1;
-    k_mse<<<v.E, 256, 0, st>>>(batch, v.N[last], out, target, target_member_stride, dz + last * hid_ls, hid_es, loss);
+    float *loss_part = part;
+    for (int l = 0; l < v.L; l++) loss_part += (size_t)v.E * nsplit * v.N[l] * v.K[l];
+    k_mse<<<dim3(MSE_BLOCKS, (unsigned)v.E), 256, 0, st>>>(batch, v.N[last], out, target, target_member_stride,
+                                                           dz + last * hid_ls, hid_es, loss_part);
     int rc = hgb::check_launch();
     if (rc) return rc;
     for (int l = last; l >= 0; l--) {
-        DwOp dw{};
-        dw.dz = dz + l * hid_ls;
-        dw.dz_es = hid_es;
-        dw.x = l == 0 ? (const bf16 *)x : (const bf16 *)act + (l - 1) * hid_ls;
-        dw.x_es = l == 0 ? x_member_stride : hid_es;
-        dw.ldx = l == 0 ? v.K[0] : WIDTH;
-        dw.part = const_cast<float *>(ga.part[l]);
-        dw.K = v.K[l];
-        dw.N = v.N[l];
-        dw.batch = batch;
-        dw.rows_per_split = HGB_MLP_SPLIT_ROWS;
-        dw.nsplit = nsplit;
-        if ((rc = launch_gemm(dw, (int)hgb::ceil_div(v.N[l], TM), v.E, d_status, st, nsplit))) return rc;
-        if (l == 0) break;
-        DxOp dx{};
-        dx.dz = dz + l * hid_ls;
-        dx.dz_es = hid_es;
-        dx.w = (const bf16 *)net->weights + v.w_off[l];
-        dx.w_es = v.n_w;
-        dx.pre = pre + (l - 1) * hid_ls;
-        dx.pre_es = hid_es;
-        dx.dzp = dz + (l - 1) * hid_ls;
-        dx.dzp_es = hid_es;
-        dx.K = v.K[l];
-        dx.N = v.N[l];
-        dx.batch = batch;
-        if ((rc = launch_gemm(dx, (int)hgb::ceil_div(batch, TM), v.E, d_status, st))) return rc;
+        BwdLayer L{};
+        L.dw.dz = dz + l * hid_ls;
+        L.dw.dz_es = hid_es;
+        L.dw.x = l == 0 ? (const bf16 *)x : (const bf16 *)act + (l - 1) * hid_ls;
+        L.dw.x_es = l == 0 ? x_member_stride : hid_es;
+        L.dw.ldx = l == 0 ? v.K[0] : WIDTH;
+        L.dw.x_aligned = l > 0 || (((uintptr_t)x | (uintptr_t)(2 * x_member_stride)) & 15) == 0;
+        L.dw.part = const_cast<float *>(ga.part[l]);
+        L.dw.K = v.K[l];
+        L.dw.N = v.N[l];
+        L.dw.batch = batch;
+        L.dw.nsplit = nsplit;
+        L.dw_rows = (int)hgb::ceil_div(v.N[l], TM);
+        L.dw_cols = (int)hgb::ceil_div(v.K[l], DwOp::NT);
+        L.nsplit = nsplit;
+        if (l > 0) {
+            L.dx.dz = dz + l * hid_ls;
+            L.dx.dz_es = hid_es;
+            L.dx.w = (const bf16 *)net->weights + v.w_off[l];
+            L.dx.w_es = v.n_w;
+            L.dx.w_aligned = ((uintptr_t)net->weights & 15) == 0;   // layers and members: multiples of 256 values
+            L.dx.pre = pre + (l - 1) * hid_ls;
+            L.dx.pre_es = hid_es;
+            L.dx.dzp = dz + (l - 1) * hid_ls;
+            L.dx.dzp_es = hid_es;
+            L.dx.K = v.K[l];
+            L.dx.N = v.N[l];
+            L.dx.batch = batch;
+            L.dx_rows = (int)hgb::ceil_div(batch, TM);
+            L.dx_cols = (int)hgb::ceil_div(v.K[l], DxOp::NT);
+        }
+        if ((rc = launch_bwd(L, v.E, d_status, st))) return rc;
     }
-    const long np = (long)v.E * v.n_p;
-    k_grad_reduce<<<(unsigned)hgb::ceil_div(np, 256), 256, 0, st>>>(ga);
+    ga.loss_part = loss_part;
+    ga.loss = loss;
+    ga.w_blocks = (int)hgb::ceil_div((long)v.E * v.n_p, 256);
+    ga.bias_tiles = 0;
+    for (int l = 0; l < v.L; l++) ga.bias_tiles += (v.N[l] + 31) / 32;
+    k_grad_reduce<<<(unsigned)(ga.w_blocks + v.E * ga.bias_tiles + 1), 256, 0, st>>>(ga);
     return hgb::check_launch();
 }
 

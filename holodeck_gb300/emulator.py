@@ -168,7 +168,7 @@ class MLPEnsemble:
         N.call("hgb_mlp_backward", ctypes.byref(self.struct), N.ptr(x), 0, batch, N.ptr(buf["act"]),
                N.ptr(buf["pre"]), N.ptr(out), N.ptr(target), 0, N.ptr(self.grad), N.ptr(buf["loss"]),
                N.ptr(buf["ws"]), buf["ws_bytes"], self.status.ptr, N.stream_handle())
-        N.add_launches(2 * self.L + 1)
+        N.add_launches(self.L + 2)
         return buf["loss"]
 
     def train_step(self, x, target, lr, weight_decay=1e-4, beta1=0.9, beta2=0.999, eps=1e-8):
