@@ -40,10 +40,10 @@
 //                             bin costs about one draw per event instead of one per lane
 //   SPARSE_MAX <= lambda < 10 a 32-column alias row per bin (n < 31 and the rest at 31): one
 //                             lookup and one comparison per draw; four realizations per Philox call
-//   10 <= lambda <= 65536     inversion against a per-bin table over lambda +- 7 sqrt(lambda) in
-//                             shared memory, with a guide table whose "pure" cells answer most draws
-//                             with one lookup; four realizations per Philox call
-//   65536 < lambda < 2^22     PTRS, transformed rejection with squeeze (Hormann 1993, Insurance:
+//   10 <= lambda <= 47000     inversion by a binary search of a per-bin table over
+//                             lambda +- 7 sqrt(lambda) in shared memory; four realizations per
+//                             Philox call
+//   47000 < lambda < 2^22     PTRS, transformed rejection with squeeze (Hormann 1993, Insurance:
 //                             Mathematics and Economics 12, 39-45) in FP32: the acceptance test uses
 //                             the log-pmf in Loader's saddle-point form (bd0 + Stirling remainder,
 //                             Loader 2000), so nothing cancels in FP32.  Each lane runs one loop
@@ -75,7 +75,7 @@ namespace {
 
 constexpr int RB = 128;                  // threads per block == bins per staged tile
 constexpr int NWARP = RB / 32;
-constexpr int RPT = 8;                   // realizations per thread
+constexpr int RPT = 8;                   // realizations per thread, at most (see with_slots)
 static_assert(RPT == 8, "the table passes draw four realizations per Philox call, two calls per bin");
 constexpr int NT = 32;                   // CDF thresholds per small-lambda bin
 constexpr double SPARSE_MAX = 0.1;       // geometric skipping over realizations below this expectation
@@ -88,13 +88,13 @@ constexpr int MAX_INVERSION = 4096;
 constexpr int MAX_PREFIX_EXTRA = 1024;   // prefix events beyond L (Normal draws below 1)
 constexpr double TABLE_MAX = 47000.0;    // table inversion up to here: k_lo..k_hi spans <= 14 sqrt(lambda) + 10
 constexpr int TMAX = 3072;               // table entries (>= 14 sqrt(TABLE_MAX) + 10 = 3046)
-constexpr int HALF_WORDS = 2048 + 512;   // tables up to 2048 entries (2^10 u16 guide cells) fit a half
-constexpr int ARENA_WORDS = 2 * HALF_WORDS;   // the halves alternate between build and draw
-static_assert(TMAX + 2048 <= ARENA_WORDS, "the largest table (2^12 guide cells) fits the whole arena");
-constexpr int BATCH_MAX = 32;            // table-kind bins built per batch
-constexpr int BULK_BLOCKS_PER_SM = 6;    // k_bulk residency (seven was measured slower: 30.7 against 29.2 ms)
-constexpr unsigned GUIDE_PURE = 0x8000u, GUIDE_ONE = 0x4000u, GUIDE_M = 0x0FFFu;   // guide cell fields
-static_assert(TMAX - 1 <= (int)GUIDE_M, "table entries fit the guide's index field");
+constexpr int ARENA_WORDS = 4224;        // words of one batch of tables
+constexpr int TABLE_PAD = 3;             // words around a table: two zeros before it, 2^32 - 1 after it
+static_assert(TMAX + TABLE_PAD <= ARENA_WORDS, "the largest table fits the arena");
+constexpr int BATCH_MAX = 32;            // table-kind bins built per batch (one per lane of a scan)
+constexpr int UNIT_MAX = 512;            // units of work (see build_tables) of one batch
+constexpr int WIDE_RUNS = 2048;          // tables of more entries than this are cut into 128 runs, not 32
+constexpr int BULK_BLOCKS_PER_SM = 6;    // k_bulk residency that chunk counts assume (7 or 8 blocks fit; the chunks fix the sums' order)
 static_assert(ARENA_WORDS >= RB * (NT + 1), "the small-lambda rows share the arena");
 constexpr int ANCHOR = 16;               // Loader-form pmf every ANCHOR-th entry, the recursion between
 constexpr float TABLE_SIGMAS = 7.0f;     // the table covers lambda +- 7 sqrt(lambda) (tails < 1e-11)
@@ -179,16 +179,18 @@ struct Tile {
         // small lambda: one padded 32-column alias row per bin (threshold << 5 | alias); the lanes of
         // a warp read one bin's row at different columns, which the padding puts in different banks
         unsigned int thr[RB][NT + 1];
-        unsigned int arena[ARENA_WORDS];          // table kind: packed cdf (u32) + guide (u16) tables
+        unsigned int arena[ARENA_WORDS];          // table kind: the batch's cdf tables
     } u;
+    unsigned int ubase[UNIT_MAX];     // table kind: cdf before each unit of the batch, saturated
+    int b_off[BATCH_MAX], b_unit[BATCH_MAX + 1];   // arena offset and first unit of the batch's tables
     unsigned char sp_lg[RB];          // sparse: log2 of the realization run length of the bin
     int sp_start[RB];                 // sparse: first run of each sparse-list entry
     unsigned long long scan[NWARP];
-    double lam[RB];
+    double lam[RB];                   // (wide kind)
     float hs[RB];                     // h2fdf * 2^100 (for the background sums)
     float frac[RB], lamf[RB];
     int lam_int[RB];
-    int tb_klo[RB], tb_S[RB], tb_gb[RB];   // table kind: first count, entries, log2 guide cells
+    unsigned short tb_klo[RB], tb_S[RB];   // table kind: first count and entries
     int pos[RB];                      // sorted position (loudest) or grid index (gwb) of the bin
     unsigned char list[NKIND][RB];    // tile-local bin indices per kind, in bin order
     int wcount[NWARP][NKIND];
@@ -206,12 +208,14 @@ __device__ __forceinline__ int kind_count(const Tile &s, int k) {
 // tail cells, PTRS, and with the parameter sums every per-lane pass), indexed [slot][thread]:
 // plain FP32 where the terms are few (a few percent of the table draws and the PTRS bins), Kahan
 // pairs for the parameter path.
+template <int NS>
 struct SlotsPlain {
-    float acc[RPT][RB];
+    float acc[NS][RB];
 };
+template <int NS>
 struct SlotsKahan {
-    float acc[RPT][RB];
-    float comp[RPT][RB];
+    float acc[NS][RB];
+    float comp[NS][RB];
 };
 
 __device__ __forceinline__ int bin_kind(double lam) {
@@ -291,9 +295,8 @@ __device__ void bin_setup(Tile &s, int j, int kind, double lam, double h) {
             const float sd = sqrtf(lf);
             const int k_lo = max(0, (int)floorf(lf - TABLE_SIGMAS * sd - 2.0f));
             const int S = min((int)ceilf(lf + TABLE_SIGMAS * sd + 6.0f) - k_lo + 1, TMAX);
-            s.tb_klo[j] = k_lo;
-            s.tb_S[j] = S;
-            s.tb_gb[j] = max(1, 31 - __clz(S - 1));   // ceil(log2 S) - 1: 2^gb >= S / 2 guide cells
+            s.tb_klo[j] = (unsigned short)k_lo;   // below TABLE_MAX
+            s.tb_S[j] = (unsigned short)S;
         }
     }
 }
@@ -444,26 +447,39 @@ __device__ int truncated_count_f32(float lam, float v, int *d_status) {
 }
 
 
-__device__ __forceinline__ void kahan_add(float &sum, float &comp, float x) {
-    float y = x - comp;
+// a * b added: the product is not rounded by itself
+__device__ __forceinline__ void kahan_add(float &sum, float &comp, float a, float b) {
+    float y = __fmaf_rn(a, b, -comp);
     float t = sum + y;
     comp = (t - sum) - y;
     sum = t;
 }
 
-__device__ __forceinline__ void add_bg(SlotsPlain &st, int sl, int t, float x) { st.acc[sl][t] += x; }
-__device__ __forceinline__ void slot_zero(SlotsPlain &st, int sl, int t) { st.acc[sl][t] = 0.0f; }
-__device__ __forceinline__ double slot_value(const SlotsPlain &st, int sl, int t) { return (double)st.acc[sl][t]; }
-__device__ __forceinline__ void slot_zero(SlotsKahan &st, int sl, int t) {
+template <int NS>
+__device__ __forceinline__ void add_bg(SlotsPlain<NS> &st, int sl, int t, float a, float b) {
+    st.acc[sl][t] = __fmaf_rn(a, b, st.acc[sl][t]);
+}
+template <int NS>
+__device__ __forceinline__ void slot_zero(SlotsPlain<NS> &st, int sl, int t) {
+    st.acc[sl][t] = 0.0f;
+}
+template <int NS>
+__device__ __forceinline__ double slot_value(const SlotsPlain<NS> &st, int sl, int t) {
+    return (double)st.acc[sl][t];
+}
+template <int NS>
+__device__ __forceinline__ void slot_zero(SlotsKahan<NS> &st, int sl, int t) {
     st.acc[sl][t] = 0.0f;
     st.comp[sl][t] = 0.0f;
 }
-__device__ __forceinline__ double slot_value(const SlotsKahan &st, int sl, int t) {
+template <int NS>
+__device__ __forceinline__ double slot_value(const SlotsKahan<NS> &st, int sl, int t) {
     return (double)st.acc[sl][t] - (double)st.comp[sl][t];
 }
-__device__ __forceinline__ void add_bg(SlotsKahan &st, int sl, int t, float x) {
+template <int NS>
+__device__ __forceinline__ void add_bg(SlotsKahan<NS> &st, int sl, int t, float a, float b) {
     float acc = st.acc[sl][t], comp = st.comp[sl][t];
-    kahan_add(acc, comp, x);
+    kahan_add(acc, comp, a, b);
     st.acc[sl][t] = acc;
     st.comp[sl][t] = comp;
 }
@@ -754,144 +770,163 @@ struct BulkArgs {
     int *wide_flag;    // set by k_bulk when it leaves bins to k_bulk_wide (zeroed before the launch)
 };
 
-// Inversion table of one table-kind bin (lambda in [10, TABLE_MAX]), built by a warp or a block:
+// Inversion table of one table-kind bin (lambda in [10, TABLE_MAX]):
 //   cdf[m]   = min(sum of q(k_lo) .. q(k_lo + m), 2^32 - 1), with q(k) = P(k) in 32.32 fixed point
 //              (rounded to nearest); cdf[S - 1] = 2^32 - 1, so the mass outside the range (< 1e-11)
 //              goes to the end entries;
-//   guide[c] = m | flags, m (bits 0-11) the smallest entry with cdf[m] > c 2^(32 - gb), for the
-//              2^gb >= S / 2 cells: about one cell per two entries.  Against 2^gb >= S cells the
-//              draws cost more (more cells hold several boundaries), but the guide builds faster,
-//              tables up to 2048 entries fit half the arena (one warp builds them, not the block) and
-//              more tables share a batch barrier: on the bench workload k_bulk takes 27.5 ms against
-//              28.9 ms (2^gb >= S / 4: 28.3 ms).  GUIDE_PURE when cdf[m] >= (c + 1) 2^(32 - gb), so
-//              every u in the cell
-//              maps to m; GUIDE_ONE when instead cdf[m + 1] >= (c + 1) 2^(32 - gb), so u maps to m or
-//              m + 1 by one comparison; neither: two or more entries end inside the cell (a "tail"
-//              cell of the distribution), resolved by a binary search between guide[c] and
-//              guide[c + 1].
-// P(k) is FP32: the Loader form at every ANCHOR-th entry and the recursion P(k) = P(k-1) lambda / k
-// in between (__fdividef: at most 2 ulp per step, so under 32 ulp of drift before the next anchor).
-// Each thread takes E consecutive entries; the guide is the merge of the cdf values with the cell
-// starts, split evenly over the threads (merge path), so no thread waits on another's long run of
-// cells or entries.
+//              two zeros before it and 2^32 - 1 after it let a draw look at its neighbours.
+// A draw is a binary search of the whole table.  A guide over 2^gb cells of u (the first entry of each
+// cell, and a flag where at most one entry ends in it) answers most draws with two loads instead of
+// log2 S, but costs more to build than it saves and a third of the arena: with it the kernel takes
+// 15.8 / 16.9 / 19.7 / 25.0 ms at 100 / 200 / 512 / 1000 realizations of the 91x81x101 grid with 40
+// frequencies, without it 7.4 / 8.8 / 11.9 / 20.1 ms (3.1 -> 2.24 ms on 30^3 with 20 frequencies and 1000
+// realizations), with the other changes named below.
+// P(k) is FP32: the Loader form at the start of a run and every ANCHOR-th entry after it, the recursion
+// P(k) = P(k-1) lambda / k in between (__fdividef: at most 2 ulp per step, so under 32 ulp of drift
+// before the next anchor).  A table is cut into 32 runs of equal length (128 for the largest): the runs
+// fix where the anchors lie, and so the table's bits, whichever thread evaluates them.
 
-// q of the entries m0 .. m1 - 1 into cdf[m]; returns their sum, which stays below 2^31 (a thread's
-// entries span at most 1/32 of the table, well under half the probability)
-__device__ __forceinline__ unsigned table_pmf(const Tile &s, int j, unsigned int *cdf, int m0, int m1) {
-    const int k_lo = s.tb_klo[j], lam_int = s.lam_int[j];
-    const float frac = s.frac[j], lamf = s.lamf[j];
-    unsigned local = 0;
-    for (int a = m0; a < m1; a += ANCHOR) {
-        float kf = (float)(k_lo + a);   // exact: k < 2^24
-        float p = pmf_f32(k_lo + a, lam_int, frac, lamf);
-        unsigned q = __float2uint_rn(p * 0x1.0p32f);
-        cdf[a] = q;
-        local += q;
-        const int n = min(ANCHOR, m1 - a);
+// log2 of the number of cells of u for which a table of S entries was once cut; they decide only which
+// of the two background sums a draw joins (crowded below), and so the sums' last FP32 bits
+__device__ __forceinline__ int cell_bits(int S) { return max(1, 31 - __clz(S - 1)); }
+
+// How a table is cut: 2^lg runs of E entries, each of `sub` units of at most ANCHOR entries; unit
+// (k << lg) + r is run r's k-th (units side by side are equally long)
+struct TableCut {
+    int lg, E, sub;
+};
+__device__ __forceinline__ TableCut table_cut(int S) {
+    TableCut c;
+    c.lg = S > WIDE_RUNS ? 7 : 5;
+    c.E = (S + (1 << c.lg) - 1) >> c.lg;
+    c.sub = (c.E + ANCHOR - 1) / ANCHOR;
+    return c;
+}
+// entries [m0, m1) of run r's k-th unit (possibly none, at the table's end)
+__device__ __forceinline__ void unit_span(const TableCut &c, int S, int r, int k, int &m0, int &m1) {
+    m0 = r * c.E + k * ANCHOR;
+    m1 = min(min(m0 + ANCHOR, (r + 1) * c.E), S);
+}
+// The tables of list entries at .. at + K - 1, as many as fit the arena, built by the whole block; returns
+// K.  Work is shared out over all tables of the batch, so a large table and many small ones alike keep
+// every warp busy:
+//   1. a thread per unit (a run's up to ANCHOR entries after an anchor): P(k) and the unit's running sums;
+//   2. a warp per table: the units' totals (their last entries) scanned into the sums before them;
+//   3. a thread per unit again: the sum before it added to its entries.
+// Instruction issue and fetch bound it (0.6-0.7 of the issue slots; a warp-per-table form and one that
+// finished short tables in their warp's registers both lost 10-20% to barriers and instruction misses),
+// so the loops are barely unrolled and the cut is shifts: a table's units fill whole warps, which find
+// their table by one ballot.
+__device__ __forceinline__ int build_tables(Tile &s, int at, int n_table) {
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    int K;
+    {   // every warp forms the batch alike
+        const bool in = at + lane < n_table;
+        const int S = in ? s.tb_S[s.list[KIND_TABLE][at + lane]] : 2;
+        const TableCut c = table_cut(S);
+        const int words = in ? S + TABLE_PAD : 0, units = in ? c.sub << c.lg : 0;
+        int wsum = words, usum = units;
 #pragma unroll
-        for (int i = 1; i < ANCHOR; i++) {
-            if (i < n) {
-                kf += 1.0f;
-                p *= __fdividef(lamf, kf);
-                q = __float2uint_rn(p * 0x1.0p32f);
-                cdf[a + i] = q;
-                local += q;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int w = __shfl_up_sync(0xffffffffu, wsum, o), u = __shfl_up_sync(0xffffffffu, usum, o);
+            if (lane >= o) {
+                wsum += w;
+                usum += u;
             }
         }
-    }
-    return local;
-}
-
-// running sums of the thread's entries on top of base (the 64-bit sum of every earlier entry),
-// saturated at 2^32 - 1 with 32-bit arithmetic
-__device__ __forceinline__ void table_prefix(unsigned int *cdf, int m0, int m1, unsigned long long base) {
-    const bool full = base >= 0xFFFFFFFFull;
-    const unsigned b32 = full ? 0xFFFFFFFFu : (unsigned)base;
-    const unsigned room = full ? 0u : (unsigned)(0xFFFFFFFFull - base);
-    unsigned run = 0;
-    for (int m = m0; m < m1; m++) {
-        run += cdf[m];
-        cdf[m] = b32 + min(run, room);
-    }
-}
-
-// the guide cells from the finished cdf: thread t of nthr walks diagonals [d0, d1) of the merge of
-// cdf[0 .. S-1] with the cell starts c 2^shift (a cdf value goes first on ties)
-__device__ __forceinline__ void table_guide(const unsigned int *cdf, unsigned short *guide, int S, int gb, int t,
-                                            int nthr) {
-    const int shift = 32 - gb, nc = 1 << gb;
-    const int total = S + nc;
-    const int D = (total + nthr - 1) / nthr;
-    const int d0 = min(t * D, total), d1 = min(d0 + D, total);
-    int lo = max(0, d0 - nc), hi = min(d0, S);   // cdf values among the first d0 merged elements
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (cdf[mid] <= ((unsigned)(d0 - 1 - mid) << shift)) lo = mid + 1;
-        else hi = mid;
-    }
-    int m = lo, c = d0 - lo;
-    unsigned am = cdf[min(m, S - 1)], an = cdf[min(m + 1, S - 1)];   // cdf[m] and cdf[m + 1]
-    for (int d = d0; d < d1 && c < nc; d++) {
-        if (am <= ((unsigned)c << shift)) {   // m < S - 1: cdf[S - 1] = 2^32 - 1 exceeds every cell start
-            m++;
-            am = an;
-            an = cdf[min(m + 1, S - 1)];
-        } else {
-            unsigned code = (unsigned)m;
-            if ((am >> shift) > (unsigned)c) code |= GUIDE_PURE;
-            else if (m + 1 < S && (an >> shift) > (unsigned)c) code |= GUIDE_ONE;
-            guide[c] = (unsigned short)code;
-            c++;
+        const unsigned fit = __ballot_sync(0xffffffffu, in && wsum <= ARENA_WORDS && usum <= UNIT_MAX);
+        K = __ffs(~fit) - 1;   // entries fit up to the first that does not (the first always does)
+        if (K < 0) K = 32;
+        __syncthreads();       // the previous batch is drawn (and its offsets are no longer read)
+        if (warp == 0) {
+            s.b_off[lane] = wsum - words + 2;
+            s.b_unit[lane] = usum - units;
+            if (lane == K - 1) s.b_unit[K] = usum;
         }
     }
-}
-
-// one warp builds the table of bin j (tables of at most HALF_WORDS words)
-__device__ void build_table_warp(const Tile &s, int j, unsigned int *cdf, unsigned short *guide, int lane) {
-    const int S = s.tb_S[j];
-    const int E = (S + 31) >> 5;
-    const int m0 = min(lane * E, S), m1 = min(m0 + E, S);
-    const unsigned local = table_pmf(s, j, cdf, m0, m1);
-    unsigned long long incl = local;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const unsigned long long y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
+    __syncthreads();
+    const int U = s.b_unit[K];
+    // a warp's 32 units are of one table (runs come in 32s): the last that starts at or below its first unit
+    const int first_l = lane < K ? s.b_unit[lane] : 0x7FFFFFFF;
+    // ---- 1
+#pragma unroll 1
+    for (int u = t; u < U; u += RB) {
+        const int i = __popc(__ballot_sync(0xffffffffu, first_l <= u - lane)) - 1, j = s.list[KIND_TABLE][at + i], S = s.tb_S[j];
+        const TableCut c = table_cut(S);
+        const int lu = u - s.b_unit[i], k = lu >> c.lg, r = lu & ((1 << c.lg) - 1);
+        int m0, m1;
+        unit_span(c, S, r, k, m0, m1);
+        if (m0 >= m1) continue;
+        unsigned int *cdf = s.u.arena + s.b_off[i];
+        const int k0 = (int)s.tb_klo[j] + m0;
+        const float lamf = s.lamf[j];
+        float kf = (float)k0;   // exact: k < 2^24
+        // P 2^32 (a power of two moves no rounding)
+        float p = pmf_f32(k0, s.lam_int[j], s.frac[j], lamf) * 0x1.0p32f;
+        unsigned run = __float2uint_rn(p);   // below 2^31: a unit is a small part of the table
+        cdf[m0] = run;
+#pragma unroll 2
+        for (int m = m0 + 1; m < m1; m++) {
+            kf += 1.0f;
+            p *= __fdividef(lamf, kf);
+            run += __float2uint_rn(p);
+            cdf[m] = run;
+        }
     }
-    table_prefix(cdf, m0, m1, incl - local);
-    if (m0 < S && m1 == S) cdf[S - 1] = 0xFFFFFFFFu;
-    __syncwarp();
-    table_guide(cdf, guide, S, s.tb_gb[j], lane, 32);
-    __syncwarp();
-}
-
-// the whole block builds the table of bin j (large tables); starts and ends with a barrier-protected
-// table
-__device__ void build_table_block(Tile &s, int j, unsigned int *cdf, unsigned short *guide) {
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int S = s.tb_S[j];
-    const int E = (S + RB - 1) / RB;
-    const int m0 = min(t * E, S), m1 = min(m0 + E, S);
-    const unsigned local = table_pmf(s, j, cdf, m0, m1);
-    unsigned long long incl = local;
+    __syncthreads();
+    // ---- 2
+#pragma unroll 1
+    for (int i = warp; i < K; i += NWARP) {
+        const int S = s.tb_S[s.list[KIND_TABLE][at + i]];
+        const TableCut c = table_cut(S);
+        unsigned int *cdf = s.u.arena + s.b_off[i];
+        if (lane < TABLE_PAD) cdf[lane < 2 ? lane - 2 : S] = lane < 2 ? 0u : 0xFFFFFFFFu;
+        const int per = 1 << (c.lg - 5);   // consecutive runs per lane
+        unsigned long long sum = 0;
+#pragma unroll 1
+        for (int q = 0; q < per; q++)
+#pragma unroll 1
+            for (int k = 0; k < c.sub; k++) {
+                int m0, m1;
+                unit_span(c, S, lane * per + q, k, m0, m1);
+                if (m1 > m0) sum += cdf[m1 - 1];
+            }
+        unsigned long long before = sum;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const unsigned long long y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long y = __shfl_up_sync(0xffffffffu, before, o);
+            if (lane >= o) before += y;
+        }
+        before -= sum;
+        unsigned int *base = s.ubase + s.b_unit[i];
+#pragma unroll 1
+        for (int q = 0; q < per; q++)
+#pragma unroll 1
+            for (int k = 0; k < c.sub; k++) {
+                int m0, m1;
+                unit_span(c, S, lane * per + q, k, m0, m1);
+                base[(k << c.lg) + lane * per + q] = before < 0xFFFFFFFFull ? (unsigned)before : 0xFFFFFFFFu;
+                if (m1 > m0) before += cdf[m1 - 1];
+            }
     }
-    if (lane == 31) s.scan[warp] = incl;
     __syncthreads();
-    unsigned long long base = incl - local;
-    for (int w = 0; w < warp; w++) base += s.scan[w];
-    table_prefix(cdf, m0, m1, base);
-    if (m0 < S && m1 == S) cdf[S - 1] = 0xFFFFFFFFu;
+    // ---- 3
+#pragma unroll 1
+    for (int u = t; u < U; u += RB) {
+        const int i = __popc(__ballot_sync(0xffffffffu, first_l <= u - lane)) - 1, S = s.tb_S[s.list[KIND_TABLE][at + i]];
+        const TableCut c = table_cut(S);
+        const int lu = u - s.b_unit[i], k = lu >> c.lg, r = lu & ((1 << c.lg) - 1);
+        int m0, m1;
+        unit_span(c, S, r, k, m0, m1);
+        unsigned int *cdf = s.u.arena + s.b_off[i];
+        const unsigned b = s.ubase[u], room = 0xFFFFFFFFu - b;   // saturated at 2^32 - 1
+#pragma unroll 1
+        for (int m = m0; m < m1; m++) cdf[m] = b + min(cdf[m], room);
+        if (m1 > m0 && m1 == S) cdf[S - 1] = 0xFFFFFFFFu;
+    }
     __syncthreads();
-    table_guide(cdf, guide, S, s.tb_gb[j], t, RB);
-    __syncthreads();
+    return K;
 }
-
-// arena words of a table-kind bin: S cdf entries and 2^gb u16 guide cells
-__device__ __forceinline__ int table_words(const Tile &s, int j) { return s.tb_S[j] + (1 << (s.tb_gb[j] - 1)); }
 
 // SORTED: lam / h are the gathered (F, B) arrays and qpos gives each realization's first bulk
 // position; otherwise lam / h are the (B, F) grids and every bin belongs to the bulk.
@@ -899,52 +934,55 @@ __device__ __forceinline__ int table_words(const Tile &s, int j) { return s.tb_S
 // shared memory [k][slot][thread], each term n * h2fdf * 2^100 * p_k * 2^-e_k (e_k the frexp exponent
 // of max |p_k|, so every scaled parameter is at most 1).
 constexpr int NPAR = 7;
-constexpr size_t PAR_SMEM = sizeof(float) * (NPAR * RB + 2 * NPAR * RPT * RB);
+template <int NS>
+constexpr size_t PAR_SMEM = sizeof(float) * (NPAR * RB + 2 * NPAR * NS * RB);
 
+template <int NS>
 __device__ __forceinline__ void add_par(float *psm, int sl, int t, int j, float n) {
     const float *pw = psm;
     float *pacc = psm + NPAR * RB;
-    float *pcomp = pacc + NPAR * RPT * RB;
+    float *pcomp = pacc + NPAR * NS * RB;
 #pragma unroll
     for (int k = 0; k < NPAR; k++) {
-        const int o = (k * RPT + sl) * RB + t;
+        const int o = (k * NS + sl) * RB + t;
         float acc = pacc[o], comp = pcomp[o];
-        kahan_add(acc, comp, n * pw[k * RB + j]);
+        kahan_add(acc, comp, n, pw[k * RB + j]);
         pacc[o] = acc;
         pcomp[o] = comp;
     }
 }
 
 // Shared state of one k_bulk block (static shared memory of the kernels that run bulk_block).
-template <bool PARAMS>
+template <bool PARAMS, int NS>
 struct BulkShared {
     Tile s;
-    typename std::conditional<PARAMS, SlotsKahan, SlotsPlain>::type st;
+    typename std::conditional<PARAMS, SlotsKahan<NS>, SlotsPlain<NS>>::type st;
     int q_min_s, q_max_s;
 };
 
 // One k_bulk block's work: chunk c (tiles c, c + nchunk, ...) of frequency f for the realizations of
-// group rg (rg * RB * RPT + thread + i * RB, i < RPT), written to part[c][f][r].  Every shared word it
+// group rg (rg * RB * NS + thread + i * RB, i < NS), written to part[c][f][r].  Every shared word it
 // reads it first writes, so a block may run it for several (c, f, rg) in turn.
-template <bool SORTED, bool PARAMS>
+template <bool SORTED, bool PARAMS, int NS>
 __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa, const double *__restrict__ lam_in,
                                            const double *__restrict__ h_in, const int *__restrict__ qpos,
                                            double *__restrict__ part, int *d_status, const int c, const int f,
-                                           const int rg, BulkShared<PARAMS> &sh, float *psm) {
+                                           const int rg, BulkShared<PARAMS, NS> &sh, float *psm) {
     Tile &s = sh.s;
     auto &st = sh.st;
     int &q_min_s = sh.q_min_s;
     int &q_max_s = sh.q_max_s;
+    constexpr int NCALL = (NS + 3) / 4;   // Philox calls a bin
     const int t = threadIdx.x;
     const int lane = t & 31, warp = t >> 5;
-    const int r0 = rg * RB * RPT + t;
+    const int r0 = rg * RB * NS + t;
     int rpt = 0;   // realizations of this thread: r0 + i * RB, i < rpt
-    while (rpt < RPT && r0 + rpt * RB < a.nr) rpt++;
+    while (rpt < NS && r0 + rpt * RB < a.nr) rpt++;
     // register accumulators for the passes with a fixed realization slot
-    float acc_r[RPT], comp_r[RPT];
+    float acc_r[NS], comp_r[NS];
     int qmin = 0x7FFFFFFF, qmax = 0;
 #pragma unroll
-    for (int i = 0; i < RPT; i++) {
+    for (int i = 0; i < NS; i++) {
         acc_r[i] = 0.0f;
         comp_r[i] = 0.0f;
         slot_zero(st, i, t);
@@ -956,7 +994,7 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
         }
     }
     if (PARAMS) {
-        for (int o = t; o < 2 * NPAR * RPT * RB; o += RB) psm[NPAR * RB + o] = 0.0f;
+        for (int o = t; o < 2 * NPAR * NS * RB; o += RB) psm[NPAR * RB + o] = 0.0f;
     }
     if (t < 16) s.lgam[t] = c_lgam[t];
     if (t == 0) {
@@ -1028,20 +1066,20 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
             const int pos = s.pos[j];
             const float hs = s.hs[j];
             const unsigned int *row = s.u.thr[j];
-            uint4 wv[RPT / 4];   // every call issued first: independent round chains interleave
+            uint4 wv[NCALL];   // every call issued first: independent round chains interleave
 #pragma unroll
-            for (int call = 0; call < RPT / 4; call++) {
+            for (int call = 0; call < NCALL; call++) {
                 uint4 ctr = ctr0;
                 ctr.x = (uint32_t)pos;
                 ctr.w |= W_SMALL | (uint32_t)call;
                 wv[call] = philox(ctr, a.key);
             }
 #pragma unroll
-            for (int call = 0; call < RPT / 4; call++) {
+            for (int call = 0; call < NCALL; call++) {
                 if (4 * call >= rpt) break;
                 const uint4 w = wv[call];
 #pragma unroll
-                for (int m = 0; m < 4; m++) {
+                for (int m = 0; m < (NS < 4 ? NS : 4); m++) {
                     const int sl = 4 * call + m;
                     const uint32_t u = (m == 0) ? w.x : (m == 1) ? w.y : (m == 2) ? w.z : w.w;
                     if (sl >= rpt) continue;
@@ -1049,22 +1087,20 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
                     const unsigned wd = row[u >> 27];
                     const int n = ((u & 0x07FFFFFFu) < (wd >> 5)) ? (int)(u >> 27) : (int)(wd & 31u);
                     if (n != 0 && (!check || pos >= __ldg(q_row + sl * RB))) {
-                        kahan_add(acc_r[sl], comp_r[sl], (float)n * hs);
-                        if (PARAMS) add_par(psm, sl, t, j, (float)n);
+                        kahan_add(acc_r[sl], comp_r[sl], (float)n, hs);
+                        if (PARAMS) add_par<NS>(psm, sl, t, j, (float)n);
                     }
                 }
             }
         }
 
-        // ---- table kind: inversion tables of up to BATCH_MAX bins at a time.  Tables that fit half the
-        // arena are built one per warp into the half the draws are not reading: batch k + 1 is built
-        // while batch k is drawn, one barrier per batch.  Larger tables use the whole arena and the
-        // whole block.  Four realizations per Philox call.
+        // ---- table kind: inversion tables, as many at a time as fit the arena, built by the whole block
+        // (build_tables) and then drawn.  Four realizations per Philox call.
         const int n_table = kind_count(s, KIND_TABLE);
         if (n_table > 0) {
-            // largest tables first: big tables come in batches of their own and the many small ones
-            // share later batches, where the warps' builds balance (rank sort of the tile's list;
-            // the draws are keyed by bin, so only the summation order of the background changes)
+            // largest tables first, so that the many small ones fill the last batches (rank sort of the
+            // tile's list; the draws are keyed by bin, so only the summation order of the background
+            // depends on it)
             int jt = 0, rank = 0;
             if (t < n_table) {
                 jt = s.list[KIND_TABLE][t];
@@ -1077,157 +1113,62 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
             __syncthreads();   // every entry is read before any is moved
             if (t < n_table) s.list[KIND_TABLE][rank] = (unsigned char)jt;
             __syncthreads();   // the sorted list is complete before any batch is formed
-            int li = 0;
-            int cur_li = 0, cur_K = 0, cur_half = 0;
-            bool cur_big = false;
-            // the batch starting at list entry li (same on every thread)
-            auto form = [&](int at, int &K, bool &big) {
-                big = table_words(s, s.list[KIND_TABLE][at]) > HALF_WORDS;
-                K = 1;
-                if (big) return;
-                int used = table_words(s, s.list[KIND_TABLE][at]);
-                while (at + K < n_table && K < BATCH_MAX) {
-                    const int words = table_words(s, s.list[KIND_TABLE][at + K]);
-                    if (words > HALF_WORDS || used + words > HALF_WORDS) break;
-                    used += words;
-                    K++;
-                }
-            };
-            // build a small batch into a half, each table by the least-loaded warp (by entries)
-            auto build_small = [&](int at, int K, int half) {
-                int load[NWARP] = {};
-                int off = half * HALF_WORDS;
+#pragma unroll 1
+            for (int at = 0; at < n_table;) {
+                const int K = build_tables(s, at, n_table);   // (waits for the small-lambda pass, too)
+#pragma unroll 1
                 for (int i = 0; i < K; i++) {
                     const int j = s.list[KIND_TABLE][at + i];
-                    int wmin = 0;
-#pragma unroll
-                    for (int w = 1; w < NWARP; w++)
-                        if (load[w] < load[wmin]) wmin = w;
-                    load[wmin] += s.tb_S[j];
-                    if (wmin == warp)
-                        build_table_warp(s, j, s.u.arena + off, (unsigned short *)(s.u.arena + off + s.tb_S[j]), lane);
-                    off += table_words(s, j);
-                }
-            };
-            form(li, cur_K, cur_big);
-            cur_li = li;
-            li += cur_K;
-            __syncthreads();   // the arena is free (the small-lambda pass is done)
-            if (cur_big) {
-                const int j = s.list[KIND_TABLE][cur_li];
-                build_table_block(s, j, s.u.arena, (unsigned short *)(s.u.arena + s.tb_S[j]));
-            } else {
-                build_small(cur_li, cur_K, 0);
-                __syncthreads();
-            }
-#pragma unroll 1
-            while (true) {
-                // prebuild the next batch when both it and the current one are small
-                int nxt_li = li, nxt_K = 0;
-                bool nxt_big = false;
-                if (!cur_big && li < n_table) {
-                    form(li, nxt_K, nxt_big);
-                    if (nxt_big) nxt_K = 0;
-                    else {
-                        li += nxt_K;
-                        build_small(nxt_li, nxt_K, cur_half ^ 1);
-                    }
-                }
-                // draw the current batch
-                int off = cur_big ? 0 : cur_half * HALF_WORDS;
-#pragma unroll 1
-                for (int i = 0; i < cur_K; i++) {
-                    const int j = s.list[KIND_TABLE][cur_li + i];
                     const int pos = s.pos[j];
                     const float hs = s.hs[j];
-                    const int k_lo = s.tb_klo[j], S = s.tb_S[j], gb = s.tb_gb[j], shift = 32 - gb;
-                    const unsigned int *cdf = s.u.arena + off;
-                    const unsigned short *guide = (const unsigned short *)(s.u.arena + off + S);
-                    off += table_words(s, j);
-                    uint4 wv[RPT / 4];   // every call issued first: independent round chains interleave
+                    const int k_lo = s.tb_klo[j], S = s.tb_S[j];
+                    const unsigned cell = ~0u << (32 - cell_bits(S));
+                    const unsigned int *cdf = s.u.arena + s.b_off[i];
 #pragma unroll
-                    for (int call = 0; call < RPT / 4; call++) {
+                    for (int call = 0; call < NCALL; call++) {
                         uint4 ctr = ctr0;
                         ctr.x = (uint32_t)pos;
                         ctr.w |= W_TABLE | (uint32_t)call;
-                        wv[call] = philox(ctr, a.key);
-                    }
-                    // Straight-line lookups (no data-dependent branch, so the eight draws
-                    // interleave): a pure cell answers from the guide, a one-boundary cell with one
-                    // comparison.  Draws in tail cells (a few percent) are marked and finished after
-                    // the bin's other draws by a binary search inside the cell.
-                    unsigned pend = 0;
+                        const uint4 w = philox(ctr, a.key);
+                        constexpr int G = NS < 4 ? NS : 4;
+                        uint32_t uc[G];
+                        int e[G];
 #pragma unroll
-                    for (int call = 0; call < RPT / 4; call++) {
-                        if (4 * call >= rpt) break;
-                        const uint4 w = wv[call];
-#pragma unroll
-                        for (int m = 0; m < 4; m++) {
-                            const int sl = 4 * call + m;
-                            const uint32_t u = (m == 0) ? w.x : (m == 1) ? w.y : (m == 2) ? w.z : w.w;
-                            if (sl >= rpt) continue;
-                            const uint32_t uc = min(u, 0xFFFFFFFEu);   // below cdf[S - 1]
-                            const unsigned g = guide[uc >> shift];
-                            int e = (int)(g & GUIDE_M);
-                            if (!HGB_IN_BOUNDS(e < S - 1 || !(g & GUIDE_ONE), d_status)) e = 0;
-                            if (g & GUIDE_ONE) e += (uc >= cdf[e]) ? 1 : 0;
-                            if (!HGB_IN_BOUNDS(e < S, d_status)) e = S - 1;
-                            const bool tail = !(g & (GUIDE_PURE | GUIDE_ONE));
-                            pend |= tail ? (1u << sl) : 0u;
-                            if (!tail && (!check || pos >= __ldg(q_row + sl * RB))) {
-                                kahan_add(acc_r[sl], comp_r[sl], (float)(k_lo + e) * hs);
-                                if (PARAMS) add_par(psm, sl, t, j, (float)(k_lo + e));
-                            }
+                        for (int g = 0; g < G; g++) {
+                            uc[g] = min(g == 0 ? w.x : g == 1 ? w.y : g == 2 ? w.z : w.w, 0xFFFFFFFEu);
+                            e[g] = 0;
                         }
-                    }
-                    if (__any_sync(0xffffffffu, pend != 0)) {
-                        // the lane's tail draws in turn; their slot is data dependent, so the sums
-                        // go to the shared-memory Kahan accumulators
+                        // entries at or below u, between e and e + n - 1 (below S: cdf[S - 1] > u); the
+                        // halves follow S, so a step's addresses spread over the banks
 #pragma unroll 1
-                        while (pend) {
-                            const int sl = __ffs(pend) - 1;
-                            pend &= pend - 1;
-                            const uint4 w = (sl < 4) ? wv[0] : wv[RPT / 4 - 1];
-                            const int q4 = sl & 3;
-                            const uint32_t u = (q4 == 0) ? w.x : (q4 == 1) ? w.y : (q4 == 2) ? w.z : w.w;
-                            const uint32_t uc = min(u, 0xFFFFFFFEu);
-                            const unsigned cell = uc >> shift;
-                            int lo = (int)(guide[cell] & GUIDE_M);
-                            int hi = (cell + 1 < (1u << gb)) ? (int)(guide[cell + 1] & GUIDE_M) : S - 1;
-                            if (!HGB_IN_BOUNDS(lo <= hi && hi < S, d_status)) lo = hi = S - 1;
-                            while (lo < hi) {   // cdf[hi] > uc throughout
-                                const int mid = (lo + hi) >> 1;
-                                if (uc >= cdf[mid]) lo = mid + 1;
-                                else hi = mid;
-                            }
-                            if (!check || pos >= __ldg(q_row + sl * RB)) {
-                                add_bg(st, sl, t, (float)(k_lo + lo) * hs);
-                                if (PARAMS) add_par(psm, sl, t, j, (float)(k_lo + lo));
+                        for (int n = S; n > 1;) {
+                            const int half = n >> 1;
+#pragma unroll
+                            for (int g = 0; g < G; g++)
+                                if (cdf[e[g] + half - 1] <= uc[g]) e[g] += half;
+                            n -= half;
+                        }
+#pragma unroll
+                        for (int g = 0; g < G; g++) {
+                            const int sl = 4 * call + g;
+                            if (!HGB_IN_BOUNDS(e[g] < S, d_status)) e[g] = S - 1;
+                            // crowded: two or more entries end inside u's cell (the table's end counts)
+                            const unsigned int *v = cdf + e[g];
+                            const bool b0 = ((v[0] ^ uc[g]) & cell) == 0, b1 = ((v[1] ^ uc[g]) & cell) == 0;
+                            const bool a0 = v[-1] > (uc[g] & cell), a1 = v[-2] > (uc[g] & cell);
+                            if (sl < rpt && (!check || pos >= __ldg(q_row + sl * RB))) {
+                                const float n = (float)(k_lo + e[g]);
+                                const bool crowded = b0 ? a0 || b1 : a1;
+                                if (crowded) add_bg(st, sl, t, n, hs);
+                                else kahan_add(acc_r[sl], comp_r[sl], n, hs);
+                                if (PARAMS) add_par<NS>(psm, sl, t, j, n);
                             }
                         }
                     }
                 }
-                __syncthreads();   // the current batch is drawn and the next one built
-                if (nxt_K > 0) {
-                    cur_li = nxt_li;
-                    cur_K = nxt_K;
-                    cur_big = false;
-                    cur_half ^= 1;
-                    continue;
-                }
-                if (li >= n_table) break;
-                form(li, cur_K, cur_big);
-                cur_li = li;
-                li += cur_K;
-                if (cur_big) {
-                    const int j = s.list[KIND_TABLE][cur_li];
-                    build_table_block(s, j, s.u.arena, (unsigned short *)(s.u.arena + s.tb_S[j]));
-                } else {
-                    cur_half = 0;
-                    build_small(cur_li, cur_K, 0);
-                    __syncthreads();
-                }
+                at += K;
             }
+            __syncthreads();   // the arena is free for the sparse pass
         }
 
         // ---- PTRS32: one loop per lane over its realizations, two attempts per Philox call
@@ -1255,8 +1196,8 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
                 it++;
                 if (k >= 0) {
                     if (!check || pos >= __ldg(q_row + sl * RB)) {
-                        add_bg(st, sl, t, (float)k * hs);
-                        if (PARAMS) add_par(psm, sl, t, j, (float)k);
+                        add_bg(st, sl, t, (float)k, hs);
+                        if (PARAMS) add_par<NS>(psm, sl, t, j, (float)k);
                     }
                     sl++;
                 } else if (it >= MAX_PTRS_ITERS) {
@@ -1264,8 +1205,8 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
                     const float kfix = floorf(pc.lamf + 0.5f);
                     for (; sl < rpt; sl++)
                         if (!check || pos >= __ldg(q_row + sl * RB)) {
-                            add_bg(st, sl, t, kfix * hs);
-                            if (PARAMS) add_par(psm, sl, t, j, kfix);
+                            add_bg(st, sl, t, kfix, hs);
+                            if (PARAMS) add_par<NS>(psm, sl, t, j, kfix);
                         }
                 }
             }
@@ -1287,7 +1228,7 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
                 ctr.x = (uint32_t)pos;
                 ctr.w |= W_SKIP;
                 int i = 0;
-                for (int step = 0; step < 2 * RPT + 2; step++) {
+                for (int step = 0; step < 2 * NS + 2; step++) {
                     uint4 cc = ctr;
                     cc.w |= (uint32_t)step;
                     const uint4 w = philox(cc, a.key);
@@ -1298,8 +1239,8 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
                     i += (int)gap;
                     const int n = truncated_count_f32(lf, u24(w.z), d_status);
                     if (!check || pos >= __ldg(q_row + i * RB)) {
-                        add_bg(st, i, t, (float)n * hs);
-                        add_par(psm, i, t, j, (float)n);
+                        add_bg(st, i, t, (float)n, hs);
+                        add_par<NS>(psm, i, t, j, (float)n);
                     }
                     i++;
                     if (i >= rpt) break;
@@ -1314,8 +1255,8 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
             // depend on the order the threads reach them (4096 times the largest term of headroom;
             // a realization sees a few events per tile).  Each thread then folds its slots into its
             // Kahan sums.
-            unsigned long long *sub = reinterpret_cast<unsigned long long *>(s.u.arena);   // [RPT * RB]
-            const int nr_blk = min(RB * RPT, a.nr - rg * RB * RPT);
+            unsigned long long *sub = reinterpret_cast<unsigned long long *>(s.u.arena);   // [NS * RB]
+            const int nr_blk = min(RB * NS, a.nr - rg * RB * NS);
             int runs = 0, e_hs = -1000;
             if (t < n_sparse) {
                 const int js = s.list[KIND_SPARSE][t];
@@ -1334,7 +1275,7 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
             __syncthreads();   // the arena and the scan words are free
             if (lane == 31) s.scan[warp] = ((unsigned long long)(unsigned)(e_hs + 2048) << 32) | (unsigned)incl;
 #pragma unroll
-            for (int i = 0; i < RPT; i++) sub[i * RB + t] = 0ull;
+            for (int i = 0; i < NS; i++) sub[i * RB + t] = 0ull;
             __syncthreads();
             int before = 0, total = 0, e_max = -1000;
 #pragma unroll
@@ -1383,8 +1324,8 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
             }
             __syncthreads();
 #pragma unroll
-            for (int i = 0; i < RPT; i++)
-                if (i < rpt) kahan_add(acc_r[i], comp_r[i], (float)ldexp((double)sub[i * RB + t], -fx_shift));
+            for (int i = 0; i < NS; i++)
+                if (i < rpt) kahan_add(acc_r[i], comp_r[i], (float)ldexp((double)sub[i * RB + t], -fx_shift), 1.0f);
         }
 
         // ---- PTRS64 / Normal (real-valued counts, cyutils.pyx:1327-1330 / :887-891); without the
@@ -1403,24 +1344,24 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
                 ctr.w |= W_WIDE | ((uint32_t)sl << 8);
                 const double num = (lam > NORMAL_THRESH) ? normal_draw(ctr, a.key, lam) : ptrs64(ctr, a.key, lam, d_status);
                 if (!check || pos >= __ldg(q_row + sl * RB)) {
-                    add_bg(st, sl, t, (float)(num * (double)hs));
-                    if (PARAMS) add_par(psm, sl, t, j, (float)num);
+                    add_bg(st, sl, t, (float)(num * (double)hs), 1.0f);
+                    if (PARAMS) add_par<NS>(psm, sl, t, j, (float)num);
                 }
             }
         }
     }
     const bool part_ok = HGB_IN_BOUNDS(c < a.nchunk && f < a.nf, d_status);
 #pragma unroll
-    for (int i = 0; i < RPT; i++)
+    for (int i = 0; i < NS; i++)
         if (i < rpt && part_ok)
             part[((long)c * a.nf + f) * a.nr + r0 + (long)i * RB] =
                 (((double)acc_r[i] - (double)comp_r[i]) + slot_value(st, i, t)) * HSCALE_INV;
     if (PARAMS) {
         const float *pacc = psm + NPAR * RB;
-        const float *pcomp = pacc + NPAR * RPT * RB;
+        const float *pcomp = pacc + NPAR * NS * RB;
         for (int k = 0; k < NPAR; k++)
             for (int i = 0; i < rpt; i++) {
-                const int o = (k * RPT + i) * RB + t;
+                const int o = (k * NS + i) * RB + t;
                 pa.part_par[(((long)c * NPAR + k) * a.nf + f) * a.nr + r0 + (long)i * RB] =
                     ldexp(((double)pacc[o] - (double)pcomp[o]) * HSCALE_INV, pa.scale_log2[k]);
             }
@@ -1428,14 +1369,14 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
 }
 
 // grid (nchunk, nf, realization groups): block (c, f, rg) runs bulk_block for itself
-template <bool SORTED, bool PARAMS>
-__global__ void __launch_bounds__(RB, PARAMS ? 2 : BULK_BLOCKS_PER_SM) k_bulk(BulkArgs a, ParArgs pa, const double *__restrict__ lam_in,
+template <bool SORTED, bool PARAMS, int NS>
+__global__ void __launch_bounds__(RB, PARAMS ? (NS == 1 ? 5 : NS == 2 ? 4 : NS == 4 ? 3 : 2) : BULK_BLOCKS_PER_SM) k_bulk(BulkArgs a, ParArgs pa, const double *__restrict__ lam_in,
                                                           const double *__restrict__ h_in,
                                                           const int *__restrict__ qpos, double *__restrict__ part,
                                                           int *d_status) {
-    __shared__ BulkShared<PARAMS> sh;
+    __shared__ BulkShared<PARAMS, NS> sh;
     extern __shared__ float psm[];   // PARAMS only: PAR_SMEM bytes
-    bulk_block<SORTED, PARAMS>(a, pa, lam_in, h_in, qpos, part, d_status, blockIdx.x, blockIdx.y, blockIdx.z, sh, psm);
+    bulk_block<SORTED, PARAMS, NS>(a, pa, lam_in, h_in, qpos, part, d_status, blockIdx.x, blockIdx.y, blockIdx.z, sh, psm);
 }
 
 // ---- 4c. many samples in one launch.  A sample's realization stage is the (chunk, frequency,
@@ -1455,7 +1396,10 @@ struct BulkJob {
 __global__ void __launch_bounds__(RB, BULK_BLOCKS_PER_SM) k_bulk_multi(const BulkJob *__restrict__ jobs,
                                                                        const int4 *__restrict__ items, int n_items,
                                                                        int *next) {
-    __shared__ BulkShared<false> sh;
+    __shared__ union {   // the blocks' width follows the item's sample (see with_slots)
+        BulkShared<false, RPT> w8;
+        BulkShared<false, 4> w4;
+    } sh;
     __shared__ int s_item;
     int it = next ? -1 : (int)blockIdx.x;
     while (true) {
@@ -1468,7 +1412,10 @@ __global__ void __launch_bounds__(RB, BULK_BLOCKS_PER_SM) k_bulk_multi(const Bul
         if (it >= n_items) break;
         const int4 w = items[it];
         const BulkJob &J = jobs[w.x];   // read where used (L1), not held in registers
-        bulk_block<true, false>(J.a, ParArgs{}, J.lam, J.h, J.q, J.part, J.status, w.y, w.z, w.w, sh, nullptr);
+        if (J.a.nr <= 4 * RB)
+            bulk_block<true, false, 4>(J.a, ParArgs{}, J.lam, J.h, J.q, J.part, J.status, w.y, w.z, w.w, sh.w4, nullptr);
+        else
+            bulk_block<true, false, RPT>(J.a, ParArgs{}, J.lam, J.h, J.q, J.part, J.status, w.y, w.z, w.w, sh.w8, nullptr);
         if (!next) break;
     }
 }
@@ -1678,6 +1625,19 @@ size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 int n_rgroups(int nr) { return (int)hgb::ceil_div(nr, (long)RB * RPT); }
 
+// Launches with the fewest realizations per thread (1, 2, 4 or RPT) that hold all of them in one block:
+// the draws are those of RPT, the slots beyond them are not there.  Fewer slots are fewer sums in
+// registers (56-64 a thread against 71, so 8 blocks fit an SM, not 7), one Philox call a bin instead of
+// two, and no lookups that are thrown away: 14.6 -> 11.5 ms at 100 realizations of the 91x81x101 grid
+// with 40 frequencies, 1.47 -> 1.29 ms of 30^3 with 20, the tables as before.
+template <typename F>
+void with_slots(int nr, F &&launch) {
+    if (nr <= RB) launch(std::integral_constant<int, 1>());
+    else if (nr <= 2 * RB) launch(std::integral_constant<int, 2>());
+    else if (nr <= 4 * RB) launch(std::integral_constant<int, 4>());
+    else launch(std::integral_constant<int, RPT>());
+}
+
 // Waves of resident k_bulk blocks (BULK_BLOCKS_PER_SM per SM) that the chunk count aims for; set by
 // hgb_set_bulk_waves.
 // A block's cost depends strongly on its frequency (the lowest frequencies hold most of the
@@ -1855,7 +1815,9 @@ int hgb_loudest_hc_from_sorted_ex(const double *number, const double *h2fdf, lon
     cudaMemsetAsync(a.wide_flag, 0, sizeof(int), st);
     dim3 grid((unsigned)a.nchunk, (unsigned)n_freq, (unsigned)n_rgroups(nreals));
     if ((rc = bulk_event(0, st))) return rc;
-    k_bulk<true, false><<<grid, RB, 0, st>>>(a, ParArgs{}, lam_s, h_s, q, part, d_status);
+    with_slots(nreals, [&](auto slots) {
+        k_bulk<true, false, decltype(slots)::value><<<grid, RB, 0, st>>>(a, ParArgs{}, lam_s, h_s, q, part, d_status);
+    });
     if ((rc = hgb::check_launch())) return rc;
     if ((rc = bulk_event(1, st))) return rc;
     k_bulk_wide<true><<<grid, RB, 0, st>>>(a, lam_s, h_s, q, part, d_status);
@@ -2078,13 +2040,18 @@ int hgb_loudest_hc_and_par_from_sorted(const double *number, const double *h2fdf
     BulkArgs a = bulk_args(n_bins, n_freq, nreals, L.nchunk, seed, 0u);
     a.wide_flag = (int *)(w + L.off_flag);   // unused: the parameter kernel draws its wide bins itself
     dim3 grid((unsigned)a.nchunk, (unsigned)n_freq, (unsigned)n_rgroups(nreals));
-    cudaError_t err = cudaFuncSetAttribute(k_bulk<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)PAR_SMEM);
+    cudaError_t err = cudaSuccess;
+    with_slots(nreals, [&](auto slots) {
+        constexpr int NS = decltype(slots)::value;
+        err = cudaFuncSetAttribute(k_bulk<true, true, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)PAR_SMEM<NS>);
+        if (err == cudaSuccess)
+            k_bulk<true, true, NS><<<grid, RB, PAR_SMEM<NS>, st>>>(a, pa, lam_s, h_s, q, part, d_status);
+    });
     if (err != cudaSuccess) {
         hgb::set_cuda_error(err);
         return HGB_ERR_CUDA;
     }
-    k_bulk<true, true><<<grid, RB, PAR_SMEM, st>>>(a, pa, lam_s, h_s, q, part, d_status);
     if ((rc = hgb::check_launch())) return rc;
     k_bg_reduce_par<<<(unsigned)hgb::ceil_div(nfr, 256), 256, 0, st>>>(a.nchunk, nfr, bgp, part, pa, hc2bg, bgpar);
     return hgb::check_launch();
@@ -2129,7 +2096,10 @@ int hgb_sam_poisson_gwb(const double *number, const double *hc2, long n_bins, in
     a.wide_flag = (int *)((char *)workspace + align256(sizeof(double) * (size_t)a.nchunk * n_freq * nreals));
     cudaMemsetAsync(a.wide_flag, 0, sizeof(int), st);
     dim3 grid((unsigned)a.nchunk, (unsigned)n_freq, (unsigned)n_rgroups(nreals));
-    k_bulk<false, false><<<grid, RB, 0, st>>>(a, ParArgs{}, number, hc2, nullptr, (double *)workspace, d_status);
+    with_slots(nreals, [&](auto slots) {
+        k_bulk<false, false, decltype(slots)::value>
+            <<<grid, RB, 0, st>>>(a, ParArgs{}, number, hc2, nullptr, (double *)workspace, d_status);
+    });
     int rc = hgb::check_launch();
     if (rc) return rc;
     k_bulk_wide<false><<<grid, RB, 0, st>>>(a, number, hc2, nullptr, (double *)workspace, d_status);
