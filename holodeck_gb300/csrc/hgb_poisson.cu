@@ -533,17 +533,23 @@ void launch_gather_sorted(const double *number, const double *h2fdf, const int32
 // ---- 2. cumulative expectation along the sorted bins: C[0] = 0, C[k + 1] = C[k] + max(lambda_k, 0)
 // (NaN counts as 0; with h_mask, bins whose h2fdf is zero count as 0 -- the parameter path skips
 // them).  Each frequency's bins are cut into CUM_SEG segments: k_cum_sum totals the segments,
-// k_cum_write scans each segment from the sum of the segments before it.
+// k_cum_write scans each segment from the sum of the segments before it.  The FP64 pipe bounds both (a
+// comparison costs it as much as an addition), so the terms are tested by their bits, and a warp whose
+// terms are all zero adds nothing: most of a population's bins are, and they sort to the end together.
+// 91x81x101 bins with 40 frequencies: 125 and 396 us before, 94 and 253 us now; 30^3 with 20: 10 and 76,
+// 13 and 9 (blocks of a segment's length, not 1024 threads); 181x161x201 with 100: 2.27 and 6.88, 1.25 and
+// 4.14 ms.
 constexpr int CUM_THREADS = 1024;
 constexpr int CUM_PER_THREAD = 4;
 constexpr int CUM_SEG = 64;   // segments per frequency: about 8 waves of scan blocks on 152 SMs at 40 frequencies
 
 __device__ __forceinline__ double cum_term(const double *lam, const double *mask, long k) {
-    double x = lam[k];
-    x = (x > 0.0) ? x : 0.0;
-    if (mask && mask[k] == 0.0) x = 0.0;
+    const double x = lam[k];
+    const bool pos = (unsigned long long)(__double_as_longlong(x) - 1) < 0x7FF0000000000000ull;   // 0 < x <= inf
+    if (!pos || (mask && (__double_as_longlong(mask[k]) << 1) == 0)) return 0.0;
     return x;
 }
+__device__ __forceinline__ bool nonzero_bits(double x) { return __double_as_longlong(x) != 0; }   // of a term
 
 __global__ void __launch_bounds__(256) k_cum_sum(long nb, const double *__restrict__ lam_s,
                                                  const double *__restrict__ h_mask, double *__restrict__ seg_tot) {
@@ -554,7 +560,19 @@ __global__ void __launch_bounds__(256) k_cum_sum(long nb, const double *__restri
     const double *lam = lam_s + (long)f * nb;
     const double *mask = h_mask ? h_mask + (long)f * nb : nullptr;
     double local = 0.0;
-    for (long k = k0 + t; k < k1; k += 256) local += cum_term(lam, mask, k);
+    for (long k = k0 + t; k < k1; k += 8 * 256) {   // eight loads in flight, added in order
+        double v[8];
+        bool any = false;
+#pragma unroll
+        for (int e = 0; e < 8; e++) {
+            v[e] = k + e * 256 < k1 ? cum_term(lam, mask, k + e * 256) : 0.0;
+            any |= nonzero_bits(v[e]);
+        }
+        if (any) {
+#pragma unroll
+            for (int e = 0; e < 8; e++) local += v[e];
+        }
+    }
     red[t] = local;
     __syncthreads();
     for (int o = 128; o > 0; o >>= 1) {
@@ -568,7 +586,7 @@ __global__ void __launch_bounds__(CUM_THREADS) k_cum_write(long nb, const double
                                                            const double *__restrict__ h_mask,
                                                            const double *__restrict__ seg_tot,
                                                            double *__restrict__ cum) {
-    __shared__ double wsum[CUM_THREADS / 32];
+    __shared__ double wsum[32], tot[CUM_SEG];
     __shared__ double carry_s;
     const int f = blockIdx.y, sg = blockIdx.x, t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const long seg = (nb + CUM_SEG - 1) / CUM_SEG;
@@ -576,30 +594,38 @@ __global__ void __launch_bounds__(CUM_THREADS) k_cum_write(long nb, const double
     const double *lam = lam_s + (long)f * nb;
     const double *mask = h_mask ? h_mask + (long)f * nb : nullptr;
     double *C = cum + (long)f * (nb + 1);
+    for (int j = t; j < sg; j += blockDim.x) tot[j] = seg_tot[(long)f * CUM_SEG + j];
+    if (t < 32) wsum[t] = 0.0;
+    __syncthreads();
     if (t == 0) {
         double c = 0.0;
-        for (int j = 0; j < sg; j++) c += seg_tot[(long)f * CUM_SEG + j];
+        for (int j = 0; j < sg; j++) c += tot[j];
         carry_s = c;
         if (sg == 0) C[0] = 0.0;
     }
     __syncthreads();
-    const long span = (long)CUM_THREADS * CUM_PER_THREAD;
+    const long span = (long)blockDim.x * CUM_PER_THREAD;
     for (long base = k0; base < k1; base += span) {
         double v[CUM_PER_THREAD];
-        double local = 0.0;
         const long kk = base + (long)t * CUM_PER_THREAD;
+        bool any = false;
 #pragma unroll
         for (int e = 0; e < CUM_PER_THREAD; e++) {
             const long k = kk + e;
-            const double x = (k < k1) ? cum_term(lam, mask, k) : 0.0;
-            v[e] = x;
-            local += x;
+            v[e] = (k < k1) ? cum_term(lam, mask, k) : 0.0;
+            any |= nonzero_bits(v[e]);
         }
-        double incl = local;   // inclusive warp scan of the thread totals
+        any = __any_sync(0xffffffffu, any);
+        double local = v[0], incl = 0.0;
+        if (any) {
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            double y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += y;
+            for (int e = 1; e < CUM_PER_THREAD; e++) local += v[e];
+            incl = local;   // inclusive warp scan of the thread totals
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                double y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += y;
+            }
         }
         if (lane == 31) wsum[warp] = incl;
         __syncthreads();
@@ -614,15 +640,22 @@ __global__ void __launch_bounds__(CUM_THREADS) k_cum_write(long nb, const double
             wsum[lane] = wi - ws;   // exclusive warp offsets
         }
         __syncthreads();
-        double run = carry_s + wsum[warp] + (incl - local);
+        double run = carry_s + wsum[warp];
+        if (any) {
+            run += incl - local;
+#pragma unroll
+            for (int e = 0; e < CUM_PER_THREAD; e++) {
+                run += v[e];
+                v[e] = run;
+            }
+        }
 #pragma unroll
         for (int e = 0; e < CUM_PER_THREAD; e++) {
             const long k = kk + e;
-            run += v[e];
-            if (k < k1) C[k + 1] = run;
+            if (k < k1) C[k + 1] = any ? v[e] : run;
         }
         __syncthreads();
-        if (t == CUM_THREADS - 1) carry_s = run;
+        if (t == blockDim.x - 1) carry_s = run;
         __syncthreads();
     }
 }
@@ -634,7 +667,11 @@ int cumulate(long nb, int nf, const double *lam_s, const double *h_mask, double 
     k_cum_sum<<<grid, 256, 0, st>>>(nb, lam_s, h_mask, seg_tot);
     int rc = hgb::check_launch();
     if (rc) return rc;
-    k_cum_write<<<grid, CUM_THREADS, 0, st>>>(nb, lam_s, h_mask, seg_tot, cum);
+    // whole warps for a segment, all of them from one pass's span on (a short segment's missing warps would
+    // add zeros)
+    const long seg = hgb::ceil_div(nb, (long)CUM_SEG);
+    const unsigned threads = (unsigned)std::min<long>(CUM_THREADS, 32 * hgb::ceil_div(seg, 32L * CUM_PER_THREAD));
+    k_cum_write<<<grid, threads, 0, st>>>(nb, lam_s, h_mask, seg_tot, cum);
     return hgb::check_launch();
 }
 
