@@ -442,6 +442,7 @@ __device__ __forceinline__ double shape_outer(double y, double p, PowPlan plan) 
 // with 20: 443 and 147 us.
 constexpr int WK_THREADS = 256;
 constexpr unsigned WK_NONE = 0xFFFFFFFFu, WK_NAN = 0xFFFFFFFEu;
+constexpr double WK_SCALE = 0x1.0p40;   // of the FP64 frequencies, some 1e-10 Hz: keeps the bracket's products in range
 
 struct WalkShape {
     int cb;       // cells walked together
@@ -509,6 +510,7 @@ __global__ void __launch_bounds__(WK_THREADS, 3) k_dbn_2pwl_walk(
     float *frf = ftf + NF;
     unsigned *code = (unsigned *)(frf + S + 1);   // [rows][wk_stride(NF)] step | interval << 16
     __shared__ int s_first;
+    __shared__ unsigned queue[WK_THREADS / 32][64];
     const int nqb = (a.n_mrat + ws.qc - 1) / ws.qc;
     const int ii = blockIdx.x / nqb, q0 = (blockIdx.x % nqb) * ws.qc, q1 = min(q0 + ws.qc, a.n_mrat);
     const double mt = mtot[ii];
@@ -518,7 +520,7 @@ __global__ void __launch_bounds__(WK_THREADS, 3) k_dbn_2pwl_walk(
         ag[i] = agrid_g[i];
     }
     for (int f = t; f < NF; f += WK_THREADS) {
-        ft[f] = fobs[f];
+        ft[f] = fobs[f] * WK_SCALE;
         ftf[f] = (float)fobs[f];
     }
     // nodes: separation, and in the steps' arrays for now the hardening shape and 1 / separation^3
@@ -537,8 +539,9 @@ __global__ void __launch_bounds__(WK_THREADS, 3) k_dbn_2pwl_walk(
             const double r = hgb::fast_range(sp) ? hgb::fast_rsqrt(sp) : 1.0 / sqrt(sp);
             const double xx = sp * inv_rchar, r2 = r * r;
             sepa[s] = sp;
-            frst[s] = kf * (r2 * r);
-            frf[s] = (float)frst[s];
+            const double fr = kf * (r2 * r);
+            frst[s] = fr * WK_SCALE;
+            frf[s] = (float)fr;
             al[s] = shape_outer(1.0 + xx, -a.go + a.gi, a.p_outer) *
                     pow_planned(xx, pin, PowPlan{a.p_inner.kind, a.p_inner.n, !a.p_inner.neg});
             be[s] = r2 * r2 * r2;
@@ -656,56 +659,75 @@ __global__ void __launch_bounds__(WK_THREADS, 3) k_dbn_2pwl_walk(
             // ---- B
             double *rf = redz_final + (cell0 * NZ + row0) * NF;
             double *dn = diff_num + (cell0 * NZ + row0) * NF;
-            const int dr = WK_THREADS / NF, df = WK_THREADS - dr * NF;
-            int r = t / NF, f = t - r * NF;
-            while (r < nr) {
+            auto element = [&](unsigned packed) {   // row << 16 | target
+                const int r = (int)(packed >> 16), f = (int)(packed & 0xFFFFu);
                 const unsigned cd = code[r * stride + f];
                 double out_r = -1.0, out_t = 0.0;
-                if (cd == WK_NAN) {
-                    out_r = 0.0;
-                    out_t = base[r];
-                } else if (cd != WK_NONE) {
-                    int s = (int)(cd & 0xFFFFu), il = (int)(cd >> 16);
-                    const double *tc = tnb + (size_t)((row0 + r) / NZ) * (S + 1);
-                    const double gmt = base[r], ra = rage[(row0 + r) % NZ], target = ft[f];
-                    for (int go = 0; go <= S; go++) {   // at most one move in practice
-                        const double tl = tc[s] + gmt + ra, tr = tc[s + 1] + gmt + ra;
-                        if (__double_as_longlong(tl) > age_bits) break;
-                        while (il < NI - 2 && __double_as_longlong(ag[il + 1]) < __double_as_longlong(tl)) il++;
-                        while (il > 0 && __double_as_longlong(ag[il]) > __double_as_longlong(tl)) il--;
-                        const double zl = __fma_rn(tl - ag[il], sz[il], zg[il]);
-                        if (__double2hiint(zl) < 0) break;
-                        const double pl = 1.0 + zl, fl = frst[s];
-                        const double x = __fma_rn(target, pl, -fl);
-                        if (__double2hiint(x) < 0) {   // below the step
-                            if (s == first) break;
-                            s--;
-                            continue;
-                        }
-                        int ir = il;
-                        while (ir < NI - 2 && __double_as_longlong(ag[ir + 1]) < __double_as_longlong(tr)) ir++;
-                        double zr = __fma_rn(tr - ag[ir], sz[ir], zg[ir]);
-                        if (__double2hiint(zr) < 0) zr = 0.0;
-                        const double pr = 1.0 + zr, fr = frst[s + 1];
-                        const double y = __fma_rn(-target, pr, fr);
-                        if (__double2hiint(y) < 0) {   // above it
-                            if (s == S - 1) break;
-                            s++;
-                            continue;
-                        }
-                        const double den = __fma_rn(fr, pl, -(fl * pr)) * 0x1.0p40;   // frequencies of 1e-10 Hz and less
-                        const double num = (tr - tl) * (x * 0x1.0p40) * pr;
-                        const double tt = hgb::fast_range(den) ? __fma_rn(num, hgb::fast_rcp(den), tl) : tl + num / den;
-                        if (!(__double_as_longlong(tt) > age_bits)) {
-                            out_r = hgb::f32_to_f64_scaled((float)il, 0);   // the interval the evaluation starts from
-                            out_t = tt;
-                        }
-                        break;
+                int s = (int)(cd & 0xFFFFu), il = (int)(cd >> 16);
+                const double *tc = tnb + (size_t)((row0 + r) / NZ) * (S + 1);
+                const double gmt = base[r], ra = rage[(row0 + r) % NZ], target = ft[f];
+                for (int go = 0; go <= S; go++) {   // at most one move in practice
+                    const double tl = tc[s] + gmt + ra, tr = tc[s + 1] + gmt + ra;
+                    if (__double_as_longlong(tl) > age_bits) break;
+                    while (il < NI - 2 && __double_as_longlong(ag[il + 1]) < __double_as_longlong(tl)) il++;
+                    while (il > 0 && __double_as_longlong(ag[il]) > __double_as_longlong(tl)) il--;
+                    const double zl = __fma_rn(tl - ag[il], sz[il], zg[il]);
+                    if (__double2hiint(zl) < 0) break;
+                    const double pl = 1.0 + zl, fl = frst[s];
+                    const double x = __fma_rn(target, pl, -fl);
+                    if (__double2hiint(x) < 0) {   // below the step
+                        if (s == first) break;
+                        s--;
+                        continue;
                     }
+                    int ir = il;
+                    while (ir < NI - 2 && __double_as_longlong(ag[ir + 1]) < __double_as_longlong(tr)) ir++;
+                    double zr = __fma_rn(tr - ag[ir], sz[ir], zg[ir]);
+                    if (__double2hiint(zr) < 0) zr = 0.0;
+                    const double pr = 1.0 + zr, fr = frst[s + 1];
+                    const double y = __fma_rn(-target, pr, fr);
+                    if (__double2hiint(y) < 0) {   // above it
+                        if (s == S - 1) break;
+                        s++;
+                        continue;
+                    }
+                    const double den = __fma_rn(fr, pl, -(fl * pr));
+                    const double num = (tr - tl) * x * pr;
+                    const double tt = hgb::fast_range(den) ? __fma_rn(num, hgb::fast_rcp(den), tl) : tl + num / den;
+                    if (!(__double_as_longlong(tt) > age_bits)) {
+                        out_r = hgb::f32_to_f64_scaled((float)il, 0);   // the interval the evaluation starts from
+                        out_t = tt;
+                    }
+                    break;
                 }
                 const long e = (long)r * NF + f;
                 rf[e] = out_r;
                 dn[e] = out_t;
+            };
+            const int dr = WK_THREADS / NF, df = WK_THREADS - dr * NF;
+            int r = t / NF, f = t - r * NF;
+            int held = 0;   // collected elements of this warp
+            unsigned *q = queue[warp];
+            for (int i0 = 32 * warp; i0 < nr * NF; i0 += WK_THREADS) {
+                const unsigned cd = r < nr ? code[r * stride + f] : WK_NONE;
+                const bool live = cd < WK_NAN;
+                if (r < nr && !live) {
+                    const long e = (long)r * NF + f;
+                    rf[e] = cd == WK_NAN ? 0.0 : -1.0;
+                    dn[e] = cd == WK_NAN ? base[r] : 0.0;
+                }
+                const unsigned m = __ballot_sync(0xffffffffu, live);
+                if (live) q[held + __popc(m & ((1u << lane) - 1u))] = (unsigned)r << 16 | (unsigned)f;
+                held += __popc(m);
+                __syncwarp();
+                if (held >= 32) {
+                    element(q[lane]);
+                    held -= 32;
+                    const unsigned more = lane < held ? q[32 + lane] : 0u;
+                    __syncwarp();
+                    if (lane < held) q[lane] = more;
+                    __syncwarp();
+                }
                 r += dr;
                 f += df;
                 if (f >= NF) {
@@ -713,6 +735,8 @@ __global__ void __launch_bounds__(WK_THREADS, 3) k_dbn_2pwl_walk(
                     r++;
                 }
             }
+            if (lane < held) element(q[lane]);
+            __syncwarp();
         }
     }
 }
