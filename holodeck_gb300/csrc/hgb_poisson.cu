@@ -40,7 +40,7 @@
 //                             bin costs about one draw per event instead of one per lane
 //   SPARSE_MAX <= lambda < 10 a 32-column alias row per bin (n < 31 and the rest at 31): one
 //                             lookup and one comparison per draw; four realizations per Philox call
-//   10 <= lambda <= 47000     inversion by a binary search of a per-bin table over
+//   10 <= lambda <= 47000     inversion from a per-bin table over
 //                             lambda +- 7 sqrt(lambda) in shared memory; four realizations per
 //                             Philox call
 //   47000 < lambda < 2^22     PTRS, transformed rejection with squeeze (Hormann 1993, Insurance:
@@ -96,6 +96,7 @@ constexpr int UNIT_MAX = 512;            // units of work (see build_tables) of 
 constexpr int WIDE_RUNS = 2048;          // tables of more entries than this are cut into 128 runs, not 32
 constexpr int BULK_BLOCKS_PER_SM = 6;    // k_bulk residency that chunk counts assume (7 or 8 blocks fit; the chunks fix the sums' order)
 static_assert(ARENA_WORDS >= RB * (NT + 1), "the small-lambda rows share the arena");
+constexpr int QUANT_OCTAVES = 13, QUANT_CELLS = 8 * QUANT_OCTAVES;
 constexpr int ANCHOR = 16;               // Loader-form pmf every ANCHOR-th entry, the recursion between
 constexpr float TABLE_SIGMAS = 7.0f;     // the table covers lambda +- 7 sqrt(lambda) (tails < 1e-11)
 // draw families (counter .w high bits)
@@ -190,6 +191,8 @@ struct Tile {
     float hs[RB];                     // h2fdf * 2^100 (for the background sums)
     float frac[RB], lamf[RB];
     int lam_int[RB];
+    float2 quant[QUANT_CELLS + 1];         // see quantile_cells
+    float tb_c0[RB], tb_sd[RB];            // table kind: a quantile's index is c0 + sd z + z^2 / 6, nearly
     unsigned short tb_klo[RB], tb_S[RB];   // table kind: first count and entries
     int pos[RB];                      // sorted position (loudest) or grid index (gwb) of the bin
     unsigned char list[NKIND][RB];    // tile-local bin indices per kind, in bin order
@@ -296,6 +299,8 @@ __device__ void bin_setup(Tile &s, int j, int kind, double lam, double h) {
             const int k_lo = max(0, (int)floorf(lf - TABLE_SIGMAS * sd - 2.0f));
             const int S = min((int)ceilf(lf + TABLE_SIGMAS * sd + 6.0f) - k_lo + 1, TMAX);
             s.tb_klo[j] = (unsigned short)k_lo;   // below TABLE_MAX
+            s.tb_c0[j] = lf - (float)k_lo - 1.0f / 6.0f;
+            s.tb_sd[j] = sd;
             s.tb_S[j] = (unsigned short)S;
         }
     }
@@ -812,12 +817,15 @@ struct BulkArgs {
 //              (rounded to nearest); cdf[S - 1] = 2^32 - 1, so the mass outside the range (< 1e-11)
 //              goes to the end entries;
 //              two zeros before it and 2^32 - 1 after it let a draw look at its neighbours.
-// A draw is a binary search of the whole table.  A guide over 2^gb cells of u (the first entry of each
-// cell, and a flag where at most one entry ends in it) answers most draws with two loads instead of
-// log2 S, but costs more to build than it saves and a third of the arena: with it the kernel takes
-// 15.8 / 16.9 / 19.7 / 25.0 ms at 100 / 200 / 512 / 1000 realizations of the 91x81x101 grid with 40
-// frequencies, without it 7.4 / 8.8 / 11.9 / 20.1 ms (3.1 -> 2.24 ms on 30^3 with 20 frequencies and 1000
-// realizations), with the other changes named below.
+// A draw starts at the entry that the normal quantile with its first skewness term names (quantile_cells;
+// right for 95 to 99 of 100 draws, off by one for nearly all others) and walks from there.  Loads bound
+// the draws as much as issue does: a warp's 32 places in a table fall on the banks at random, three to
+// four to the fullest, so a draw takes two loads, and a third only where the cell test below needs it.
+// Before, a guide over 2^gb cells of u (the first entry of each cell, and a flag where at most one entry
+// ends in it) answered most draws with two loads, but cost more to build than it saved, and a third of
+// the arena.  91x81x101 grid, 40 frequencies, 100 / 200 / 512 / 1000 realizations: 15.8 / 16.9 / 19.7 /
+// 25.0 ms with guides, 7.4 / 8.8 / 11.9 / 20.1 ms with a binary search of the table instead (and the
+// changes named at build_tables and with_slots), 6.6 / 7.9 / 11.0 / 19.0 ms from the quantile.
 // P(k) is FP32: the Loader form at the start of a run and every ANCHOR-th entry after it, the recursion
 // P(k) = P(k-1) lambda / k in between (__fdividef: at most 2 ulp per step, so under 32 ulp of drift
 // before the next anchor).  A table is cut into 32 runs of equal length (128 for the largest): the runs
@@ -965,6 +973,26 @@ __device__ __forceinline__ int build_tables(Tile &s, int at, int n_table) {
     return K;
 }
 
+// The normal quantile z(v / 2^32) for v = f in [2^18, 2^31], eight cells to an octave, as intercept and
+// slope in f: within 0.002 of it.  Only the start of a search depends on it.
+__device__ __forceinline__ void quantile_cells(float2 *cell) {
+    for (int i = threadIdx.x; i <= QUANT_CELLS; i += RB) {
+        const int bits = (((127 + 31 - QUANT_OCTAVES) << 3) + i) << 20;
+        const float f0 = __int_as_float(bits), f1 = __int_as_float(bits + (1 << 20));
+        const float z0 = normcdfinvf(f0 * 0x1.0p-32f), z1 = normcdfinvf(f1 * 0x1.0p-32f);
+        const float slope = (z1 - z0) / (f1 - f0);
+        cell[i] = make_float2(fmaf(-f0, slope, z0), slope);
+    }
+}
+// z(u / 2^32), nearly (far too high in the 2^-13 tails)
+__device__ __forceinline__ float quantile(const float2 *cell, unsigned u) {
+    const int upper = (int)u >> 31;
+    const float f = (float)(int)(u ^ (unsigned)upper);   // to the nearer end
+    const int i = max((__float_as_int(f) >> 20) - ((127 + 31 - QUANT_OCTAVES) << 3), 0);
+    const float2 c = cell[i];
+    return __int_as_float(__float_as_int(fmaf(f, c.y, c.x)) ^ (upper & 0x80000000));
+}
+
 // SORTED: lam / h are the gathered (F, B) arrays and qpos gives each realization's first bulk
 // position; otherwise lam / h are the (B, F) grids and every bin belongs to the bulk.
 // Parameter path: the seven weighted background sums per realization, FP32 Kahan in dynamic
@@ -1034,6 +1062,7 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
         for (int o = t; o < 2 * NPAR * NS * RB; o += RB) psm[NPAR * RB + o] = 0.0f;
     }
     if (t < 16) s.lgam[t] = c_lgam[t];
+    quantile_cells(s.quant);
     if (t == 0) {
         q_min_s = 0x7FFFFFFF;
         q_max_s = 0;
@@ -1160,6 +1189,7 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
                     const float hs = s.hs[j];
                     const int k_lo = s.tb_klo[j], S = s.tb_S[j];
                     const unsigned cell = ~0u << (32 - cell_bits(S));
+                    const float c0 = s.tb_c0[j], sd = s.tb_sd[j];
                     const unsigned int *cdf = s.u.arena + s.b_off[i];
 #pragma unroll
                     for (int call = 0; call < NCALL; call++) {
@@ -1169,37 +1199,42 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
                         const uint4 w = philox(ctr, a.key);
                         constexpr int G = NS < 4 ? NS : 4;
                         uint32_t uc[G];
-                        int e[G];
+                        int e[G];   // entries at or below u
 #pragma unroll
                         for (int g = 0; g < G; g++) {
                             uc[g] = min(g == 0 ? w.x : g == 1 ? w.y : g == 2 ? w.z : w.w, 0xFFFFFFFEu);
-                            e[g] = 0;
-                        }
-                        // entries at or below u, between e and e + n - 1 (below S: cdf[S - 1] > u); the
-                        // halves follow S, so a step's addresses spread over the banks
-#pragma unroll 1
-                        for (int n = S; n > 1;) {
-                            const int half = n >> 1;
-#pragma unroll
-                            for (int g = 0; g < G; g++)
-                                if (cdf[e[g] + half - 1] <= uc[g]) e[g] += half;
-                            n -= half;
+                            const float z = quantile(s.quant, uc[g]);
+                            const float x = fmaf(z * z, 1.0f / 6.0f, fmaf(z, sd, c0));
+                            e[g] = min(max(__float2int_rn(x), 0), S - 1);
                         }
 #pragma unroll
                         for (int g = 0; g < G; g++) {
                             const int sl = 4 * call + g;
-                            if (!HGB_IN_BOUNDS(e[g] < S, d_status)) e[g] = S - 1;
-                            // crowded: two or more entries end inside u's cell (the table's end counts)
-                            const unsigned int *v = cdf + e[g];
-                            const bool b0 = ((v[0] ^ uc[g]) & cell) == 0, b1 = ((v[1] ^ uc[g]) & cell) == 0;
-                            const bool a0 = v[-1] > (uc[g] & cell), a1 = v[-2] > (uc[g] & cell);
-                            if (sl < rpt && (!check || pos >= __ldg(q_row + sl * RB))) {
-                                const float n = (float)(k_lo + e[g]);
-                                const bool crowded = b0 ? a0 || b1 : a1;
-                                if (crowded) add_bg(st, sl, t, n, hs);
-                                else kahan_add(acc_r[sl], comp_r[sl], n, hs);
-                                if (PARAMS) add_par<NS>(psm, sl, t, j, n);
+                            unsigned hi = cdf[e[g]], lo = cdf[e[g] - 1];
+                            if (hi <= uc[g] || lo > uc[g]) {   // one in a hundred, nearly always off by one
+                                while (hi <= uc[g]) {          // (cdf[S - 1] > u)
+                                    lo = hi;
+                                    hi = cdf[++e[g]];
+                                }
+                                while (lo > uc[g]) {           // (cdf[-1] = 0)
+                                    hi = lo;
+                                    lo = cdf[--e[g] - 1];
+                                }
                             }
+                            if (!HGB_IN_BOUNDS(e[g] >= 0 && e[g] < S, d_status)) e[g] = S - 1;
+                            // crowded: two or more entries end inside u's cell (the table's end counts)
+                            const bool b0 = ((hi ^ uc[g]) & cell) == 0, a0 = lo > (uc[g] & cell);
+                            bool crowded = b0 && a0;
+                            if (b0 != a0) {
+                                const unsigned next = cdf[b0 ? e[g] + 1 : e[g] - 2];
+                                crowded = ((next ^ uc[g]) & cell) == 0 && next != (uc[g] & cell);
+                            }
+                            bool on = sl < rpt;
+                            if (check && on) on = pos >= __ldg(q_row + sl * RB);
+                            const float n = (float)(k_lo + e[g]);
+                            if (on && !crowded) kahan_add(acc_r[sl], comp_r[sl], n, hs);
+                            if (on && crowded) add_bg(st, sl, t, n, hs);
+                            if (PARAMS && on) add_par<NS>(psm, sl, t, j, n);
                         }
                     }
                 }
