@@ -105,7 +105,10 @@ __global__ void k_gradients(hgb_scatter_plan P, const double *__restrict__ dens,
 // FP64 bounds a phase: 90 points of about 6 neighbours are 6 warps of 13 to 15 FP64 instructions on
 // four sub-partitions, 1900 of its 2400 cycles.  91 x 81 points, 101 slices: 4283 us one level at a
 // time, 1896 us with sweeps in flight (and 69 us for c); 181 x 161, 201 slices, where the slice exceeds
-// shared memory and its gradients stay in L2: 78.5 and 18.1 ms.
+// shared memory and its gradients stay in L2: 78.5 and 13.0 ms.  There the loads are the longer chain
+// and the second wave of blocks costs as much as the first, so with more slices than multiprocessors
+// (AHEAD off) two blocks of 128 registers share one and no entries are loaded ahead: 16.8 ms with, 201
+// slices, and 13.0 without, 304 slices 18.4 and 13.6; 152 slices 9.3 and 12.2.
 constexpr int PH_WARPS = 8;    // most warps of a block: two prefetched sets of entries need 200 registers
 constexpr int PH_RING = 16;    // sweeps whose test is open (at most HGB_SCATTER_STAGES + 1)
 constexpr int PH_DEG = HGB_SCATTER_DEG;
@@ -174,8 +177,8 @@ __device__ __forceinline__ bool ph_over(double d, double v, double tol, float to
     return over;
 }
 
-template <bool SMEM>
-__global__ void __launch_bounds__(32 * PH_WARPS, 1) k_gradients_ph(hgb_scatter_plan P, int nz,
+template <bool SMEM, bool AHEAD>
+__global__ void __launch_bounds__(32 * PH_WARPS, AHEAD ? 1 : 2) k_gradients_ph(hgb_scatter_plan P, int nz,
                                                                   const double *__restrict__ cvec,
                                                                   double *__restrict__ hist, double *grads,
                                                                   int *d_status) {
@@ -195,11 +198,11 @@ __global__ void __launch_bounds__(32 * PH_WARPS, 1) k_gradients_ph(hgb_scatter_p
     for (int p = t; p < n; p += blockDim.x) ((double2 *)g)[p] = make_double2(0.0, 0.0);
     if (t < PH_RING) s_over[t] = 0;
     __syncthreads();
-    // prefetch: a warp's points two phases ahead, their entries one phase ahead
+    // prefetch: a warp's points two phases ahead (one without AHEAD), their entries one phase ahead
     const int base0 = 16 * warp;
     PhPre nxt;
     nxt.info = ph_point(P, ptr[0], base0, lane);
-    ph_entries(P, ptr[0], base0, lane, cz, nxt);
+    if (AHEAD) ph_entries(P, ptr[0], base0, lane, cz, nxt);
     int f1 = nph > 1 ? 1 : 0;   // the next phase
     int4 info1 = ph_point(P, ptr[f1], base0, lane);
     bool converged = false;
@@ -207,10 +210,11 @@ __global__ void __launch_bounds__(32 * PH_WARPS, 1) k_gradients_ph(hgb_scatter_p
     for (int T = 0; k_end < 0; T++) {
         if (t == 0) s_over[(T + 1) & (PH_RING - 1)] = 0;   // sweep T + 1 starts after this pass
         for (int phase = 0; phase < nph; phase++) {
-            const PhPre cur = nxt;
             const int4 now = ptr[phase];
+            if (!AHEAD) ph_entries(P, now, base0, lane, cz, nxt);
+            const PhPre cur = nxt;
             nxt.info = info1;
-            ph_entries(P, ptr[f1], base0, lane, cz, nxt);
+            if (AHEAD) ph_entries(P, ptr[f1], base0, lane, cz, nxt);
             f1 = f1 + 1 < nph ? f1 + 1 : 0;
             info1 = ph_point(P, ptr[f1], base0, lane);
             for (int base = base0; base < now.z; base += 16 * nw) {
@@ -571,10 +575,13 @@ int hgb_add_scatter_to_masses(const hgb_scatter_plan *plan, double *dens, int n_
         nw = std::min(PH_WARPS, (nw + 3) / 4 * 4);
         const bool in_smem = gradients_smem(P, true) + 1024 <= (size_t)smem_optin;
         const size_t smem = gradients_smem(P, in_smem);
-        const void *fn = in_smem ? (const void *)k_gradients_ph<true> : (const void *)k_gradients_ph<false>;
-        if ((rc = hgb::ensure_dyn_smem(fn, smem))) return rc;
-        if (in_smem) k_gradients_ph<true><<<n_redz, 32 * nw, smem, st>>>(P, n_redz, cvec, hist, grads, d_status);
-        else k_gradients_ph<false><<<n_redz, 32 * nw, smem, st>>>(P, n_redz, cvec, hist, grads, d_status);
+        // more slices than multiprocessors, outside shared memory: two blocks side by side hide each
+        // other's loads, and no second wave remains
+        const auto fn = in_smem                        ? k_gradients_ph<true, true>
+                        : n_redz <= hgb::sm_count() ? k_gradients_ph<false, true>
+                                                       : k_gradients_ph<false, false>;
+        if ((rc = hgb::ensure_dyn_smem((const void *)fn, smem))) return rc;
+        fn<<<n_redz, 32 * nw, smem, st>>>(P, n_redz, cvec, hist, grads, d_status);
     } else {
         k_gradients<<<n_redz, 256, 0, st>>>(P, dens, n_redz, vals, grads, d_status);
     }
