@@ -1075,57 +1075,74 @@ __global__ void __launch_bounds__(GW_ROWS) k_dbn_gw(CyConst cc, const double *__
 // keeps the alpha and beta of a run of consecutive steps in registers.  Each cell's lanes share its Brent
 // state (an xor-butterfly leaves the same total in all of them); the root finding itself, one exp10 and
 // some fifty uniform FP64 operations a round, is shared by the warp's CPW cells, neighbours in the grid
-// that need about the same number of rounds.  The log10 separations are init - s dx, one rounding each.
+// that need about the same number of rounds.  A node's separation, shape and 1 / x^3 depend on the total
+// mass only, so a block evaluates them once for all its cells of one mass.  The log10 separations are
+// init - s dx, one rounding each.
 // (Separations as products of a few shared powers of ten would save another tenth of the time, and two
 // roundings that come out cubed: the norm's error doubles, 4e-17 to 9e-17, so each is its own exp10.)
 // The sum's grouping moves the lifetime by about 1e-16 relative, far below the root tolerance of 1e-3,
 // which the root follows unless a Brent comparison falls within that margin (checked against the
 // reference at 1e-10 in log10).  FP64 bounds it.  91 x 81 cells: 2822 us with one cell per warp and a
-// quotient per node and round, 841 us with four (896 and 1081 with two and one); general exponents
-// (two pow() a node) 3626 and 1769 us.
+// quotient per node and round, 841 us with four (896 and 1081 with two and one), 534 us with the nodes
+// shared; general exponents (two pow() a node) 3626, 1769 and 606 us.
 constexpr int NB_STEPS = 320;   // steps the kernel holds in registers
-
+constexpr int NB_WARPS = 4;     // of a block, which shares the nodes
 
 template <int CPW>
-__global__ void __launch_bounds__(32) k_hardening_norm_sub(CyConst cc, NormArgs a, const double *__restrict__ mtot,
+__global__ void __launch_bounds__(32 * NB_WARPS) k_hardening_norm_sub(CyConst cc, NormArgs a, const double *__restrict__ mtot,
                                                            const double *__restrict__ mrat, int n,
                                                            double *__restrict__ norm_log10,
                                                            double *__restrict__ norm, int *d_status) {
     constexpr int LPC = 32 / CPW, NL = NB_STEPS / LPC;   // lanes per cell, steps per lane
-    const int S = a.nsteps;
-    const int sub = threadIdx.x % LPC;
-    const int own = blockIdx.x * CPW + threadIdx.x / LPC;
-    const int cell = min(own, n - 1);   // a last, partly filled warp repeats its last cell
+    __shared__ double s_x[NB_STEPS + 1], s_r[NB_STEPS + 1], s_i[NB_STEPS + 1];   // nodes
+    __shared__ double s_al[NB_STEPS], s_be[NB_STEPS];                            // steps
+    __shared__ unsigned s_next;
+    const int S = a.nsteps, t = threadIdx.x;
+    const int sub = t % LPC;
+    const int own = blockIdx.x * (CPW * NB_WARPS) + t / LPC;
+    const int cell = min(own, n - 1);   // the last block repeats its last cell
     const double mt = mtot[cell], mr = mrat[cell];
     const double opq = 1.0 + mr;
     const double gw_k = -cc.c_dadt * (mt * mt * mt) * mr / (opq * opq);
-    const double dx = (a.sepa_init_log10 - log10(3.0 * HGB_CY_SCHW * mt)) / S;
-    const double inv_rchar = 1.0 / a.rchar;
     double al[NL], be[NL];
-    {
-        const double pin = 1.0 - a.gi;
-        double x0 = 0.0, r0 = 0.0, g0 = 0.0;   // the previous node: separation, hardening shape, GW rate
-        double sd = (double)(sub * NL);
+    // the nodes of one total mass at a time (a block of grid cells meets one or two), for all its cells
+    for (bool loaded = false;;) {
+        if (t == 0) s_next = 0xFFFFFFFFu;
+        __syncthreads();   // (and the previous mass's steps are read)
+        const unsigned first = __reduce_min_sync(0xffffffffu, loaded ? 0xFFFFFFFFu : (unsigned)cell);
+        if ((t & 31) == 0 && first != 0xFFFFFFFFu) atomicMin(&s_next, first);
+        __syncthreads();
+        const unsigned next = s_next;
+        if (next == 0xFFFFFFFFu) break;
+        const double mt_n = mtot[next];
+        const double dx = (a.sepa_init_log10 - log10(3.0 * HGB_CY_SCHW * mt_n)) / S;
+        const double inv_rchar = 1.0 / a.rchar, pin = 1.0 - a.gi;
+        for (int s = t; s <= S; s += 32 * NB_WARPS) {
+            const double x = exp10(__fma_rn(-(double)s, dx, a.sepa_init_log10));
+            const double xx = x * inv_rchar, x3 = x * x * x;
+            s_x[s] = x;
+            s_r[s] = shape_outer(1.0 + xx, -a.go + a.gi, a.p_outer) *
+                     pow_planned(xx, pin, PowPlan{a.p_inner.kind, a.p_inner.n, !a.p_inner.neg});
+            s_i[s] = hgb::fast_range(x3) ? hgb::fast_rcp(x3) : 1.0 / x3;
+        }
+        __syncthreads();
+        for (int s = t; s < S; s += 32 * NB_WARPS) {
+            const double w = s_x[s] - s_x[s + 1];
+            const double c = 0.5 * (hgb::fast_range(w) ? hgb::fast_rcp(w) : 1.0 / w);
+            s_al[s] = (s_r[s] + s_r[s + 1]) * c;
+            s_be[s] = (s_i[s] + s_i[s + 1]) * c;
+        }
+        __syncthreads();
+        if (!loaded && __double_as_longlong(mt) == __double_as_longlong(mt_n)) {
+            loaded = true;
 #pragma unroll
-        for (int k = 0; k <= NL; k++) {
-            const int s = sub * NL + k;
-            const double x1 = exp10(__fma_rn(-sd, dx, a.sepa_init_log10));
-            sd += 1.0;
-            const double xx = x1 * inv_rchar;
-            const double r1 = shape_outer(1.0 + xx, -a.go + a.gi, a.p_outer) *
-                              pow_planned(xx, pin, PowPlan{a.p_inner.kind, a.p_inner.n, !a.p_inner.neg});
-            const double x3 = x1 * x1 * x1;
-            const double g1 = hgb::fast_range(x3) ? gw_k * hgb::fast_rcp(x3) : gw_k / x3;
-            if (k > 0) {
-                const double w = x0 - x1;
-                const double c = 0.5 * (hgb::fast_range(w) ? hgb::fast_rcp(w) : 1.0 / w);
-                // steps beyond the last add 1e-60 s
-                al[k - 1] = s <= S ? (r0 + r1) * c : 0.0;
-                be[k - 1] = s <= S ? (g0 + g1) * c : 1e60;
+            for (int k = 0; k < NL; k++) {
+                // every LPC-th step is a lane's, so the lanes read side by side; steps beyond the last add
+                // 1e-60 s
+                const int s = k * LPC + sub;
+                al[k] = s < S ? s_al[s] : 0.0;
+                be[k] = s < S ? gw_k * s_be[s] : 1e60;
             }
-            x0 = x1;
-            r0 = r1;
-            g0 = g1;
         }
     }
 
@@ -1259,14 +1276,14 @@ int hgb_find_2pwl_hardening_norm(double target_time, const double *mtot, const d
                pow_plan(-gamma_outer + gamma_inner), pow_plan(gamma_inner - 1.0)};
     if (nsteps <= NB_STEPS) {
         cudaStream_t st = (cudaStream_t)stream;
-        // four cells a warp do least work, but below about one warp per sub-partition two are faster:
-        // 30 x 30 cells 246 and 153 us, 60 x 60 cells 496 and 558 us
-        if (n >= 4 * 4 * hgb::sm_count())
-            k_hardening_norm_sub<4><<<(unsigned)hgb::ceil_div(n, 4), 32, 0, st>>>(hgb::cy_const(), a, mtot, mrat, n,
-                                                                                  norm_log10, norm, d_status);
+        // four cells a warp do least work, but two spread further while their blocks leave
+        // multiprocessors idle: 30 x 30 cells 174 and 128 us, 40 x 40 cells 172 and 197 us
+        if (n > 2 * NB_WARPS * hgb::sm_count())
+            k_hardening_norm_sub<4><<<(unsigned)hgb::ceil_div(n, 4 * NB_WARPS), 32 * NB_WARPS, 0, st>>>(
+                hgb::cy_const(), a, mtot, mrat, n, norm_log10, norm, d_status);
         else
-            k_hardening_norm_sub<2><<<(unsigned)hgb::ceil_div(n, 2), 32, 0, st>>>(hgb::cy_const(), a, mtot, mrat, n,
-                                                                                  norm_log10, norm, d_status);
+            k_hardening_norm_sub<2><<<(unsigned)hgb::ceil_div(n, 2 * NB_WARPS), 32 * NB_WARPS, 0, st>>>(
+                hgb::cy_const(), a, mtot, mrat, n, norm_log10, norm, d_status);
         return hgb::check_launch();
     }
     unsigned blocks = (unsigned)hgb::ceil_div(n, wpb);
