@@ -29,6 +29,9 @@ def device(dev=None):
     return t.device("cuda" if dev is None else dev)
 
 
+_STAGED_BYTES = 32768   # host arrays up to here are uploaded without waiting for the stream
+
+
 def as_device(arr, dev=None, dtype=None):
     """Contiguous float64 (or `dtype`) CUDA tensor from a numpy array / tensor / scalar sequence."""
     t = torch()
@@ -36,7 +39,12 @@ def as_device(arr, dev=None, dtype=None):
     dev = device(dev)
     if isinstance(arr, t.Tensor):
         return arr.to(device=dev, dtype=dtype).contiguous()
-    return t.as_tensor(np.ascontiguousarray(arr), dtype=dtype, device=dev)
+    host = np.ascontiguousarray(arr)
+    if host.nbytes > _STAGED_BYTES:
+        return t.as_tensor(host, dtype=dtype, device=dev)
+    # A blocking upload waits for the stream's queued work, which a handful of edges needs not: a private
+    # pageable copy is staged by the driver before the call returns.
+    return t.from_numpy(np.array(host)).to(dtype).to(dev, non_blocking=True)
 
 
 def is_torch(x):

@@ -273,9 +273,14 @@ def run_model_grids(sam, hard, pta_dur=DEF_PTA_DUR, nfreqs=DEF_NUM_FBINS, nreals
         if log is not None:
             log.exception(err)
         raise RuntimeError(err)
-    redz_final, diff_num = sam._dbn_scheduled(hard, fobs_orb_cents, precision=precision)
-    edges = [sam.mtot, sam.mrat, sam.redz, fobs_orb_edges]
-    number, h2fdf = sam._number_and_strain(fobs_orb_edges, diff_num, redz_final, precision=precision)
+    pending = []
+    try:   # the scatter's check waits for the next one's host read
+        redz_final, diff_num = sam._dbn_scheduled(hard, fobs_orb_cents, precision=precision, pending=pending)
+        edges = [sam.mtot, sam.mrat, sam.redz, fobs_orb_edges]
+        number, h2fdf = sam._number_and_strain(fobs_orb_edges, diff_num, redz_final, precision=precision)
+    finally:
+        for check in pending:
+            check()
     if details_flag:
         data['static_binary_density'] = sam.static_binary_density
         data['number'] = D.to_host(number)

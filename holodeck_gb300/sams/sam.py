@@ -26,6 +26,12 @@ GPF_USES_MTOT = False        #: sam.py:58
 GMT_USES_MTOT = False        #: sam.py:59
 
 
+def _settle(pending):
+    """Run the checks that stages left for later, in order."""
+    for check in pending:
+        check()
+
+
 class Semi_Analytic_Model:
     """Semi-analytic model of MBH-binary populations on an (mtot, mrat, redz) grid (sam.py:66-234)."""
 
@@ -142,15 +148,26 @@ class Semi_Analytic_Model:
                N.ptr(rz), rz.numel(), N.ptr(dens), N.ptr(gmt_time), N.ptr(redz_prime), st.ptr, N.stream_handle())
         return dens, gmt_time, redz_prime
 
-    def _scatter_finish(self, dens, gmt_time, redz_prime):
-        """Scatter and stalled-bin zeroing in place; caches the final density on the instance."""
+    def _scatter_finish(self, dens, gmt_time, redz_prime, pending=None):
+        """Scatter and stalled-bin zeroing in place; caches the final density on the instance.  With a
+        list as ``pending`` the scatter's check is left to the caller (see add_scatter_to_masses_device);
+        one that raises drops the cached density."""
         scatter = self._mmbulge._scatter_dex
+        checks = None if pending is None else []
         if scatter > 0.0:
             from . import scatter as _scatter
-            _scatter.add_scatter_to_masses_device(self.mtot, self.mrat, dens, scatter)
+            _scatter.add_scatter_to_masses_device(self.mtot, self.mrat, dens, scatter, pending=checks)
         if redz_prime is not None:
             N.call("hgb_zero_stalled", N.ptr(dens), N.ptr(redz_prime), int(dens.numel()), N.stream_handle())
         self._density_t, self._gmt_time_t, self._redz_prime_t = dens, gmt_time, redz_prime
+        if checks:
+            def check():
+                try:
+                    _settle(checks)
+                except BaseException:
+                    self._density_t = self._gmt_time_t = self._redz_prime_t = None
+                    raise
+            pending.append(check)
         return dens
 
     @property
@@ -192,7 +209,7 @@ class Semi_Analytic_Model:
             return sam_cyutils.dbn_gw_device(fobs_orb, dens, mt, mr, redz_prime, cosmo=cosmo)
         raise ValueError(f"Unexpected `hard` value {hard}!")
 
-    def _dbn_2pwl_overlapped(self, hard, fobs_orb, precision="fp64"):
+    def _dbn_2pwl_overlapped(self, hard, fobs_orb, precision="fp64", pending=None):
         """_dbn_device for Fixed_Time_2PL_SAM on a fresh instance, with the separation-step walk (which
         needs gmt_time but not the density) on a second stream while a high-priority third stream
         applies the M-Mbulge scatter; the evaluation, which needs the final density, follows on the
@@ -217,7 +234,7 @@ class Semi_Analytic_Model:
         hi = D.side_stream("mbulge_scatter", main.device, priority=-1)
         hi.wait_event(static_done)
         with t.cuda.stream(hi), D.nvtx("hgb:mbulge_scatter"):
-            self._scatter_finish(dens, gmt_time, redz_prime)
+            self._scatter_finish(dens, gmt_time, redz_prime, pending=pending)
             scatter_done = t.cuda.Event()
             scatter_done.record(hi)
         for x in (dens, gmt_time, redz_prime):
@@ -230,11 +247,12 @@ class Semi_Analytic_Model:
         return sam_cyutils.dbn_2pwl_device(fobs_orb, hard, dens, mt, mr, rz, gmt_time, cosmo=self._cosmo, phase=2,
                                            out=(redz_final, diff_num), precision=precision)
 
-    def _dbn_scheduled(self, hard, fobs_orb, precision="fp64"):
-        """_dbn_device, overlapping the separation-step walk with the scatter where that applies."""
+    def _dbn_scheduled(self, hard, fobs_orb, precision="fp64", pending=None):
+        """_dbn_device, overlapping the separation-step walk with the scatter where that applies (whose
+        check then goes to the list ``pending``, if there is one)."""
         if (self._density_t is None and self._gmt is not None and isinstance(hard, hardening.Fixed_Time_2PL_SAM)
                 and self._mmbulge._scatter_dex > 0.0):
-            return self._dbn_2pwl_overlapped(hard, fobs_orb, precision=precision)
+            return self._dbn_2pwl_overlapped(hard, fobs_orb, precision=precision, pending=pending)
         return self._dbn_device(hard, fobs_orb, precision=precision)
 
     def dynamic_binary_number_at_fobs(self, hard, fobs_orb, use_cython=True, **kwargs):
@@ -259,17 +277,28 @@ class Semi_Analytic_Model:
         fobs_gw_cents = utils.midpoints(fobs_gw_edges)
         fobs_orb_edges = fobs_gw_edges / 2.0
         fobs_orb_cents = fobs_gw_cents / 2.0
-        with D.nvtx("hgb:density_scatter_dbn"):
-            redz_final, diff_num = self._dbn_scheduled(hard, fobs_orb_cents, precision=precision)
-        with D.nvtx("hgb:number_and_strain"):
-            number, h2fdf = self._number_and_strain(fobs_orb_edges, diff_num, redz_final, precision=precision)
-        with D.nvtx("hgb:realizations"):
-            if params:
-                edges = [self.mtot, self.mrat, self.redz, fobs_orb_edges]
-                return single_sources.ss_params_device(edges, redz_final, number, h2fdf, realize, loudest,
-                                                       seed=seed, replay=replay, order=order, cosmo=self._cosmo)
-            return single_sources.ss_realize_device(number, h2fdf, realize, loudest, seed=seed, replay=replay,
-                                                    order=order)
+        # every stage is launched before the first status is read, so the device does not wait for the
+        # host between stages (30^3 edges: a third of the call); the checks then run in stage order
+        pending = []
+        try:
+            with D.nvtx("hgb:density_scatter_dbn"):
+                redz_final, diff_num = self._dbn_scheduled(hard, fobs_orb_cents, precision=precision, pending=pending)
+            with D.nvtx("hgb:number_and_strain"):
+                st = D.StatusWord(redz_final.device)
+                number, h2fdf = self._number_and_strain(fobs_orb_edges, diff_num, redz_final, status=st,
+                                                        precision=precision)
+                pending.append(lambda: single_sources.check_redshift_status(st))
+            with D.nvtx("hgb:realizations"):
+                if params:
+                    edges = [self.mtot, self.mrat, self.redz, fobs_orb_edges]
+                    out = single_sources.ss_params_device(edges, redz_final, number, h2fdf, realize, loudest,
+                                                          seed=seed, replay=replay, order=order, cosmo=self._cosmo)
+                else:
+                    out = single_sources.ss_realize_device(number, h2fdf, realize, loudest, seed=seed,
+                                                           replay=replay, order=order)
+        finally:
+            _settle(pending)   # an earlier stage's failure before a later one's
+        return out
 
     def _number_and_strain(self, fobs_orb_edges, diff_num, redz_final, status=None, precision="fp64"):
         """Device (number, h2fdf) on the (M-1, Q-1, Z-1, F) bins.  With ``status`` the redshift check

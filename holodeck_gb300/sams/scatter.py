@@ -115,10 +115,13 @@ def clear_plan_cache():
         _PLANS.clear()
 
 
-def add_scatter_to_masses_device(mtot, mrat, dens, scatter, refine=4, tol=GRAD_TOL, maxiter=GRAD_MAXITER):
+def add_scatter_to_masses_device(mtot, mrat, dens, scatter, refine=4, tol=GRAD_TOL, maxiter=GRAD_MAXITER,
+                                 pending=None):
     """Scatter the device density tensor ``dens`` (M, Q, Z) in place.  ``tol`` / ``maxiter`` are the
     gradient solve's stopping rule and sweep limit (CloughTocher2DInterpolator's arguments of those
-    names; the reference uses their defaults).  Running out of sweeps warns, as scipy does."""
+    names; the reference uses their defaults).  Running out of sweeps warns, as scipy does.  With a
+    list as ``pending`` the check of the solve's status (a host read) is appended to it for the caller
+    to run; it holds what the kernels in flight use."""
     plan = device_plan(mtot, mrat, scatter, refine)
     struct = plan.struct
     if tol != GRAD_TOL or maxiter != GRAD_MAXITER:
@@ -134,10 +137,17 @@ def add_scatter_to_masses_device(mtot, mrat, dens, scatter, refine=4, tol=GRAD_T
     st = D.StatusWord(dens.device)
     N.call("hgb_add_scatter_to_masses", ctypes.byref(struct), N.ptr(dens), nz, N.ptr(ws), int(ws_bytes), st.ptr,
            N.stream_handle())
-    code = st.read()
-    N.check_bounds(code, "M-Mbulge scatter")
-    if code & N.STATUS_GRADIENT_NOT_CONVERGED:
-        warnings.warn("Gradient estimation did not converge, the results may be inaccurate")
+
+    def check(in_use=(plan, ws)):
+        code = st.read()
+        N.check_bounds(code, "M-Mbulge scatter")
+        if code & N.STATUS_GRADIENT_NOT_CONVERGED:
+            warnings.warn("Gradient estimation did not converge, the results may be inaccurate")
+
+    if pending is None:
+        check()
+    else:
+        pending.append(check)
     return dens
 
 
