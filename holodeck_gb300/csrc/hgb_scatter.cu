@@ -99,7 +99,7 @@ __global__ void k_gradients(hgb_scatter_plan P, const double *__restrict__ dens,
 // slice's values, k_scatter_rhs) is taken once per solve and M_ij (geometry) comes with the plan, so a
 // neighbour costs 4 fused multiply-adds instead of 6 and the 2x2 solve is gone.  Rounding differs
 // from k_gradients by regrouping only.
-// Two lanes per point, one per component: 16 points per warp.  A point with more than HGB_SCATTER_DEG
+// Two lanes per point, one per component, 16 points per warp, or four, a component's neighbours halved.  A point with more than HGB_SCATTER_DEG
 // neighbours (the hull's fans, up to 82) takes a warp: 16 lane pairs share its neighbours.  The static
 // entries of a warp's points in the next phase are loaded while the current phase computes.
 // FP64 bounds a phase: 90 points of about 6 neighbours are 6 warps of 13 to 15 FP64 instructions on
@@ -109,7 +109,8 @@ __global__ void k_gradients(hgb_scatter_plan P, const double *__restrict__ dens,
 // and the second wave of blocks costs as much as the first, so with more slices than multiprocessors
 // (AHEAD off) two blocks of 128 registers share one and no entries are loaded ahead: 16.8 ms with, 201
 // slices, and 13.0 without, 304 slices 18.4 and 13.6; 152 slices 9.3 and 12.2.
-constexpr int PH_WARPS = 8;    // most warps of a block: two prefetched sets of entries need 200 registers
+// most warps of a block, by registers: two sets of entries of eight neighbours take 200 a thread
+__host__ __device__ constexpr int ph_warps(bool ahead, int split) { return ahead && split == 2 ? 16 : 8; }
 constexpr int PH_RING = 16;    // sweeps whose test is open (at most HGB_SCATTER_STAGES + 1)
 constexpr int PH_DEG = HGB_SCATTER_DEG;
 
@@ -132,27 +133,31 @@ __global__ void __launch_bounds__(256) k_scatter_rhs(hgb_scatter_plan P, const d
     cvec[(long)z * n + p] = make_double2(__fma_rn(q[1], sy, q[0] * sx), __fma_rn(q[3], sy, q[2] * sx));
 }
 
-struct PhPre {   // a lane's point (16 per warp, two lanes each) and its row of M
+template <int SPLIT>
+struct PhPre {   // a lane's point (16 / SPLIT per warp) and its part of the row of M
     int4 info;   // point, stage, neighbours (-1: no point), first entry
-    int nbr[PH_DEG];
-    double2 m[PH_DEG];
+    int nbr[PH_DEG / SPLIT];
+    double2 m[PH_DEG / SPLIT];
     double c;
 };
 
 // lane's point of chunk `base` of a phase (points with few neighbours): what ph_entries needs
+template <int SPLIT>
 __device__ __forceinline__ int4 ph_point(const hgb_scatter_plan &P, const int4 ph, int base, int lane) {
-    const int q = base + (lane >> 1);
+    const int q = base + lane / (2 * SPLIT);
     return q < ph.z ? __ldg((const int4 *)P.ph_info + ph.x + q) : make_int4(0, 0, -1, 0);
 }
 
+template <int SPLIT>
 __device__ __forceinline__ void ph_entries(const hgb_scatter_plan &P, const int4 ph, int base, int lane,
-                                           const double *cz, PhPre &x) {
+                                           const double *cz, PhPre<SPLIT> &x) {
     if (x.info.z < 0) return;
-    x.c = __ldg(cz + 2 * (ph.x + base + (lane >> 1)) + (lane & 1));
+    const int part = (lane >> 1) & (SPLIT - 1);
+    x.c = part ? 0.0 : __ldg(cz + 2 * (ph.x + base + lane / (2 * SPLIT)) + (lane & 1));
 #pragma unroll
-    for (int e = 0; e < PH_DEG; e++) {
-        if (e < x.info.z) {
-            const long k = x.info.w + (long)e * ph.z;
+    for (int e = 0; e < PH_DEG / SPLIT; e++) {
+        if (SPLIT * e + part < x.info.z) {
+            const long k = x.info.w + (long)(SPLIT * e + part) * ph.z;
             x.nbr[e] = __ldg(P.ph_nbr + k);
             x.m[e] = __ldg((const double2 *)(P.ph_m + 4 * k + 2 * (lane & 1)));
         }
@@ -177,8 +182,8 @@ __device__ __forceinline__ bool ph_over(double d, double v, double tol, float to
     return over;
 }
 
-template <bool SMEM, bool AHEAD>
-__global__ void __launch_bounds__(32 * PH_WARPS, AHEAD ? 1 : 2) k_gradients_ph(hgb_scatter_plan P, int nz,
+template <bool SMEM, bool AHEAD, int SPLIT>
+__global__ void __launch_bounds__(32 * ph_warps(AHEAD, SPLIT), AHEAD ? 1 : 2) k_gradients_ph(hgb_scatter_plan P, int nz,
                                                                   const double *__restrict__ cvec,
                                                                   double *__restrict__ hist, double *grads,
                                                                   int *d_status) {
@@ -199,31 +204,32 @@ __global__ void __launch_bounds__(32 * PH_WARPS, AHEAD ? 1 : 2) k_gradients_ph(h
     if (t < PH_RING) s_over[t] = 0;
     __syncthreads();
     // prefetch: a warp's points two phases ahead (one without AHEAD), their entries one phase ahead
-    const int base0 = 16 * warp;
-    PhPre nxt;
-    nxt.info = ph_point(P, ptr[0], base0, lane);
-    if (AHEAD) ph_entries(P, ptr[0], base0, lane, cz, nxt);
+    constexpr int PPW = 16 / SPLIT;   // points per warp
+    const int base0 = PPW * warp, part = (lane >> 1) & (SPLIT - 1);
+    PhPre<SPLIT> nxt;
+    nxt.info = ph_point<SPLIT>(P, ptr[0], base0, lane);
+    if (AHEAD) ph_entries<SPLIT>(P, ptr[0], base0, lane, cz, nxt);
     int f1 = nph > 1 ? 1 : 0;   // the next phase
-    int4 info1 = ph_point(P, ptr[f1], base0, lane);
+    int4 info1 = ph_point<SPLIT>(P, ptr[f1], base0, lane);
     bool converged = false;
     int k_end = -1;
     for (int T = 0; k_end < 0; T++) {
         if (t == 0) s_over[(T + 1) & (PH_RING - 1)] = 0;   // sweep T + 1 starts after this pass
         for (int phase = 0; phase < nph; phase++) {
             const int4 now = ptr[phase];
-            if (!AHEAD) ph_entries(P, now, base0, lane, cz, nxt);
-            const PhPre cur = nxt;
+            if (!AHEAD) ph_entries<SPLIT>(P, now, base0, lane, cz, nxt);
+            const PhPre<SPLIT> cur = nxt;
             nxt.info = info1;
-            if (AHEAD) ph_entries(P, ptr[f1], base0, lane, cz, nxt);
+            if (AHEAD) ph_entries<SPLIT>(P, ptr[f1], base0, lane, cz, nxt);
             f1 = f1 + 1 < nph ? f1 + 1 : 0;
-            info1 = ph_point(P, ptr[f1], base0, lane);
-            for (int base = base0; base < now.z; base += 16 * nw) {
-                PhPre x;
+            info1 = ph_point<SPLIT>(P, ptr[f1], base0, lane);
+            for (int base = base0; base < now.z; base += PPW * nw) {
+                PhPre<SPLIT> x;
                 if (base == base0) {
                     x = cur;
                 } else {
-                    x.info = ph_point(P, now, base, lane);
-                    ph_entries(P, now, base, lane, cz, x);
+                    x.info = ph_point<SPLIT>(P, now, base, lane);
+                    ph_entries<SPLIT>(P, now, base, lane, cz, x);
                 }
                 const int k = T - x.info.y;
                 const bool live = x.info.z >= 0 && k >= 0 && k < P.grad_maxiter;
@@ -231,14 +237,17 @@ __global__ void __launch_bounds__(32 * PH_WARPS, AHEAD ? 1 : 2) k_gradients_ph(h
                 if (live) {
                     v = x.c;
 #pragma unroll
-                    for (int e = 0; e < PH_DEG; e++) {
-                        if (e < x.info.z) {
+                    for (int e = 0; e < PH_DEG / SPLIT; e++) {
+                        if (SPLIT * e + part < x.info.z) {
                             const double2 gj = ((const double2 *)g)[x.nbr[e]];
                             v = __fma_rn(x.m[e].x, gj.x, v);
                             v = __fma_rn(x.m[e].y, gj.y, v);
                         }
                     }
-                    const int o = 2 * (now.x + base + (lane >> 1)) + (lane & 1);
+                }
+                if (SPLIT == 2) v += __shfl_xor_sync(0xffffffffu, v, 2);
+                if (live && part == 0) {
+                    const int o = 2 * (now.x + base + lane / (2 * SPLIT)) + (lane & 1);
                     d = v - g[o];
                     g[o] = v;
                     hist[2L * n * ((long)z * nring + k % nring) + o] = v;
@@ -570,16 +579,23 @@ int hgb_add_scatter_to_masses(const hgb_scatter_plan *plan, double *dens, int n_
         k_scatter_rhs<<<dim3((unsigned)hgb::ceil_div((long)n, 8), (unsigned)hgb::ceil_div(n_redz, 32)), dim3(32, 8), 0,
                         st>>>(P, dens, n_redz, vals, (double2 *)cvec);
         if ((rc = hgb::check_launch())) return rc;
-        // a warp per 16 points of the widest phase and one for a fan point, whole sub-partitions
-        int nw = (int)hgb::ceil_div(P.phase_width, 16) + 1;
-        nw = std::min(PH_WARPS, (nw + 3) / 4 * 4);
         const bool in_smem = gradients_smem(P, true) + 1024 <= (size_t)smem_optin;
         const size_t smem = gradients_smem(P, in_smem);
         // more slices than multiprocessors, outside shared memory: two blocks side by side hide each
         // other's loads, and no second wave remains
-        const auto fn = in_smem                        ? k_gradients_ph<true, true>
-                        : n_redz <= hgb::sm_count() ? k_gradients_ph<false, true>
-                                                       : k_gradients_ph<false, false>;
+        const bool ahead = in_smem || n_redz <= hgb::sm_count();
+        // Four lanes a point instead of two halve the chain of a phase and add some work: the faster form
+        // while a phase leaves FP64 units idle (us with two and with four lanes: 30x30 points, 30 to a
+        // phase, 538 and 445; 50x45 878 and 822; 61x57 1111 and 1124; 91x81 1899 and 2032) and outside
+        // shared memory, where loads make the chain (181x161 points, 152 slices: 9.3 and 8.6 ms), unless
+        // two blocks fill the FP64 units, which the walk beside them needs (201 slices: 13.0 and 12.8,
+        // but the whole call is 0.4% longer)
+        const int split = (in_smem ? P.phase_width <= 56 : ahead) ? 2 : 1;
+        // the widest phase's points and a warp for a fan point, whole sub-partitions
+        int nw = (int)hgb::ceil_div(P.phase_width, 16 / split) + 1;
+        nw = std::min(ph_warps(ahead, split), (nw + 3) / 4 * 4);
+        const auto fn = !in_smem ? (ahead ? k_gradients_ph<false, true, 2> : k_gradients_ph<false, false, 1>)
+                        : split == 1 ? k_gradients_ph<true, true, 1> : k_gradients_ph<true, true, 2>;
         if ((rc = hgb::ensure_dyn_smem((const void *)fn, smem))) return rc;
         fn<<<n_redz, 32 * nw, smem, st>>>(P, n_redz, cvec, hist, grads, d_status);
     } else {
