@@ -995,27 +995,68 @@ __device__ __forceinline__ float quantile(const float2 *cell, unsigned u) {
 
 // SORTED: lam / h are the gathered (F, B) arrays and qpos gives each realization's first bulk
 // position; otherwise lam / h are the (B, F) grids and every bin belongs to the bulk.
-// Parameter path: the seven weighted background sums per realization, FP32 Kahan in dynamic
-// shared memory [k][slot][thread], each term n * h2fdf * 2^100 * p_k * 2^-e_k (e_k the frexp exponent
-// of max |p_k|, so every scaled parameter is at most 1).
+// Parameter path: the seven weighted background sums per realization, FP32 Kahan, each term
+// n * h2fdf * 2^100 * p_k * 2^-e_k (e_k the frexp exponent of max |p_k|, so every scaled parameter is at
+// most 1).  The bins' weights lie in dynamic shared memory, [k][bin]; the sums are registers for one or
+// two realizations a thread, and lie behind the weights, [k][slot][thread], for more (fourteen words a
+// slot).  In shared memory a draw's sums are 28 accesses: 41x31x37 edges, 20
+// frequencies, 100 realizations 897 us before, 830 us now.
 constexpr int NPAR = 7;
 template <int NS>
-constexpr size_t PAR_SMEM = sizeof(float) * (NPAR * RB + 2 * NPAR * NS * RB);
+constexpr bool PAR_REGS = NS <= 2;
+template <int NS>
+constexpr size_t PAR_SMEM = sizeof(float) * (NPAR * RB + (PAR_REGS<NS> ? 0 : 2 * NPAR * NS * RB));
 
 template <int NS>
-__device__ __forceinline__ void add_par(float *psm, int sl, int t, int j, float n) {
-    const float *pw = psm;
-    float *pacc = psm + NPAR * RB;
-    float *pcomp = pacc + NPAR * NS * RB;
+struct ParSums {
+    float acc[NPAR][NS], comp[NPAR][NS];   // PAR_REGS only
+    float *psm;
+
+    __device__ __forceinline__ void zero(int t) {
+        if (PAR_REGS<NS>) {
 #pragma unroll
-    for (int k = 0; k < NPAR; k++) {
-        const int o = (k * NS + sl) * RB + t;
-        float acc = pacc[o], comp = pcomp[o];
-        kahan_add(acc, comp, n, pw[k * RB + j]);
-        pacc[o] = acc;
-        pcomp[o] = comp;
+            for (int k = 0; k < NPAR; k++)
+#pragma unroll
+                for (int i = 0; i < NS; i++) acc[k][i] = comp[k][i] = 0.0f;
+        } else {
+            for (int o = t; o < 2 * NPAR * NS * RB; o += RB) psm[NPAR * RB + o] = 0.0f;
+        }
     }
-}
+    __device__ __forceinline__ void add(int sl, int t, int j, float n) {
+        if (PAR_REGS<NS>) {
+#pragma unroll
+            for (int i = 0; i < NS; i++)
+                if (NS == 1 || i == sl) {
+#pragma unroll
+                    for (int k = 0; k < NPAR; k++) kahan_add(acc[k][i], comp[k][i], n, psm[k * RB + j]);
+                }
+        } else {
+            float *pacc = psm + NPAR * RB, *pcomp = pacc + NPAR * NS * RB;
+#pragma unroll
+            for (int k = 0; k < NPAR; k++) {
+                const int o = (k * NS + sl) * RB + t;
+                float a = pacc[o], c = pcomp[o];
+                kahan_add(a, c, n, psm[k * RB + j]);
+                pacc[o] = a;
+                pcomp[o] = c;
+            }
+        }
+    }
+    __device__ __forceinline__ double value(int k, int i, int t) const {
+        if (PAR_REGS<NS>) {
+            double v = 0.0;
+#pragma unroll
+            for (int kk = 0; kk < NPAR; kk++)
+#pragma unroll
+                for (int ii = 0; ii < NS; ii++)
+                    if (kk == k && ii == i) v = (double)acc[kk][ii] - (double)comp[kk][ii];
+            return v;
+        }
+        const float *pacc = psm + NPAR * RB, *pcomp = pacc + NPAR * NS * RB;
+        const int o = (k * NS + i) * RB + t;
+        return (double)pacc[o] - (double)pcomp[o];
+    }
+};
 
 // Shared state of one k_bulk block (static shared memory of the kernels that run bulk_block).
 template <bool PARAMS, int NS>
@@ -1058,9 +1099,9 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
             qmax = max(qmax, q);
         }
     }
-    if (PARAMS) {
-        for (int o = t; o < 2 * NPAR * NS * RB; o += RB) psm[NPAR * RB + o] = 0.0f;
-    }
+    ParSums<NS> par;
+    par.psm = psm;
+    if (PARAMS) par.zero(t);
     if (t < 16) s.lgam[t] = c_lgam[t];
     quantile_cells(s.quant);
     if (t == 0) {
@@ -1154,7 +1195,7 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
                     const int n = ((u & 0x07FFFFFFu) < (wd >> 5)) ? (int)(u >> 27) : (int)(wd & 31u);
                     if (n != 0 && (!check || pos >= __ldg(q_row + sl * RB))) {
                         kahan_add(acc_r[sl], comp_r[sl], (float)n, hs);
-                        if (PARAMS) add_par<NS>(psm, sl, t, j, (float)n);
+                        if (PARAMS) par.add(sl, t, j, (float)n);
                     }
                 }
             }
@@ -1234,7 +1275,7 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
                             const float n = (float)(k_lo + e[g]);
                             if (on && !crowded) kahan_add(acc_r[sl], comp_r[sl], n, hs);
                             if (on && crowded) add_bg(st, sl, t, n, hs);
-                            if (PARAMS && on) add_par<NS>(psm, sl, t, j, n);
+                            if (PARAMS && on) par.add(sl, t, j, n);
                         }
                     }
                 }
@@ -1269,7 +1310,7 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
                 if (k >= 0) {
                     if (!check || pos >= __ldg(q_row + sl * RB)) {
                         add_bg(st, sl, t, (float)k, hs);
-                        if (PARAMS) add_par<NS>(psm, sl, t, j, (float)k);
+                        if (PARAMS) par.add(sl, t, j, (float)k);
                     }
                     sl++;
                 } else if (it >= MAX_PTRS_ITERS) {
@@ -1278,7 +1319,7 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
                     for (; sl < rpt; sl++)
                         if (!check || pos >= __ldg(q_row + sl * RB)) {
                             add_bg(st, sl, t, kfix, hs);
-                            if (PARAMS) add_par<NS>(psm, sl, t, j, kfix);
+                            if (PARAMS) par.add(sl, t, j, kfix);
                         }
                 }
             }
@@ -1312,7 +1353,7 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
                     const int n = truncated_count_f32(lf, u24(w.z), d_status);
                     if (!check || pos >= __ldg(q_row + i * RB)) {
                         add_bg(st, i, t, (float)n, hs);
-                        add_par<NS>(psm, i, t, j, (float)n);
+                        par.add(i, t, j, (float)n);
                     }
                     i++;
                     if (i >= rpt) break;
@@ -1417,7 +1458,7 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
                 const double num = (lam > NORMAL_THRESH) ? normal_draw(ctr, a.key, lam) : ptrs64(ctr, a.key, lam, d_status);
                 if (!check || pos >= __ldg(q_row + sl * RB)) {
                     add_bg(st, sl, t, (float)(num * (double)hs), 1.0f);
-                    if (PARAMS) add_par<NS>(psm, sl, t, j, (float)num);
+                    if (PARAMS) par.add(sl, t, j, (float)num);
                 }
             }
         }
@@ -1429,20 +1470,19 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
             part[((long)c * a.nf + f) * a.nr + r0 + (long)i * RB] =
                 (((double)acc_r[i] - (double)comp_r[i]) + slot_value(st, i, t)) * HSCALE_INV;
     if (PARAMS) {
-        const float *pacc = psm + NPAR * RB;
-        const float *pcomp = pacc + NPAR * NS * RB;
+#pragma unroll
         for (int k = 0; k < NPAR; k++)
-            for (int i = 0; i < rpt; i++) {
-                const int o = (k * NS + i) * RB + t;
-                pa.part_par[(((long)c * NPAR + k) * a.nf + f) * a.nr + r0 + (long)i * RB] =
-                    ldexp(((double)pacc[o] - (double)pcomp[o]) * HSCALE_INV, pa.scale_log2[k]);
-            }
+#pragma unroll
+            for (int i = 0; i < NS; i++)
+                if (i < rpt)
+                    pa.part_par[(((long)c * NPAR + k) * a.nf + f) * a.nr + r0 + (long)i * RB] =
+                        ldexp(par.value(k, i, t) * HSCALE_INV, pa.scale_log2[k]);
     }
 }
 
 // grid (nchunk, nf, realization groups): block (c, f, rg) runs bulk_block for itself
 template <bool SORTED, bool PARAMS, int NS>
-__global__ void __launch_bounds__(RB, PARAMS ? (NS == 1 ? 5 : NS == 2 ? 4 : NS == 4 ? 3 : 2) : BULK_BLOCKS_PER_SM) k_bulk(BulkArgs a, ParArgs pa, const double *__restrict__ lam_in,
+__global__ void __launch_bounds__(RB, PARAMS ? (NS == 1 ? 5 : NS == 2 ? 3 : NS == 4 ? 3 : 2) : BULK_BLOCKS_PER_SM) k_bulk(BulkArgs a, ParArgs pa, const double *__restrict__ lam_in,
                                                           const double *__restrict__ h_in,
                                                           const int *__restrict__ qpos, double *__restrict__ part,
                                                           int *d_status) {
