@@ -76,6 +76,12 @@ namespace {
 constexpr int RB = 128;                  // threads per block == bins per staged tile
 constexpr int NWARP = RB / 32;
 constexpr int RPT = 8;                   // realizations per thread, at most (see with_slots)
+constexpr int BULK_HELP_BLOCKS = 6;      // blocks per SM up to which a k_bulk block has helping threads
+template <bool PARAMS, int NS>
+constexpr bool BULK_HELP = !PARAMS && NS < RPT;   // blocks may have RB more threads (see bulk_threads)
+constexpr int bulk_residency(bool params, int ns) {   // blocks per SM that registers are kept to
+    return params ? (ns == 1 ? 5 : ns == 8 ? 2 : 3) : ns == 8 ? 6 : 3;
+}
 static_assert(RPT == 8, "the table passes draw four realizations per Philox call, two calls per bin");
 constexpr int NT = 32;                   // CDF thresholds per small-lambda bin
 constexpr double SPARSE_MAX = 0.1;       // geometric skipping over realizations below this expectation
@@ -895,7 +901,7 @@ __device__ __forceinline__ int build_tables(Tile &s, int at, int n_table) {
     const int first_l = lane < K ? s.b_unit[lane] : 0x7FFFFFFF;
     // ---- 1
 #pragma unroll 1
-    for (int u = t; u < U; u += RB) {
+    for (int u = t; u < U; u += blockDim.x) {
         const int i = __popc(__ballot_sync(0xffffffffu, first_l <= u - lane)) - 1, j = s.list[KIND_TABLE][at + i], S = s.tb_S[j];
         const TableCut c = table_cut(S);
         const int lu = u - s.b_unit[i], k = lu >> c.lg, r = lu & ((1 << c.lg) - 1);
@@ -921,7 +927,7 @@ __device__ __forceinline__ int build_tables(Tile &s, int at, int n_table) {
     __syncthreads();
     // ---- 2
 #pragma unroll 1
-    for (int i = warp; i < K; i += NWARP) {
+    for (int i = warp; i < K; i += blockDim.x >> 5) {
         const int S = s.tb_S[s.list[KIND_TABLE][at + i]];
         const TableCut c = table_cut(S);
         unsigned int *cdf = s.u.arena + s.b_off[i];
@@ -957,7 +963,7 @@ __device__ __forceinline__ int build_tables(Tile &s, int at, int n_table) {
     __syncthreads();
     // ---- 3
 #pragma unroll 1
-    for (int u = t; u < U; u += RB) {
+    for (int u = t; u < U; u += blockDim.x) {
         const int i = __popc(__ballot_sync(0xffffffffu, first_l <= u - lane)) - 1, S = s.tb_S[s.list[KIND_TABLE][at + i]];
         const TableCut c = table_cut(S);
         const int lu = u - s.b_unit[i], k = lu >> c.lg, r = lu & ((1 << c.lg) - 1);
@@ -1083,7 +1089,8 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
     const int lane = t & 31, warp = t >> 5;
     const int r0 = rg * RB * NS + t;
     int rpt = 0;   // realizations of this thread: r0 + i * RB, i < rpt
-    while (rpt < NS && r0 + rpt * RB < a.nr) rpt++;
+    const bool draws = !BULK_HELP<PARAMS, NS> || t < RB;   // the threads beyond RB help to build tables and to walk sparse runs
+    while (draws && rpt < NS && r0 + rpt * RB < a.nr) rpt++;
     // register accumulators for the passes with a fixed realization slot
     float acc_r[NS], comp_r[NS];
     int qmin = 0x7FFFFFFF, qmax = 0;
@@ -1091,7 +1098,7 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
     for (int i = 0; i < NS; i++) {
         acc_r[i] = 0.0f;
         comp_r[i] = 0.0f;
-        slot_zero(st, i, t);
+        if (draws) slot_zero(st, i, t);
         int q = 0x7FFFFFFF;
         if (i < rpt) q = SORTED ? qpos[(long)f * a.nr + r0 + i * RB] : 0;
         if (i < rpt) {
@@ -1101,7 +1108,7 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
     }
     ParSums<NS> par;
     par.psm = psm;
-    if (PARAMS) par.zero(t);
+    if (PARAMS && draws) par.zero(t);
     if (t < 16) s.lgam[t] = c_lgam[t];
     quantile_cells(s.quant);
     if (t == 0) {
@@ -1154,7 +1161,7 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
         for (int k = 1; k < NKIND; k++) {
             const unsigned m = __ballot_sync(0xffffffffu, kind == k);
             if (kind == k) rank_mask = m;
-            if (lane == 0) s.wcount[warp][k] = __popc(m);
+            if (draws && lane == 0) s.wcount[warp][k] = __popc(m);
         }
         __syncthreads();
         if (kind != KIND_NONE) {
@@ -1168,7 +1175,7 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
         // ---- small lambda: per-bin 32-entry table, four realizations per Philox call
         const int n_small = kind_count(s, KIND_SMALL);
 #pragma unroll 1
-        for (int li = 0; li < n_small; li++) {
+        for (int li = 0; draws && li < n_small; li++) {
             const int j = s.list[KIND_SMALL][li];
             const int pos = s.pos[j];
             const float hs = s.hs[j];
@@ -1224,7 +1231,7 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
             for (int at = 0; at < n_table;) {
                 const int K = build_tables(s, at, n_table);   // (waits for the small-lambda pass, too)
 #pragma unroll 1
-                for (int i = 0; i < K; i++) {
+                for (int i = 0; draws && i < K; i++) {
                     const int j = s.list[KIND_TABLE][at + i];
                     const int pos = s.pos[j];
                     const float hs = s.hs[j];
@@ -1386,9 +1393,10 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
                 if (lane >= o) incl += y;
             }
             __syncthreads();   // the arena and the scan words are free
-            if (lane == 31) s.scan[warp] = ((unsigned long long)(unsigned)(e_hs + 2048) << 32) | (unsigned)incl;
+            if (draws && lane == 31) s.scan[warp] = ((unsigned long long)(unsigned)(e_hs + 2048) << 32) | (unsigned)incl;
 #pragma unroll
-            for (int i = 0; i < NS; i++) sub[i * RB + t] = 0ull;
+            for (int i = 0; i < NS; i++)
+                if (draws) sub[i * RB + t] = 0ull;
             __syncthreads();
             int before = 0, total = 0, e_max = -1000;
 #pragma unroll
@@ -1404,7 +1412,7 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
             __syncthreads();
             const int *q_blk = SORTED ? q_row - t : nullptr;   // first bulk positions of the block's realizations
 #pragma unroll 1
-            for (int k = t; k < total; k += RB) {
+            for (int k = t; k < total; k += blockDim.x) {
                 int lo = 0, hi = n_sparse - 1;   // the last list entry whose runs start at or before k
                 while (lo < hi) {
                     const int mid = (lo + hi + 1) >> 1;
@@ -1482,7 +1490,7 @@ __device__ __forceinline__ void bulk_block(const BulkArgs &a, const ParArgs &pa,
 
 // grid (nchunk, nf, realization groups): block (c, f, rg) runs bulk_block for itself
 template <bool SORTED, bool PARAMS, int NS>
-__global__ void __launch_bounds__(RB, PARAMS ? (NS == 1 ? 5 : NS == 2 ? 3 : NS == 4 ? 3 : 2) : BULK_BLOCKS_PER_SM) k_bulk(BulkArgs a, ParArgs pa, const double *__restrict__ lam_in,
+__global__ void __launch_bounds__(BULK_HELP<PARAMS, NS> ? 2 * RB : RB, bulk_residency(PARAMS, NS)) k_bulk(BulkArgs a, ParArgs pa, const double *__restrict__ lam_in,
                                                           const double *__restrict__ h_in,
                                                           const int *__restrict__ qpos, double *__restrict__ part,
                                                           int *d_status) {
@@ -1739,6 +1747,18 @@ size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 int n_rgroups(int nr) { return (int)hgb::ceil_div(nr, (long)RB * RPT); }
 
+// Threads of a k_bulk block.  On small grids the blocks of the lowest frequencies, with the longest
+// tables, run on after the others: RB more threads build tables and walk sparse runs with them.  Where
+// there are more blocks than an SM holds at once they only take their room (us without and with, 100
+// realizations: 30^3 bins with 20 frequencies, 3.5 blocks per SM, 630 and 557; 40x30x36 with 20, 5.7 per
+// SM, 673 and 623; 50x45x50 with 30, 20 per SM, 1186 and 1454).  Eight realizations a thread leave no
+// registers for them, nor do the parameter sums.
+template <int NS>
+unsigned bulk_threads(const dim3 &grid) {
+    const long blocks = (long)grid.x * grid.y * grid.z;
+    return BULK_HELP<false, NS> && blocks <= (long)hgb::sm_count() * BULK_HELP_BLOCKS ? 2 * RB : RB;
+}
+
 // Launches with the fewest realizations per thread (1, 2, 4 or RPT) that hold all of them in one block:
 // the draws are those of RPT, the slots beyond them are not there.  Fewer slots are fewer sums in
 // registers (56-64 a thread against 71, so 8 blocks fit an SM, not 7), one Philox call a bin instead of
@@ -1930,7 +1950,7 @@ int hgb_loudest_hc_from_sorted_ex(const double *number, const double *h2fdf, lon
     dim3 grid((unsigned)a.nchunk, (unsigned)n_freq, (unsigned)n_rgroups(nreals));
     if ((rc = bulk_event(0, st))) return rc;
     with_slots(nreals, [&](auto slots) {
-        k_bulk<true, false, decltype(slots)::value><<<grid, RB, 0, st>>>(a, ParArgs{}, lam_s, h_s, q, part, d_status);
+        k_bulk<true, false, decltype(slots)::value><<<grid, bulk_threads<decltype(slots)::value>(grid), 0, st>>>(a, ParArgs{}, lam_s, h_s, q, part, d_status);
     });
     if ((rc = hgb::check_launch())) return rc;
     if ((rc = bulk_event(1, st))) return rc;
@@ -2212,7 +2232,7 @@ int hgb_sam_poisson_gwb(const double *number, const double *hc2, long n_bins, in
     dim3 grid((unsigned)a.nchunk, (unsigned)n_freq, (unsigned)n_rgroups(nreals));
     with_slots(nreals, [&](auto slots) {
         k_bulk<false, false, decltype(slots)::value>
-            <<<grid, RB, 0, st>>>(a, ParArgs{}, number, hc2, nullptr, (double *)workspace, d_status);
+            <<<grid, bulk_threads<decltype(slots)::value>(grid), 0, st>>>(a, ParArgs{}, number, hc2, nullptr, (double *)workspace, d_status);
     });
     int rc = hgb::check_launch();
     if (rc) return rc;
