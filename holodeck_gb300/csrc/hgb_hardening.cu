@@ -1345,6 +1345,12 @@ int hgb_dbn_2pwl_phase(const double *fobs_orb, int n_freq, int fobs_sorted, doub
     }
     if (phase & 2) {
         size_t smem2 = sizeof(double) * ((size_t)5 * cosmo->grid_size + n_freq);
+        if (smem2 > 48 * 1024) {
+            hgb::set_cuda_error(cudaErrorInvalidValue);
+            return HGB_ERR_CUDA;
+        }
+        const int erc = hgb::ensure_dyn_smem((const void *)k_dbn_2pwl_eval, smem2);   // beside the static queues
+        if (erc) return erc;
         k_dbn_2pwl_eval<<<blocks, 256, smem2, (cudaStream_t)stream>>>(hgb::cy_const(), a, fobs_orb, hard_norm, nden,
                                                                       mtot, mrat, cosmo->grid_z, cosmo->grid_age,
                                                                       cosmo->grid_dcom, redz_final, diff_num);

@@ -50,7 +50,7 @@ int sm_count() {
 int ensure_dyn_smem(const void *func, size_t bytes) {
     static std::mutex mu;
     static std::map<std::pair<const void *, int>, size_t> raised;   // (function, device) -> cap set
-    if (bytes <= 48 * 1024) return HGB_OK;   // within the default cap
+    if (bytes == 0) return HGB_OK;
     int dev = 0;
     cudaError_t err = cudaGetDevice(&dev);
     if (err != cudaSuccess) {
@@ -59,14 +59,26 @@ int ensure_dyn_smem(const void *func, size_t bytes) {
     }
     std::lock_guard<std::mutex> lock(mu);
     size_t &cap = raised[std::make_pair(func, dev)];
-    if (bytes <= cap) return HGB_OK;
-    err = cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (err != cudaSuccess) {
-        set_cuda_error(err);
-        return HGB_ERR_CUDA;
+    if (cap == 0) {
+        // once, to all that the device gives the function (its default, 48 KB, counts its static shared
+        // memory too)
+        cudaFuncAttributes fa;
+        int most = 0;
+        err = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+        if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, func);
+        if (err == cudaSuccess) {
+            most -= (int)fa.sharedSizeBytes;
+            err = cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        }
+        if (err != cudaSuccess) {
+            set_cuda_error(err);
+            return HGB_ERR_CUDA;
+        }
+        cap = (size_t)most;
     }
-    cap = bytes;
-    return HGB_OK;
+    if (bytes <= cap) return HGB_OK;
+    set_cuda_error(cudaErrorInvalidValue);   // as raising the cap beyond the device's limit
+    return HGB_ERR_CUDA;
 }
 
 CyConst cy_const() {
