@@ -120,7 +120,7 @@ class ClockSampler:
 OPS_UNIFORM = 10                 # Philox4x32-10: 10 rounds x (2 wide multiplies + 2 three-input XORs) / 4 words
 OPS_ACCUM = 5                    # count to float, times strain, Kahan add
 OPS_ALIAS = OPS_UNIFORM + 4 + OPS_ACCUM          # 0.1 <= lambda < 10: column, row word, compare, select
-OPS_TABLE = OPS_UNIFORM + 5 + OPS_ACCUM          # 10 <= lambda <= 47000: guide cell, flags, one compare
+OPS_TABLE = OPS_UNIFORM + 5 + OPS_ACCUM          # 10 <= lambda <= 47000: a lookup with one compare
 OPS_TABLE_ENTRY = 4              # per table entry and realization group: recursion, to fixed point, prefix, store
 OPS_PTRS_ATTEMPT = 2 * OPS_UNIFORM + 25          # lambda > 47000: one transformed-rejection attempt
 PTRS_ATTEMPTS = 1.15             # expected attempts per draw (Hormann 1993)
