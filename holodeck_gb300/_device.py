@@ -32,15 +32,16 @@ def device(dev=None):
 _STAGED_BYTES = 32768   # host arrays up to here are uploaded without waiting for the stream
 
 
-def as_device(arr, dev=None, dtype=None):
-    """Contiguous float64 (or `dtype`) CUDA tensor from a numpy array / tensor / scalar sequence."""
+def as_device(arr, dev=None, dtype=None, wait=False):
+    """Contiguous float64 (or `dtype`) CUDA tensor from a numpy array / tensor / scalar sequence, for the
+    current stream; `wait`: uploaded when the call returns, for tensors that other streams may read."""
     t = torch()
     dtype = t.float64 if dtype is None else dtype
     dev = device(dev)
     if isinstance(arr, t.Tensor):
         return arr.to(device=dev, dtype=dtype).contiguous()
     host = np.ascontiguousarray(arr)
-    if host.nbytes > _STAGED_BYTES:
+    if wait or host.nbytes > _STAGED_BYTES or t.cuda.is_current_stream_capturing():
         return t.as_tensor(host, dtype=dtype, device=dev)
     # A blocking upload waits for the stream's queued work, which a handful of edges needs not: a private
     # pageable copy is staged by the driver before the call returns.

@@ -99,7 +99,7 @@ class Semi_Analytic_Model:
 
     def _edges_device(self):
         if self._edges_t is None:
-            self._edges_t = [D.as_device(ee) for ee in self.edges]
+            self._edges_t = [D.as_device(ee, wait=True) for ee in self.edges]   # kept: any stream may read them
         return self._edges_t
 
     # ---- static binary density (sam.py:280-398)

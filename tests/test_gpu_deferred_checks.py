@@ -67,3 +67,32 @@ def test_uploads_hold_the_values_of_the_call(n):
     got = D.as_device(arr)
     arr[:] = -1.0
     assert torch.equal(got.cpu(), torch.arange(n, dtype=torch.float64))
+
+
+def test_kept_edges_are_there_for_other_streams(built_lib):
+    """A model's edges are read on another stream than the one whose queue was busy when they were made."""
+    import torch
+    from holodeck_gb300.sams import sam as S
+    model = S.Semi_Analytic_Model(shape=(14, 11, 9))
+    one, other = torch.cuda.Stream(), torch.cuda.Stream()
+    big = torch.zeros(1 << 27, device="cuda")
+    torch.cuda.synchronize()
+    with torch.cuda.stream(one):
+        for _ in range(20):
+            big.add_(1.0)
+        edges = model._edges_device()
+    with torch.cuda.stream(other):
+        got = [e.clone() for e in edges]
+        other.synchronize()
+    for g, want in zip(got, model.edges):
+        assert np.array_equal(g.cpu().numpy(), np.asarray(want, dtype=np.float64))
+
+
+def test_uploads_are_refused_under_capture():
+    import torch
+    from holodeck_gb300 import _device as D
+    graph = torch.cuda.CUDAGraph()
+    with pytest.raises(RuntimeError):
+        with torch.cuda.graph(graph):
+            D.as_device(np.arange(4.0))
+    torch.cuda.synchronize()
