@@ -436,12 +436,17 @@ __device__ __forceinline__ double shape_outer(double y, double p, PowPlan plan) 
 //      between the first node and the last belongs to a step.  Of the time in the bracket,
 //        t_l + (t_r - t_l) (ft - f_l) / (f_r - f_l),  f = frst / (1 + z),
 //      both frequencies' quotients and the interpolation's are one reciprocal: twenty FP64 operations.
+// That a target lies in one step needs nodes whose frequencies and times ascend, and a time to start from.
+// Where they do not (a normalisation, mass, redshift or merger time that is NaN or negative, an infinite
+// step, a start inside the ISCO),
+//   C  takes the row's steps one after another, as k_dbn_2pwl does: the same brackets, and a NaN where a
+//      time is one.  (At the end, so that the rows' walk and search keep their registers.)
 // FP64 bounds both forms, but the walk in FP64 spent some 25 operations a step on 80 steps a row,
 // comparisons among them, with lanes idle where their neighbours walk longer, and wrote its outputs
 // eight bytes to a line.  91 x 81 x 101 points, 40 targets: 3130 us before, 1002 us now (FP64 pipe 75% busy); 30^3 points
 // with 20: 443 and 147 us.
 constexpr int WK_THREADS = 256;
-constexpr unsigned WK_NONE = 0xFFFFFFFFu, WK_NAN = 0xFFFFFFFEu;
+constexpr unsigned WK_NONE = 0xFFFFFFFFu, WK_LATER = 0xFFFFFFFEu;   // no bracket; a row of C
 constexpr double WK_SCALE = 0x1.0p40;   // of the FP64 frequencies, some 1e-10 Hz: keeps the bracket's products in range
 
 struct WalkShape {
@@ -490,6 +495,64 @@ __device__ int log_nodes(double init, double dx, int S, double *first, double *s
     return k;
 }
 
+// One row's steps in turn, with the comparisons of k_dbn_2pwl in their order (NaN fails them all, so a step
+// without a time brackets every target).  tc: time of the nodes from the first, norm al + gw be: one over
+// a step's time.
+__device__ __forceinline__ void walk_stepwise(const Dbn2plArgs &a, const double *ft, const double *zg, const double *ag,
+                                           const double *sz, const double *frst, const double *al, const double *be,
+                                           const double *tc, double norm, double gw, double zk, double rage, double gmt,
+                                           double *rf, double *dn) {
+    const int S = a.num_steps, NI = a.n_interp, NF = a.n_freq;
+    for (int f = 0; f < NF; f++) {
+        rf[f] = -1.0;
+        dn[f] = 0.0;
+    }
+    const double fstop = ft[NF - 1] * (1.0 + zk) * (1.0 + 1e-12);
+    int first = 0, il = 0;
+    while (first < S && frst[first + 1] < ft[0]) first++;
+    bool have_prev = false;
+    double prev_tr = 0.0, prev_zr = 0.0, prev_fr = 0.0;
+    for (int s = first; s < S; s++) {
+        if (frst[s] > fstop) break;
+        const bool reuse = have_prev;
+        have_prev = false;
+        const double tr = tc[s + 1] + gmt + rage;
+        const double tl = reuse ? prev_tr : tr - 1.0 / __fma_rn(norm, al[s], gw * be[s]);
+        if (tl > ag[NI - 1]) continue;
+        double zl = prev_zr;
+        if (!reuse) {
+            il = hgb::while_while_increasing(il, NI, tl, ag);
+            zl = zg[il] + (tl - ag[il]) * sz[il];
+        }
+        if (zl < 0.0) continue;
+        const double fl = reuse ? prev_fr : frst[s] / (1.0 + zl);
+        const int ir = hgb::while_while_increasing(il, NI, tr, ag);
+        const double zr = zg[ir] + (tr - ag[ir]) * sz[ir];
+        const double fr = frst[s + 1] / (1.0 + (zr < 0.0 ? 0.0 : zr));
+        if (zr >= 0.0) {
+            have_prev = true;
+            prev_tr = tr;
+            prev_zr = zr;
+            prev_fr = fr;
+        }
+        const int il_step = il;
+        il = ir;
+        for (int f = 0; f < NF; f++) {
+            if (ft[f] < fl || fr < ft[f]) continue;
+            const double tt = hgb::interp_between(ft[f], fl, fr, tl, tr);
+            if (tt > ag[NI - 1]) break;
+            rf[f] = (double)il_step;
+            dn[f] = tt;
+        }
+    }
+}
+
+// a merger time before the start or none, or no age to start from
+__device__ __forceinline__ bool wk_odd_row(double gmt, double rage) {
+    const float sum = hgb::f64_to_f32_rz(gmt + rage);
+    return __double2hiint(gmt) < 0 || sum != sum;
+}
+
 __host__ __device__ inline int wk_stride(int nf) { return nf | 1; }   // an odd row length keeps the lanes' rows in different banks
 
 __global__ void __launch_bounds__(WK_THREADS, 3) k_dbn_2pwl_walk(
@@ -510,18 +573,27 @@ __global__ void __launch_bounds__(WK_THREADS, 3) k_dbn_2pwl_walk(
     float *frf = ftf + NF;
     unsigned *code = (unsigned *)(frf + S + 1);   // [rows][wk_stride(NF)] step | interval << 16
     __shared__ int s_first;
+    __shared__ unsigned s_odd;   // the block's cells (bit per cell) whose rows are C's
+    __shared__ int s_later;      // whether C has rows
     __shared__ unsigned queue[WK_THREADS / 32][64];
     const int nqb = (a.n_mrat + ws.qc - 1) / ws.qc;
     const int ii = blockIdx.x / nqb, q0 = (blockIdx.x % nqb) * ws.qc, q1 = min(q0 + ws.qc, a.n_mrat);
     const double mt = mtot[ii];
 
+    if (t == 0) {
+        s_odd = 0u;
+        s_later = 0;
+    }
     for (int i = t; i < NI; i += WK_THREADS) {
         zg[i] = zgrid_g[i];
         ag[i] = agrid_g[i];
     }
+    bool odd = false;   // a NaN among the targets, frequencies that do not ascend
     for (int f = t; f < NF; f += WK_THREADS) {
-        ft[f] = fobs[f] * WK_SCALE;
-        ftf[f] = (float)fobs[f];
+        const double x = fobs[f];
+        ft[f] = x * WK_SCALE;
+        ftf[f] = (float)x;
+        odd |= (__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFll) > 0x7FF0000000000000ll;
     }
     // nodes: separation, and in the steps' arrays for now the hardening shape and 1 / separation^3
     double *sepa = tn;   // the first cell's times come later
@@ -579,6 +651,8 @@ __global__ void __launch_bounds__(WK_THREADS, 3) k_dbn_2pwl_walk(
             const double c = 0.5 * (hgb::fast_range(w) ? hgb::fast_rcp(w) : 1.0 / w);
             av = (al[s] + al[s + 1]) * c;
             bv = (be[s] + be[s + 1]) * c;
+            const long long lo = __double_as_longlong(frst[s]), hi = __double_as_longlong(frst[s + 1]);
+            odd |= !(lo > 0 && hi > lo && hi < 0x7FF0000000000000ll);
         }
         __syncthreads();   // every node of this run is read, and node s0 + WK_THREADS is rewritten next
         if (s < S) {
@@ -586,6 +660,7 @@ __global__ void __launch_bounds__(WK_THREADS, 3) k_dbn_2pwl_walk(
             be[s] = bv;
         }
     }
+    if (odd) atomicOr(&s_odd, ~0u);
     __syncthreads();
     const int first = s_first;
     const float age_f = (float)ag[NI - 1] * 1.000001f;   // beyond it in FP32: beyond the table's end in FP64
@@ -601,9 +676,12 @@ __global__ void __launch_bounds__(WK_THREADS, 3) k_dbn_2pwl_walk(
         const double mr = mrat[q0 + c], opq = 1.0 + mr;
         const double gw_k = -cc.c_dadt * (mt * mt * mt) * mr / (opq * opq);
         const double y = __fma_rn(hard_norm[(long)ii * a.n_mrat + q0 + c], al[s], gw_k * be[s]);
-        tn[(size_t)c * (S + 1) + s + 1] = hgb::fast_range(y) ? hgb::fast_rcp(y) : 1.0 / y;
+        const bool plain = hgb::fast_range(y);   // positive and finite, as its reciprocal
+        if (!plain) atomicOr(&s_odd, 1u << c);
+        tn[(size_t)c * (S + 1) + s + 1] = plain ? hgb::fast_rcp(y) : 1.0 / y;
     }
     __syncthreads();
+    const unsigned odd_cells = s_odd;
     if (t < nq) {
         double *tc = tn + (size_t)t * (S + 1);
         double te = 0.0;
@@ -632,8 +710,9 @@ __global__ void __launch_bounds__(WK_THREADS, 3) k_dbn_2pwl_walk(
                 unsigned *cd = code + t * stride;
                 int f = 0;
                 unsigned rest = WK_NONE;
-                if (b != b) {
-                    rest = WK_NAN;   // every step brackets every target, with no time
+                if (((odd_cells >> (qb - q0 + c)) & 1u) || wk_odd_row(b, rage[kk])) {
+                    rest = WK_LATER;
+                    s_later = 1;
                 } else {
                     float tl = bf + hgb::f64_to_f32_rz(tc[first]);
                     int il = 0, hi = NI - 2;   // interval of the first node
@@ -710,11 +789,11 @@ __global__ void __launch_bounds__(WK_THREADS, 3) k_dbn_2pwl_walk(
             unsigned *q = queue[warp];
             for (int i0 = 32 * warp; i0 < nr * NF; i0 += WK_THREADS) {
                 const unsigned cd = r < nr ? code[r * stride + f] : WK_NONE;
-                const bool live = cd < WK_NAN;
-                if (r < nr && !live) {
+                const bool live = cd < WK_LATER;
+                if (r < nr && cd == WK_NONE) {
                     const long e = (long)r * NF + f;
-                    rf[e] = cd == WK_NAN ? 0.0 : -1.0;
-                    dn[e] = cd == WK_NAN ? base[r] : 0.0;
+                    rf[e] = -1.0;
+                    dn[e] = 0.0;
                 }
                 const unsigned m = __ballot_sync(0xffffffffu, live);
                 if (live) q[held + __popc(m & ((1u << lane) - 1u))] = (unsigned)r << 16 | (unsigned)f;
@@ -738,6 +817,18 @@ __global__ void __launch_bounds__(WK_THREADS, 3) k_dbn_2pwl_walk(
             if (lane < held) element(q[lane]);
             __syncwarp();
         }
+    }
+    __syncthreads();
+    if (!s_later) return;
+    // ---- C
+    for (int i = t; i < nq * NZ; i += WK_THREADS) {
+        const int c = i / NZ, kk = i % NZ;
+        const long cell = (long)ii * a.n_mrat + q0 + c;
+        const double b = gmt_time[cell * NZ + kk], mr = mrat[q0 + c], opq = 1.0 + mr;
+        if (((odd_cells >> c) & 1u) || wk_odd_row(b, rage[kk]))
+            walk_stepwise(a, ft, zg, ag, sz, frst, al, be, tn + (size_t)c * (S + 1), hard_norm[cell],
+                          -cc.c_dadt * (mt * mt * mt) * mr / (opq * opq), redz[kk], rage[kk], b,
+                          redz_final + (cell * NZ + kk) * NF, diff_num + (cell * NZ + kk) * NF);
     }
 }
 
