@@ -21,6 +21,9 @@ namespace hgb {
 
 void set_cuda_error(cudaError_t err);
 int check_launch();
+// Host values to dst (whole 32-bit words) in stream order, in the arguments of one launch per 32,000 bytes;
+// the host memory may go when the call returns.
+int upload_words(void *dst, const void *host, size_t bytes, cudaStream_t st);
 
 // Loudest-first argsort at the first frequency (hgb_sort.cu): scratch bytes for n_bins, and the sort
 // itself with the caller's scratch (at least argsort_f0_scratch_bytes(n_bins), 256-byte aligned).

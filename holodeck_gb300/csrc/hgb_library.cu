@@ -1,7 +1,9 @@
 // Library-level entry points: version, error strings, shared host helpers.
 #include <math.h>
 #include <stdio.h>
+#include <string.h>
 
+#include <algorithm>
 #include <atomic>
 #include <map>
 #include <mutex>
@@ -16,9 +18,43 @@ __global__ void k_sqrt(double *x, long n) {
     if (i < n) x[i] = sqrt(x[i]);
 }
 
+// Host words in a kernel's arguments, which the launch (or the capture of it) copies: their source may go
+// when the call returns.  cudaMemcpyAsync promises that of pageable memory only where it stages the copy, and
+// a device that addresses host memory need not.
+template <int WORDS>
+struct HostWords {
+    uint32_t w[WORDS];
+};
+template <int WORDS>
+__global__ void k_put_words(const __grid_constant__ HostWords<WORDS> h, uint32_t *dst, int n) {
+    const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (i < n) dst[i] = h.w[i];
+}
+
+template <int WORDS>
+void put_words(uint32_t *dst, const char *host, int n, cudaStream_t st) {
+    HostWords<WORDS> h;
+    memcpy(h.w, host, sizeof(uint32_t) * n);
+    k_put_words<WORDS><<<(unsigned)hgb::ceil_div(n, 128), 128, 0, st>>>(h, dst, n);
+}
+
 }  // namespace
 
 namespace hgb {
+
+int upload_words(void *dst, const void *host, size_t bytes, cudaStream_t st) {
+    constexpr int MOST = 8000;   // words of one launch: its arguments stay below 32,764 bytes
+    for (size_t at = 0; at < bytes; at += sizeof(uint32_t) * MOST) {
+        const int n = (int)(std::min(bytes - at, sizeof(uint32_t) * MOST) / sizeof(uint32_t));
+        uint32_t *d = (uint32_t *)((char *)dst + at);
+        const char *h = (const char *)host + at;
+        if (n <= 250) put_words<250>(d, h, n, st);
+        else put_words<MOST>(d, h, n, st);
+        const int rc = check_launch();
+        if (rc) return rc;
+    }
+    return HGB_OK;
+}
 
 static thread_local char g_last_cuda_error[256] = "";
 
@@ -109,6 +145,11 @@ const char *hgb_error_string(int code) {
 }
 
 const char *hgb_last_cuda_error(void) { return hgb::g_last_cuda_error; }
+
+int hgb_upload(void *dst, const void *host, size_t bytes, void *stream) {
+    if ((bytes && (!dst || !host)) || (bytes & 3) || ((uintptr_t)dst & 3)) return HGB_ERR_INVALID_ARGUMENT;
+    return hgb::upload_words(dst, host, bytes, (cudaStream_t)stream);
+}
 
 int hgb_sqrt_inplace(double *x, long n, void *stream) {
     if (!x || n < 0) return HGB_ERR_INVALID_ARGUMENT;

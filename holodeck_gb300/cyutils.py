@@ -219,7 +219,7 @@ def loudest_par_device(number, h2fdf, nreals, nloudest, order, mt, mr, rz, grids
         rep = D.as_device(replay)
         if tuple(rep.shape) != (nreals, nf, nb):
             raise ValueError(f"replay must be shaped (R, F, B)=({nreals}, {nf}, {nb}), got {tuple(rep.shape)}")
-    mt_d, mr_d, rz_d = (D.as_device(np.ascontiguousarray(x, dtype=np.float64), dev) for x in (mt, mr, rz))
+    mt_d, mr_d, rz_d = D.as_devices(*[np.ascontiguousarray(x, dtype=np.float64) for x in (mt, mr, rz)], dev=dev)
     scales = t.cat([t.tensor([_frexp_exponent(x) for x in (mt, mr, rz)], dtype=t.int32, device=dev),
                     grid_scales.to(t.int32)])
     lib = N.load()

@@ -18,7 +18,7 @@ def char_strain_sq_device(edges, redz, cosmo=None, status=None):
     t = D.torch()
     cosmo = _cosmo if cosmo is None else cosmo
     dc = D.device_cosmology(cosmo)
-    mt, mr, fe = D.as_device(edges[0]), D.as_device(edges[1]), D.as_device(edges[3])
+    mt, mr, fe = D.as_devices(edges[0], edges[1], edges[3])
     nm, nq, nz, nf = int(mt.numel()), int(mr.numel()), int(redz.shape[2]), int(fe.numel()) - 1
     out = t.empty((nm - 1, nq - 1, nz - 1, nf), dtype=t.float64, device=redz.device)
     st = status if status is not None else D.StatusWord(redz.device)

@@ -305,9 +305,7 @@ class Semi_Analytic_Model:
         is left to the caller (no host read here).  ``precision="fp32"``: hgb_number_and_strain_f32."""
         t = D.torch()
         mt, mr, rz = self._edges_device()
-        lm = D.as_device(np.log10(self.mtot))
-        fe = D.as_device(fobs_orb_edges)
-        dlnf = D.as_device(np.diff(np.log(fobs_orb_edges)))
+        lm, fe, dlnf = D.as_devices(np.log10(self.mtot), fobs_orb_edges, np.diff(np.log(fobs_orb_edges)))
         dc = D.device_cosmology(self._cosmo, mt.device)
         nm, nq, nz = self.shape
         nf = int(dlnf.numel())

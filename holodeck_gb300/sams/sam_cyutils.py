@@ -123,7 +123,7 @@ def _axis_host(edges):
 def integrate_device(edges, dnum):
     t = D.torch()
     lm, dlnf = _axis_host(edges)
-    lm, mr, rz, dlnf = D.as_device(lm), D.as_device(edges[1]), D.as_device(edges[2]), D.as_device(dlnf)
+    lm, mr, rz, dlnf = D.as_devices(lm, edges[1], edges[2], dlnf)
     out = t.empty((lm.numel() - 1, mr.numel() - 1, rz.numel() - 1, dlnf.numel()), dtype=t.float64,
                   device=dnum.device)
     N.call("hgb_integrate_3dx1d", N.ptr(lm), int(lm.numel()), N.ptr(mr), int(mr.numel()), N.ptr(rz),

@@ -78,8 +78,8 @@ def param_grids_device(edges, redz, h2fdf=None, cosmo=None):
     t = D.torch()
     cosmo = _cosmo if cosmo is None else cosmo
     dc = D.device_cosmology(cosmo)
-    mt = D.as_device(utils.midpoints(np.asarray(D.to_host(edges[0]) if D.is_torch(edges[0]) else edges[0])))
-    fc = D.as_device(utils.midpoints(np.asarray(D.to_host(edges[3]) if D.is_torch(edges[3]) else edges[3])))
+    mt, fc = D.as_devices(*[utils.midpoints(np.asarray(D.to_host(e) if D.is_torch(e) else e))
+                            for e in (edges[0], edges[3])])
     nm, nq, nz, nf = int(np.size(edges[0])), int(np.size(edges[1])), int(redz.shape[2]), int(fc.numel())
     shape = (nm - 1, nq - 1, nz - 1, nf)
     grids = [t.empty(shape, dtype=t.float64, device=redz.device) for _ in range(4)]

@@ -215,6 +215,11 @@ int hgb_find_2pwl_hardening_norm(double target_time, const double *mtot, const d
                                  double sepa_init, double rchar, double gamma_inner, double gamma_outer,
                                  int nsteps, double *norm_log10, double *norm, int *d_status, void *stream);
 
+/* Copies `bytes` (a multiple of 4) of HOST memory to dst (device, 4-byte aligned) in stream order, in the
+ * arguments of one launch per 32,000 bytes: `host` may be freed or changed when the call returns.  For small
+ * inputs of calls that should not wait for the stream. */
+int hgb_upload(void *dst, const void *host, size_t bytes, void *stream);
+
 /* x[i] = sqrt(x[i]) (the hc^2 -> hc step of single_sources.py:166-167). */
 int hgb_sqrt_inplace(double *x, long n, void *stream);
 
