@@ -2061,11 +2061,10 @@ int hgb_loudest_hc_batch(const hgb_loudest_sample *samples, int n_samples, int n
                 for (int c = 0; c < nchunk[j]; c++) items.push_back(make_int4(j, c, f, rg));
     const int n_items = (int)items.size();
     int *d_next = (int *)(w + align256(sizeof(int4) * items.size()));
-    // pageable host sources: each copy is staged before the call returns, so the vectors may go
-    cudaError_t err = cudaMemcpyAsync(d_jobs, jobs.data(), sizeof(BulkJob) * nj, cudaMemcpyHostToDevice, st);
-    if (err == cudaSuccess)
-        err = cudaMemcpyAsync(d_items, items.data(), sizeof(int4) * items.size(), cudaMemcpyHostToDevice, st);
-    if (err == cudaSuccess) err = cudaMemsetAsync(d_flags, 0, sizeof(int) * nj, st);
+    // in launches' arguments: the vectors may go when the call returns (or while a graph that holds it lives)
+    if ((rc = hgb::upload_words(d_jobs, jobs.data(), sizeof(BulkJob) * nj, st))) return rc;
+    if ((rc = hgb::upload_words(d_items, items.data(), sizeof(int4) * items.size(), st))) return rc;
+    cudaError_t err = cudaMemsetAsync(d_flags, 0, sizeof(int) * nj, st);
     if (err == cudaSuccess) err = cudaMemsetAsync(d_next, 0, sizeof(int), st);
     if (err != cudaSuccess) {
         hgb::set_cuda_error(err);

@@ -66,3 +66,33 @@ def test_arrays_that_travel_together():
             a = a.cpu().numpy() if a is tensor else a
             assert g.dtype == torch.float64 and g.is_contiguous() and g.data_ptr() % 16 == 0
             assert np.array_equal(g.cpu().numpy(), a)
+
+
+def test_batch_work_list_outlives_the_call(built_lib):
+    """A captured multi-sample launch replays from its own copy of the work list, whatever the host memory that
+    the call built it in holds by then (lists of one and of several uploads)."""
+    import torch
+    from holodeck_gb300 import _device as D, cyutils, single_sources
+    rng = np.random.default_rng(3)
+    for nf, sizes in ((2, ((300, 5),)), (40, ((9000, 60), (7000, 1100)))):
+        samples = []
+        for nb, nr in sizes:
+            num, hh = (torch.as_tensor(10.0 ** rng.uniform(lo, hi, size=(nb, nf)), device="cuda")
+                       for lo, hi in ((-4.0, 6.0), (-32.0, -26.0)))
+            samples.append(dict(number=num, h2fdf=hh, order=single_sources.sort_order_device(hh), nreals=nr, seed=nb,
+                                status=D.StatusWord()))
+        want = cyutils.loudest_batch_device(samples, 3)
+        graph = torch.cuda.CUDAGraph()
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph):
+            got = cyutils.loudest_batch_device(samples, 3)
+        fill = [np.full(1 << k, 0xFFFFFFFF, dtype=np.uint32) for k in range(4, 18) for _ in range(8)]
+        for _ in range(2):
+            for ss, bg in got:
+                ss.fill_(-1.0)
+                bg.fill_(-1.0)
+            graph.replay()
+            torch.cuda.synchronize()
+            for (ss, bg), (want_ss, want_bg) in zip(got, want):
+                assert torch.equal(ss, want_ss) and torch.equal(bg, want_bg)
+        del fill
