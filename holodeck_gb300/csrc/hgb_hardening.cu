@@ -1474,6 +1474,8 @@ int hgb_dbn_2pwl_phase_f32(const double *fobs_orb, int n_freq, int fobs_sorted, 
     unsigned blocks = (unsigned)((long)n_mtot * n_mrat);
     size_t smem = sizeof(double) * (size_t)5 * cosmo->grid_size + sizeof(float) * (size_t)n_freq;
     HGB_CHECK_ARG(smem <= 48 * 1024);
+    const int erc = hgb::ensure_dyn_smem((const void *)k_dbn_2pwl_eval_f32, smem);   // beside the static words
+    if (erc) return erc;
     k_dbn_2pwl_eval_f32<<<blocks, 256, smem, (cudaStream_t)stream>>>(hgb::cy_const(), a, fobs_orb, hard_norm, nden,
                                                                      mtot, mrat, cosmo->grid_z, cosmo->grid_age,
                                                                      cosmo->grid_dcom, redz_final, diff_num);
