@@ -10,7 +10,7 @@
 //    age -> redshift / distance interpolations use per-interval slopes computed once per block
 //    (a multiply instead of a divide per lookup; results differ from the reference's divide by an ulp).
 //  * hgb_dbn_gw: differential binary number for Hard_GW (sam_cyutils.pyx:788-899); one block per
-//    (mtot, mrat) cell.
+//    run of up to 256 (mtot, mrat, redz) points.
 // FP64 throughout (the hardening integral and the lookback-time -> redshift inversion are the
 // FP64 islands of the path).  Built with -fmad=false so operation order and rounding follow the
 // reference loops; the remaining differences are the last-ulp behaviour of pow/log10.
@@ -1057,41 +1057,63 @@ __global__ void k_dbn_2pwl_eval_f32(CyConst cc, Dbn2plArgs a, const double *__re
 // differential binary number, Hard_GW
 // ------------------------------------------------------------------------------------------------
 
-// One block per (mtot, mrat) cell.  For GW-driven hardening the residence time is a product of powers,
+// One block per run of grid points, rows of the outputs, across cells.  For GW-driven hardening the residence time is a product of powers,
 //   tres = (2/3) sepa / |da/dt| = (2/3) ksepa^4 mt^(4/3) (1 + mr)^2 / (|c_dadt| mt^3 mr) (f (1 + z))^(-8/3),
 // so an element is A(cell, z) B(f) with B = f^(-8/3) taken once per block and A once per grid point:
 // one FP64 product per element in place of two pow() and six divisions (on this GPU an FP64 warp
 // instruction holds its pipe for 64 cycles, so those set the time).  Targets are the block's fastest
 // index, so the two (M, Q, Z, F) outputs are written in contiguous runs; with one thread per grid
-// point walking its targets every store of a warp touched 32 lines.  61 x 47 x 53 points, 37 targets:
-// 5059 us with one thread per point, 121 us so (FP64 of the per-point terms).
+// point walking its targets every store of a warp touched 32 lines.  A block takes up to 256 rows, so that
+// the powers of the targets and of its cells' masses are shared by many points and the per-point terms
+// fill its threads, whatever the grid's shape; fewer where that would leave multiprocessors without four
+// blocks.  us with one thread per point, one block per cell, and so (each with the call's launch
+// and allocation): 61 x 47 x 53 points, 37 targets 5059, 121, 52; 181 x 161 x 1, one target 103, 705, 70.
 // The reference stops at the first target above the ISCO frequency, so target f is empty when any
 // f' <= f lies above it: the running maximum of the targets decides (products by 1 + z > 0 keep the
 // order).  B and the cell's constant carry 2^-80 and 2^80, which keeps A within a few decades of the
 // result.  f^(2/3) and mt^(1/3) are pow() of the rounded exponents, as in the reference: a cube root is
 // nearer to the real power but 4e-15 from the reference's value once it is raised to the fourth.
-constexpr int GW_ROWS = 256;    // redshifts staged at a time, one per thread
+constexpr int GW_ROWS = 256;    // rows of a block at most, one per thread
 constexpr int GW_FREQS = 512;   // targets staged at a time
 constexpr double GW_SCALE = 0x1.0p80, GW_SCALE_INV = 0x1.0p-80;
 
 __global__ void __launch_bounds__(GW_ROWS) k_dbn_gw(CyConst cc, const double *__restrict__ fobs, int NF,
                                                     const double *__restrict__ nden, const double *__restrict__ mtot,
-                                                    const double *__restrict__ mrat, int nq, int nz,
-                                                    const double *__restrict__ redz_prime,
+                                                    const double *__restrict__ mrat, int nq, int nz, long total,
+                                                    int rows, const double *__restrict__ redz_prime,
                                                     const double *__restrict__ zgrid, const double *__restrict__ dgrid,
                                                     int NI, double *__restrict__ redz_final,
                                                     double *__restrict__ diff_num) {
     __shared__ double fb[GW_FREQS], ftop[GW_FREQS];   // B and the running maximum of the targets
     __shared__ double s_amp[GW_ROWS], s_z[GW_ROWS];
     __shared__ int s_cut[GW_ROWS];                    // first empty target of the staged ones
-    __shared__ double s_k, s_isco;
-    const int t = threadIdx.x, cell = blockIdx.x;
-    if (t == 32) {
-        const double mt = mtot[cell / nq], mr = mrat[cell % nq];
+    __shared__ double s_k[GW_ROWS], s_isco[GW_ROWS];  // of the block's cells
+    const int t = threadIdx.x;
+    const long row0 = (long)blockIdx.x * rows;
+    const int nrb = (int)(total - row0 < rows ? total - row0 : rows);
+    const long cell0 = row0 / nz;
+    const int z0 = (int)(row0 - cell0 * nz);
+    if (t < (z0 + nrb - 1) / nz + 1) {
+        const double mt = mtot[(cell0 + t) / nq], mr = mrat[(cell0 + t) % nq];
         const double ks2 = cc.ksepa * cc.ksepa, opq = 1.0 + mr;
         const double m13 = pow(mt, 1.0 / 3.0), m23 = m13 * m13;
-        s_k = (2.0 / 3.0) * (ks2 * ks2) * (opq * opq) / (-cc.c_dadt * mr) * (m23 * m23 / mt / mt / mt) * GW_SCALE;
-        s_isco = cc.kfreq * sqrt(mt) / pow(3.0 * HGB_CY_SCHW * mt, 1.5);
+        s_k[t] = (2.0 / 3.0) * (ks2 * ks2) * (opq * opq) / (-cc.c_dadt * mr) * (m23 * m23 / mt / mt / mt) * GW_SCALE;
+        s_isco[t] = cc.kfreq * sqrt(mt) / pow(3.0 * HGB_CY_SCHW * mt, 1.5);
+    }
+    // the row's redshift terms: A without the cell's constant
+    double rzp = -1.0, zp1 = 0.0, part = 0.0, z_third = 0.0;
+    const int cell = (z0 + t) / nz;
+    if (t < nrb) {
+        rzp = redz_prime[row0 + t];
+        if (!(rzp <= 0.0)) {
+            int zi = hgb::bracket_decreasing_from0(NI, rzp, zgrid);
+            if (zi > NI - 2) zi = NI - 2;
+            const double dcom = hgb::interp_between(rzp, zgrid[zi], zgrid[zi + 1], dgrid[zi], dgrid[zi + 1]);
+            const double dcm = dcom / HGB_CY_MPC;
+            zp1 = 1.0 + rzp;
+            part = nden[row0 + t] * (cc.fourpi * zp1 * (dcm * dcm));
+            z_third = cbrt(zp1);
+        }
     }
     double top = -INFINITY;   // (thread 0) largest target so far
     for (int f0 = 0; f0 < NF; f0 += GW_FREQS) {
@@ -1109,49 +1131,38 @@ __global__ void __launch_bounds__(GW_ROWS) k_dbn_gw(CyConst cc, const double *__
             }
         }
         __syncthreads();
-        const double kc = s_k, isco = s_isco;
-        for (int z0 = 0; z0 < nz; z0 += GW_ROWS) {
-            const int nzb = min(GW_ROWS, nz - z0);
-            const long row0 = (long)cell * nz + z0;
-            if (z0 > 0) __syncthreads();   // the previous rows are written
-            if (t < nzb) {
-                const double rzp = redz_prime[row0 + t];
-                double amp = 0.0;
-                int cut = 0;
-                if (!(rzp <= 0.0)) {
-                    int zi = hgb::bracket_decreasing_from0(NI, rzp, zgrid);
-                    if (zi > NI - 2) zi = NI - 2;
-                    const double dcom = hgb::interp_between(rzp, zgrid[zi], zgrid[zi + 1], dgrid[zi], dgrid[zi + 1]);
-                    const double dcm = dcom / HGB_CY_MPC, zp1 = 1.0 + rzp;
-                    const double cosmo_fact = cc.fourpi * zp1 * (dcm * dcm);
-                    // (1 + z)^(-8/3) = cbrt(1 + z) / (1 + z)^3
-                    amp = nden[row0 + t] * cosmo_fact * (kc * cbrt(zp1) / (zp1 * zp1 * zp1));
-                    int hi = nfb;   // first f with ftop[f] (1 + z) > isco
-                    while (cut < hi) {
-                        const int mid = (cut + hi) >> 1;
-                        if (ftop[mid] * zp1 > isco) hi = mid;
-                        else cut = mid + 1;
-                    }
+        if (t < nrb) {
+            double amp = 0.0;
+            int cut = 0;
+            if (!(rzp <= 0.0)) {
+                // (1 + z)^(-8/3) = cbrt(1 + z) / (1 + z)^3
+                amp = part * (s_k[cell] * z_third / (zp1 * zp1 * zp1));
+                const double isco = s_isco[cell];
+                int hi = nfb;   // first f with ftop[f] (1 + z) > isco
+                while (cut < hi) {
+                    const int mid = (cut + hi) >> 1;
+                    if (ftop[mid] * zp1 > isco) hi = mid;
+                    else cut = mid + 1;
                 }
-                s_amp[t] = amp;
-                s_z[t] = rzp <= 0.0 ? -1.0 : rzp;
-                s_cut[t] = cut;
             }
-            __syncthreads();
-            double *rf = redz_final + row0 * NF + f0;
-            double *dn = diff_num + row0 * NF + f0;
-            const int dz = GW_ROWS / nfb, df = GW_ROWS - dz * nfb;
-            int z = t / nfb, f = t - z * nfb;
-            while (z < nzb) {
-                const long e = (long)z * NF + f;
-                rf[e] = s_z[z];
-                dn[e] = f < s_cut[z] ? s_amp[z] * fb[f] : 0.0;
-                z += dz;
-                f += df;
-                if (f >= nfb) {
-                    f -= nfb;
-                    z++;
-                }
+            s_amp[t] = amp;
+            s_z[t] = rzp <= 0.0 ? -1.0 : rzp;
+            s_cut[t] = cut;
+        }
+        __syncthreads();
+        double *rf = redz_final + row0 * NF + f0;
+        double *dn = diff_num + row0 * NF + f0;
+        const int dz = GW_ROWS / nfb, df = GW_ROWS - dz * nfb;
+        int z = t / nfb, f = t - z * nfb;
+        while (z < nrb) {
+            const long e = (long)z * NF + f;
+            rf[e] = s_z[z];
+            dn[e] = f < s_cut[z] ? s_amp[z] * fb[f] : 0.0;
+            z += dz;
+            f += df;
+            if (f >= nfb) {
+                f -= nfb;
+                z++;
             }
         }
     }
@@ -1498,8 +1509,11 @@ int hgb_dbn_gw(const double *fobs_orb, int n_freq, const double *nden, const dou
     HGB_CHECK_ARG(fobs_orb && nden && mtot && mrat && redz_prime && cosmo && redz_final && diff_num);
     HGB_CHECK_ARG(n_freq > 0 && n_mtot > 0 && n_mrat > 0 && n_redz > 0);
     HGB_CHECK_ARG(cosmo->grid_size >= 2 && cosmo->grid_z && cosmo->grid_dcom);
-    k_dbn_gw<<<(unsigned)((long)n_mtot * n_mrat), GW_ROWS, 0, (cudaStream_t)stream>>>(
-        hgb::cy_const(), fobs_orb, n_freq, nden, mtot, mrat, n_mrat, n_redz, redz_prime, cosmo->grid_z,
+    const long total = (long)n_mtot * n_mrat * n_redz;
+    long rows = hgb::ceil_div(total, 4L * hgb::sm_count());
+    if (rows > 32) rows = std::min((rows + 31) / 32 * 32, (long)GW_ROWS);   // whole warps of points
+    k_dbn_gw<<<(unsigned)hgb::ceil_div(total, rows), GW_ROWS, 0, (cudaStream_t)stream>>>(
+        hgb::cy_const(), fobs_orb, n_freq, nden, mtot, mrat, n_mrat, n_redz, total, (int)rows, redz_prime, cosmo->grid_z,
         cosmo->grid_dcom, cosmo->grid_size, redz_final, diff_num);
     return hgb::check_launch();
 }
