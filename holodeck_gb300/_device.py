@@ -30,6 +30,8 @@ def device(dev=None):
 
 
 _SMALL_BYTES = 32000   # host arrays up to here are uploaded without waiting for the stream (one launch)
+_SMALL_TYPES = {"torch.float64": np.dtype(np.float64), "torch.float32": np.dtype(np.float32),
+                "torch.int32": np.dtype(np.int32)}
 
 
 def as_device(arr, dev=None, dtype=None, wait=False):
@@ -41,37 +43,33 @@ def as_device(arr, dev=None, dtype=None, wait=False):
     if isinstance(arr, t.Tensor):
         return arr.to(device=dev, dtype=dtype).contiguous()
     host = np.ascontiguousarray(arr)
-    plain = host.dtype.kind in "biuf" and host.dtype.isnative and host.dtype.itemsize <= 8
-    if (wait or not plain or dtype not in (t.float64, t.float32, t.int32)
-            or host.size * dtype.itemsize > _SMALL_BYTES or dev.index not in (None, t.cuda.current_device())
-            or t.cuda.is_current_stream_capturing()):
+    small = _SMALL_TYPES.get(str(dtype))
+    if wait or small is None or t.cuda.is_current_stream_capturing():
+        return t.as_tensor(host, dtype=dtype, device=dev)
+    own = host.dtype
+    if (host.size * small.itemsize > _SMALL_BYTES or (dev.index is not None and dev.index != t.cuda.current_device())
+            or not (own is small or (own.kind in "biuf" and own.isnative and own.itemsize <= 8))):
         return t.as_tensor(host, dtype=dtype, device=dev)
     # A blocking upload waits for the stream's queued work, which a handful of edges needs not: the values
     # travel with a launch.  (A copy that does not wait may read pageable memory after it was freed.)
-    host = host.astype(str(dtype)[6:], copy=False)   # torch.float64 -> float64
+    host = host.astype(small, copy=False)
     out = t.empty(host.shape, dtype=dtype, device=dev)
-    N.call("hgb_upload", N.ptr(out), host.ctypes.data, host.nbytes, N.stream_handle())
+    N.call("hgb_upload", out.data_ptr(), host.ctypes.data, host.nbytes, N.raw_stream(out.get_device()))
     return out
 
 
 def as_devices(*arrs, dev=None):
-    """:func:`as_device` of several float64 arrays; those of the host travel together, each on 16 bytes."""
+    """:func:`as_device` of several float64 arrays; the one-dimensional ones of the host travel together."""
     t = torch()
-    out = list(arrs)
     host = [ii for ii, aa in enumerate(arrs) if not isinstance(aa, t.Tensor)]
-    flat = [np.ascontiguousarray(arrs[ii]) for ii in host]
-    if any(aa.dtype != np.float64 or aa.size == 0 for aa in flat):
-        host = []
-    if len(host) > 1:
-        ends = np.cumsum([aa.size + (aa.size & 1) for aa in flat])
-        pack = np.zeros(int(ends[-1]))
-        for aa, end in zip(flat, ends):
-            begin = end - aa.size - (aa.size & 1)
-            pack[begin:begin + aa.size] = aa.ravel()
-        both = as_device(pack, dev)
-        for ii, aa, end in zip(host, flat, ends.tolist()):
-            out[ii] = both[end - aa.size - (aa.size & 1):][:aa.size].view(aa.shape)
-    return [as_device(aa, dev) for aa in out]
+    flat = [np.asarray(arrs[ii]) for ii in host]
+    if len(flat) < 2 or any(aa.dtype != np.float64 or aa.ndim != 1 for aa in flat):
+        return [as_device(aa, dev) for aa in arrs]
+    out = list(arrs)
+    parts = as_device(np.concatenate(flat), dev).split_with_sizes([aa.size for aa in flat])
+    for ii, part in zip(host, parts):
+        out[ii] = part
+    return out if len(host) == len(out) else [as_device(aa, dev) for aa in out]
 
 
 def is_torch(x):

@@ -258,6 +258,12 @@ def ptr(t):
     return ctypes.c_void_p(t.data_ptr())
 
 
+def raw_stream(index):
+    """The current stream of a device as an integer, without a stream object."""
+    import torch
+    return torch._C._cuda_getCurrentRawStream(index)
+
+
 def stream_handle(stream=None):
     import torch
     s = stream if stream is not None else torch.cuda.current_stream()

@@ -64,7 +64,7 @@ def test_arrays_that_travel_together():
         got = D.as_devices(*arrs)
         for g, a in zip(got, arrs):
             a = a.cpu().numpy() if a is tensor else a
-            assert g.dtype == torch.float64 and g.is_contiguous() and g.data_ptr() % 16 == 0
+            assert g.dtype == torch.float64 and g.is_contiguous() and g.data_ptr() % 8 == 0
             assert np.array_equal(g.cpu().numpy(), a)
 
 
