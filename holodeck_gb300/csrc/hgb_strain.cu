@@ -9,6 +9,8 @@
 #include <limits.h>
 #include <math.h>
 
+#include <algorithm>
+
 #include "hgb_common.cuh"
 
 namespace {
@@ -81,20 +83,56 @@ __device__ __forceinline__ double bin_strain(const StrainArgs &s, double z, doub
 // product.  9 and 26 FP64 operations an element where 16 and some 55 were, and FP64 bounds it.
 // 67 x 59 x 83 edges, 37 frequencies: number 305 us before, 263 us now, strain 1593 and 504 us;
 // both together (gwb), 41 x 31 x 37, 20 frequencies: 148 and 72 us.
-constexpr int CELL_THREADS = 256;
+constexpr int CELL_THREADS = 512;   // of a block, at most
+constexpr int CELL_FREQS = 256;     // frequencies side by side, at most
+
+// How a cell's (redshift bin, frequency) elements are shared out: `fb` frequencies side by side, runs of
+// `zlen` redshift bins, blockDim / fb runs a block and `parts` blocks a cell.
+struct CellSplit {
+    int fb, zlen, threads, parts;
+};
+
+// A warp's instruction costs the FP64 pipe the same with one live lane as with 32, and a run pays for the
+// plane below its first bin (a third of a bin's work), so the runs of a block minimise warps times steps;
+// of splits within 2% the widest, for the shorter chain.  With 256 threads whatever the counts, 129 to 255
+// frequencies left up to half of them idle and 257 took a second walk for one; number and strain together in
+// FP64 and in FP32, us before and now: 30^3 edges, 129 frequencies 318 and 270, 164 and 126; 181x161x20, 30
+// 1660 and 1261, 754 and 597; 91x81x101, 40 2180 and 2008, 943 and 881 (redshifts in every bin).
+// Cells that leave multiprocessors short of 16 warps are shared by several blocks, down to runs of 8 (3x3
+// cells of 299 redshift bins, 129 frequencies, the whole call in FP64: 739 and 126).
+CellSplit cell_split(int nf, int nzb, long cells) {
+    CellSplit c;
+    const int passes = (nf + CELL_FREQS - 1) / CELL_FREQS;
+    c.fb = (nf + passes - 1) / passes;
+    const int most = std::min(CELL_THREADS / c.fb, nzb);
+    auto cost = [&](int runs) { return (c.fb * runs + 31) / 32 * ((nzb + runs - 1) / runs + 0.33); };
+    const int step = std::max(1, most / 32);   // (a short search)
+    double best = cost(1);
+    for (int r = most; r > 1; r -= step) best = std::min(best, cost(r));
+    int runs = most;
+    while (runs > 1 && cost(runs) > 1.02 * best) runs = std::max(1, runs - step);
+    c.zlen = (nzb + runs - 1) / runs;
+    runs = (nzb + c.zlen - 1) / c.zlen;
+    c.threads = (c.fb * runs + 31) / 32 * 32;
+    runs = c.threads / c.fb;   // a small fb may leave room for more
+    const long warps = cells * (c.threads / 32);
+    const long want = std::min(hgb::ceil_div(16L * hgb::sm_count(), warps), hgb::ceil_div(c.zlen, 8L));
+    if (want > 1) c.zlen = (int)hgb::ceil_div(c.zlen, want);
+    c.parts = (int)hgb::ceil_div(nzb, (long)runs * c.zlen);
+    return c;
+}
 
 template <bool NUMBER, bool STRAIN>
-__global__ void __launch_bounds__(CELL_THREADS) k_cells(BinGeom g, StrainArgs s, const double *__restrict__ mtot, const double *__restrict__ log10_mtot,
+__global__ void __launch_bounds__(CELL_THREADS) k_cells(BinGeom g, CellSplit sp, StrainArgs s, const double *__restrict__ mtot, const double *__restrict__ log10_mtot,
                         const double *__restrict__ mrat, const double *__restrict__ redz,
                         const double *__restrict__ fedges, const double *__restrict__ dln_freq,
                         const double *__restrict__ dnum, const double *__restrict__ redz_final,
                         double *__restrict__ number, double *__restrict__ h2fdf, int *d_status) {
     const int cell = blockIdx.x;
     const int m = cell / (g.nq - 1), q = cell % (g.nq - 1);
-    const int fb = min(g.nf, CELL_THREADS);        // frequencies side by side
-    const int runs = CELL_THREADS / fb;            // redshift runs side by side
-    const int nzb = g.nz - 1, zlen = (nzb + runs - 1) / runs;
-    const int run = threadIdx.x / fb, z0 = run * zlen, z1 = min(z0 + zlen, nzb);
+    const int fb = sp.fb, runs = blockDim.x / fb;
+    const int nzb = g.nz - 1, run = threadIdx.x / fb;
+    const int z0 = (blockIdx.y * runs + run) * sp.zlen, z1 = min(z0 + sp.zlen, nzb);
     __shared__ double amp_mq;
     if (STRAIN) {
         if (threadIdx.x == 0) {
@@ -106,7 +144,7 @@ __global__ void __launch_bounds__(CELL_THREADS) k_cells(BinGeom g, StrainArgs s,
         }
         __syncthreads();
     }
-    if (run >= runs) return;
+    if (run >= runs || z0 >= z1) return;
     double dmdq = 0.0;
     if (NUMBER) dmdq = (log10_mtot[m + 1] - log10_mtot[m]) * (mrat[q + 1] - mrat[q]);
     const long plane = (long)g.nq * g.nz * g.nf, row = (long)g.nz * g.nf;   // steps along mtot, mrat
@@ -121,7 +159,7 @@ __global__ void __launch_bounds__(CELL_THREADS) k_cells(BinGeom g, StrainArgs s,
         }
         if (NUMBER) dlnf8 = dln_freq[f] * 0.125;
         double n00 = 0.0, n01 = 0.0, n10 = 0.0, n11 = 0.0, below = 0.0;   // the lower plane's values, its redshift sum
-        for (int z = z0; z <= z1 && z0 < z1; z++) {
+        for (int z = z0; z <= z1; z++) {
             const long v = vtx(g, m, q, z, f);
             const long out = ((long)cell * nzb + (z - 1)) * g.nf + f;
             const bool bin = z > z0;   // vertex z closes bin z - 1
@@ -199,9 +237,9 @@ __device__ __forceinline__ float dc_over_dh_f32(const StrainArgs32 &s, float z) 
 }
 
 constexpr int F32_MAX_FREQ = 256;   // per-frequency terms staged in shared memory, a thread for each
-static_assert(F32_MAX_FREQ <= CELL_THREADS, "every frequency has a thread");
+static_assert(F32_MAX_FREQ <= CELL_FREQS, "every frequency has a thread");
 
-__global__ void __launch_bounds__(CELL_THREADS) k_cells_f32(BinGeom g, StrainArgs32 s, double amp_scale, const double *__restrict__ mtot,
+__global__ void __launch_bounds__(CELL_THREADS) k_cells_f32(BinGeom g, CellSplit sp, StrainArgs32 s, double amp_scale, const double *__restrict__ mtot,
                             const double *__restrict__ log10_mtot, const double *__restrict__ mrat,
                             const double *__restrict__ redz, const double *__restrict__ fedges,
                             const double *__restrict__ dln_freq, const double *__restrict__ dnum,
@@ -245,11 +283,9 @@ __global__ void __launch_bounds__(CELL_THREADS) k_cells_f32(BinGeom g, StrainArg
     __syncthreads();
     const float amp_mq = s_amp_mq;
     const int ka = s_ka;
-    const int fb = g.nf;                             // frequencies side by side (F32_MAX_FREQ at most)
-    const int runs = CELL_THREADS / fb;              // redshift runs side by side
-    const int nzb = g.nz - 1, zlen = (nzb + runs - 1) / runs;
-    const int run = threadIdx.x / fb, f = threadIdx.x - run * fb;
-    const int z0 = run * zlen, z1 = min(z0 + zlen, nzb);
+    const int fb = sp.fb, runs = blockDim.x / fb;    // every frequency side by side
+    const int nzb = g.nz - 1, run = threadIdx.x / fb, f = threadIdx.x - run * fb;
+    const int z0 = (blockIdx.y * runs + run) * sp.zlen, z1 = min(z0 + sp.zlen, nzb);
     if (run >= runs || z0 >= z1) return;
     const float amp_f = s_amp_f[f], fcdf = s_fcdf[f], dlnf = s_dlnf[f];
     const int e2 = 2 * (ka + s_kf[f]);
@@ -443,8 +479,10 @@ int hgb_integrate_3dx1d(const double *log10_mtot, int n_mtot, const double *mrat
     HGB_CHECK_ARG(n_mtot >= 2 && n_mrat >= 2 && n_redz >= 2 && n_freq >= 1);
     BinGeom g{n_mtot, n_mrat, n_redz, n_freq};
     const StrainArgs s{0.0, nullptr, nullptr, nullptr, 0, -1, 0.0};
-    unsigned cells = (unsigned)((n_mtot - 1) * (n_mrat - 1));
-    k_cells<true, false><<<cells, CELL_THREADS, 0, (cudaStream_t)stream>>>(g, s, nullptr, log10_mtot, mrat, redz, nullptr,
+    const long cells = (long)(n_mtot - 1) * (n_mrat - 1);
+    const CellSplit sp = cell_split(n_freq, n_redz - 1, cells);
+    const dim3 grid((unsigned)cells, (unsigned)sp.parts);
+    k_cells<true, false><<<grid, sp.threads, 0, (cudaStream_t)stream>>>(g, sp, s, nullptr, log10_mtot, mrat, redz, nullptr,
                                                                   dln_freq, dnum, nullptr, number, nullptr, nullptr);
     return hgb::check_launch();
 }
@@ -457,8 +495,10 @@ int hgb_char_strain_sq(const double *mtot, int n_mtot, const double *mrat, int n
     HGB_CHECK_ARG(cosmo->dc_val && cosmo->dc_der && cosmo->dc_n >= 2);
     BinGeom g{n_mtot, n_mrat, n_redz, n_freq};
     const StrainArgs s = strain_args(gw_src_const, cosmo);
-    unsigned cells = (unsigned)((n_mtot - 1) * (n_mrat - 1));
-    k_cells<false, true><<<cells, CELL_THREADS, 0, (cudaStream_t)stream>>>(g, s, mtot, nullptr, mrat, nullptr, fobs_orb_edges,
+    const long cells = (long)(n_mtot - 1) * (n_mrat - 1);
+    const CellSplit sp = cell_split(n_freq, n_redz - 1, cells);
+    const dim3 grid((unsigned)cells, (unsigned)sp.parts);
+    k_cells<false, true><<<grid, sp.threads, 0, (cudaStream_t)stream>>>(g, sp, s, mtot, nullptr, mrat, nullptr, fobs_orb_edges,
                                                                      nullptr, nullptr, redz_final, nullptr, h2fdf,
                                                                      d_status);
     return hgb::check_launch();
@@ -476,10 +516,12 @@ int hgb_number_and_strain_f32(const double *mtot, const double *log10_mtot, int 
     HGB_CHECK_ARG(gw_src_const > 0.0);
     BinGeom g{n_mtot, n_mrat, n_redz, n_freq};
     StrainArgs32 s{cosmo->dcg_val, cosmo->dcg_der, cosmo->dc_n, 1.0f / (float)cosmo->dc_n};
-    unsigned cells = (unsigned)((n_mtot - 1) * (n_mrat - 1));
+    const long cells = (long)(n_mtot - 1) * (n_mrat - 1);
+    const CellSplit sp = cell_split(n_freq, n_redz - 1, cells);
+    const dim3 grid((unsigned)cells, (unsigned)sp.parts);
     size_t smem = sizeof(float) * (size_t)(n_redz - 1);
     HGB_CHECK_ARG(smem <= 32 * 1024);
-    k_cells_f32<<<cells, CELL_THREADS, smem, (cudaStream_t)stream>>>(g, s, gw_src_const / cosmo->hubble_distance, mtot,
+    k_cells_f32<<<grid, sp.threads, smem, (cudaStream_t)stream>>>(g, sp, s, gw_src_const / cosmo->hubble_distance, mtot,
                                                              log10_mtot, mrat, redz, fobs_orb_edges, dln_freq, dnum,
                                                              redz_final, number, h2fdf, d_status);
     return hgb::check_launch();
@@ -495,8 +537,10 @@ int hgb_number_and_strain(const double *mtot, const double *log10_mtot, int n_mt
     HGB_CHECK_ARG(cosmo->dc_val && cosmo->dc_der && cosmo->dc_n >= 2);
     BinGeom g{n_mtot, n_mrat, n_redz, n_freq};
     const StrainArgs s = strain_args(gw_src_const, cosmo);
-    unsigned cells = (unsigned)((n_mtot - 1) * (n_mrat - 1));
-    k_cells<true, true><<<cells, CELL_THREADS, 0, (cudaStream_t)stream>>>(g, s, mtot, log10_mtot, mrat, redz, fobs_orb_edges,
+    const long cells = (long)(n_mtot - 1) * (n_mrat - 1);
+    const CellSplit sp = cell_split(n_freq, n_redz - 1, cells);
+    const dim3 grid((unsigned)cells, (unsigned)sp.parts);
+    k_cells<true, true><<<grid, sp.threads, 0, (cudaStream_t)stream>>>(g, sp, s, mtot, log10_mtot, mrat, redz, fobs_orb_edges,
                                                                     dln_freq, dnum, redz_final, number, h2fdf, d_status);
     return hgb::check_launch();
 }
