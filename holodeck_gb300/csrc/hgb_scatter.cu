@@ -541,7 +541,8 @@ size_t hgb_scatter_workspace_bytes(int n_mtot, int n_mrat, int n_redz, int n_gri
     size_t n = (size_t)n_mtot * n_mrat, NN = (size_t)n_grid * n_grid;
     const size_t last = std::max(NN, 2 * HGB_SCATTER_STAGES * n);   // the regular grid; the sweeps in flight
     return align256(sizeof(double) * n * n_redz) + 2 * align256(sizeof(double) * 2 * n * n_redz) +
-           align256(sizeof(double) * last * n_redz) + align256(sizeof(short) * n_grid * (((size_t)n_grid + 31) / 32) * n_redz);
+           align256(sizeof(double) * last * n_redz) +
+           align256(sizeof(short) * n_grid * (((size_t)n_grid + 31) / 32) * n_redz) + 16;   // the base, rounded up
 }
 
 int hgb_add_scatter_to_masses(const hgb_scatter_plan *plan, double *dens, int n_redz, void *workspace,
@@ -555,7 +556,7 @@ int hgb_add_scatter_to_masses(const hgb_scatter_plan *plan, double *dens, int n_
     size_t need = hgb_scatter_workspace_bytes(P.n_mtot, P.n_mrat, n_redz, P.n_grid);
     if (!workspace || workspace_bytes < need) return HGB_ERR_WORKSPACE;
     const size_t n = (size_t)P.n_mtot * P.n_mrat, NN = (size_t)P.n_grid * P.n_grid;
-    char *w = (char *)workspace;
+    char *w = (char *)(((uintptr_t)workspace + 15) & ~(uintptr_t)15);   // pairs of doubles are read whole
     double *vals = (double *)w;
     w += align256(sizeof(double) * n * n_redz);
     double *grads = (double *)w;
@@ -573,7 +574,8 @@ int hgb_add_scatter_to_masses(const hgb_scatter_plan *plan, double *dens, int n_
     cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     // the phases where the plan has them and their table fits one SM; the gradients beside it where
     // they fit too (grids up to about 14000 points)
-    if (P.ph_ptr && P.ph_info && P.ph_nbr && P.ph_m && P.n_phases >= 1 && P.phase_width >= 1 &&
+    const bool aligned = (((uintptr_t)P.ph_ptr | (uintptr_t)P.ph_info | (uintptr_t)P.ph_m) & 15) == 0;   // rows of 16 bytes
+    if (P.ph_ptr && P.ph_info && P.ph_nbr && P.ph_m && aligned && P.n_phases >= 1 && P.phase_width >= 1 &&
         gradients_smem(P, false) + 1024 <= (size_t)smem_optin) {
         HGB_CHECK_ARG((P.n_levels - 1) / P.n_phases < HGB_SCATTER_STAGES);
         k_scatter_rhs<<<dim3((unsigned)hgb::ceil_div((long)n, 8), (unsigned)hgb::ceil_div(n_redz, 32)), dim3(32, 8), 0,

@@ -32,7 +32,8 @@ struct StrainArgs {
 };
 
 StrainArgs strain_args(double k, const hgb_cosmo *c) {
-    StrainArgs s{k, c->dc_val, c->dc_der, (const double2 *)c->dc_cub, c->dc_n, -1, 1.0 / c->dc_n};
+    const bool pairs = ((uintptr_t)c->dc_cub & 15) == 0;   // else as without the table
+    StrainArgs s{k, c->dc_val, c->dc_der, pairs ? (const double2 *)c->dc_cub : nullptr, c->dc_n, -1, 1.0 / c->dc_n};
     if ((c->dc_n & (c->dc_n - 1)) == 0 && c->dc_n <= (1 << 20)) {
         s.dc_log2 = 0;
         while ((1 << s.dc_log2) < c->dc_n) s.dc_log2++;

@@ -73,8 +73,8 @@ typedef struct {
      * g (dimensionless) and dg/du on the same nodes u = k / dc_n, cubic Hermite between them */
     const float *dcg_val;   /* [dc_n + 1] */
     const float *dcg_der;   /* [dc_n + 1] */
-    /* the Hermite cubics of dc_val / dc_der as polynomials in t = u dc_n - k, lowest power first (16-byte
-     * aligned; may be NULL: formed from dc_val / dc_der where they are used) */
+    /* the Hermite cubics of dc_val / dc_der as polynomials in t = u dc_n - k, lowest power first (may be
+     * NULL or off a 16-byte boundary: then formed from dc_val / dc_der where they are used) */
     const double *dc_cub;   /* [dc_n][4] */
 } hgb_cosmo;
 
@@ -191,7 +191,7 @@ typedef struct {    /* the same arrays on the device */
     const double *ph_m;
     double grad_tol;    /* 1e-6 in the reference */
     int grad_maxiter;   /* 400 in the reference */
-    int n_phases, phase_width;   /* 0 (or a NULL ph_ array): sweeps one after another */
+    int n_phases, phase_width;   /* 0 (or a ph_ array that is NULL or off a 16-byte boundary): sweeps one after another */
 } hgb_scatter_plan;
 
 #define HGB_SCATTER_DEG 8      /* a point with more neighbours is summed by a whole warp */
