@@ -142,6 +142,8 @@ __global__ void __launch_bounds__(CELL_THREADS) k_cells(BinGeom g, CellSplit sp,
             const double mr = 0.5 * (mrat[q + 1] + mrat[q]);
             const double c = cbrt(mt), opq = 1.0 + mr;
             amp_mq = s.gw_src_const * 1.5874010519681994748 * (mt * (c * c) * mr / (opq * opq));   // 2^(2/3)
+            // the fractional powers of a negative ratio or chirp mass are NaN
+            if (mr < 0.0 || (mt < 0.0 && mr > 0.0)) amp_mq = NAN;
         }
         __syncthreads();
     }
@@ -155,7 +157,7 @@ __global__ void __launch_bounds__(CELL_THREADS) k_cells(BinGeom g, CellSplit sp,
         if (STRAIN) {
             const double fc = 0.5 * (fedges[f + 1] + fedges[f]);
             const double c = cbrt(fc);
-            amp = amp_mq * (c * c);
+            amp = fc < 0.0 ? NAN : amp_mq * (c * c);
             fc_df = fc / (fedges[f + 1] - fedges[f]);
         }
         if (NUMBER) dlnf8 = dln_freq[f] * 0.125;
