@@ -1412,6 +1412,10 @@ int hgb_dbn_2pwl_phase(const double *fobs_orb, int n_freq, int fobs_sorted, doub
     unsigned blocks = (unsigned)((long)n_mtot * n_mrat);
     if (phase & 1) {
         const WalkShape ws = walk_shape(a);
+        // what the walk in any order needs for one cell bounds the tables of both
+        const size_t base = sizeof(double) * ((size_t)4 * cosmo->grid_size + n_freq);
+        const size_t per_cell = sizeof(double) * (3 * (size_t)(num_steps + 1) + 2 * (size_t)num_steps);
+        HGB_CHECK_ARG(base + per_cell <= 200 * 1024);
         // ascending targets, step and interval numbers that fit the walk's 16-bit notes, and tables that
         // fit one SM; any other call takes the FP64 walk
         if (fobs_sorted && num_steps < 0xFFFF && cosmo->grid_size < 0xFFFF && ws.smem <= 200 * 1024) {
@@ -1425,9 +1429,6 @@ int hgb_dbn_2pwl_phase(const double *fobs_orb, int n_freq, int fobs_sorted, doub
             if (rc) return rc;
         } else {
             // cells per block: fill up to 512 rows (cpb x n_redz), within a shared-memory budget
-            const size_t base = sizeof(double) * ((size_t)4 * cosmo->grid_size + n_freq);
-            const size_t per_cell = sizeof(double) * (3 * (size_t)(num_steps + 1) + 2 * (size_t)num_steps);
-            HGB_CHECK_ARG(base + per_cell <= 200 * 1024);
             int cpb = 512 / n_redz;
             cpb = std::min<long>(cpb, (long)((160 * 1024 - std::min<size_t>(base, 160 * 1024)) / per_cell));
             cpb = std::max(1, std::min(cpb, WALK_MAX_CELLS));

@@ -86,6 +86,7 @@ __device__ __forceinline__ double bin_strain(const StrainArgs &s, double z, doub
 // both together (gwb), 41 x 31 x 37, 20 frequencies: 148 and 72 us.
 constexpr int CELL_THREADS = 512;   // of a block, at most
 constexpr int CELL_FREQS = 256;     // frequencies side by side, at most
+constexpr int STRAIN_MAX_FREQ = 3072;   // that the strain's entry points take
 
 // How a cell's (redshift bin, frequency) elements are shared out: `fb` frequencies side by side, runs of
 // `zlen` redshift bins, blockDim / fb runs a block and `parts` blocks a cell.
@@ -497,6 +498,7 @@ int hgb_char_strain_sq(const double *mtot, int n_mtot, const double *mrat, int n
     HGB_CHECK_ARG(n_mtot >= 2 && n_mrat >= 2 && n_redz >= 2 && n_freq >= 1);
     HGB_CHECK_ARG(cosmo->dc_val && cosmo->dc_der && cosmo->dc_n >= 2);
     BinGeom g{n_mtot, n_mrat, n_redz, n_freq};
+    HGB_CHECK_ARG(n_freq <= STRAIN_MAX_FREQ);
     const StrainArgs s = strain_args(gw_src_const, cosmo);
     const long cells = (long)(n_mtot - 1) * (n_mrat - 1);
     const CellSplit sp = cell_split(n_freq, n_redz - 1, cells);
@@ -539,6 +541,7 @@ int hgb_number_and_strain(const double *mtot, const double *log10_mtot, int n_mt
     HGB_CHECK_ARG(n_mtot >= 2 && n_mrat >= 2 && n_redz >= 2 && n_freq >= 1);
     HGB_CHECK_ARG(cosmo->dc_val && cosmo->dc_der && cosmo->dc_n >= 2);
     BinGeom g{n_mtot, n_mrat, n_redz, n_freq};
+    HGB_CHECK_ARG(n_freq <= STRAIN_MAX_FREQ);
     const StrainArgs s = strain_args(gw_src_const, cosmo);
     const long cells = (long)(n_mtot - 1) * (n_mrat - 1);
     const CellSplit sp = cell_split(n_freq, n_redz - 1, cells);
