@@ -387,8 +387,7 @@ def run_gpu(args):
     emulator = run_emulator(args) if (args.emulator_samples > 0 and world == 1) else None
     cpu = hc_error = None
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
-        cpu, keep = cpu_baseline_sample(args)
-        hc_error = hc_error_vs_reference(keep, args.precision)
+        cpu, hc_error = cpu_fields(args)
     if rank == 0:
         line = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
@@ -645,6 +644,23 @@ def cpu_baseline_sample(args):
                        f"91x81x{SAMPLE_Z} with {SAMPLE_R} realizations, extrapolated linearly in redshift bins and "
                        f"realizations: grid stages {grid:.1f} s + {per_real:.2f} s/realization "
                        f"({', '.join(f'{k} {v:.2f}s' for k, v in t.items())})")}, keep
+
+
+def cpu_fields(args):
+    """The line's (cpu_baseline, hc_error).  Both need the reference's kernels built on this host; without them
+    (or with a leg that raises) the field says why, and the line keeps its measurements."""
+    def unavailable(exc):
+        print(f"bench: CPU leg left out: {exc!r}", file=sys.stderr)
+        return {"unavailable": " ".join(f"{type(exc).__name__}: {exc}".split())}
+
+    try:
+        cpu, keep = cpu_baseline_sample(args)
+    except Exception as exc:
+        return unavailable(exc), None
+    try:
+        return cpu, hc_error_vs_reference(keep, args.precision)
+    except Exception as exc:
+        return cpu, unavailable(exc)
 
 
 def hc_error_vs_reference(keep, precision, nreals=8):
