@@ -178,10 +178,11 @@ __device__ __forceinline__ double f32_to_f64_scaled(float v, int k) {
 // the bit pattern of -1.0, the "no target reached" sentinel of redz_final
 constexpr long long F64_MINUS_ONE_BITS = (long long)0xBFF0000000000000ull;
 
-// 1 / y and 1 / sqrt(y) in FP64 from the hardware's estimate r (relative error a few 2^-21 of the value
-// with y's low word cleared): with e = 1 - y r, 1 / y = r (1 + e + e^2 + ...), and with e = 1 - y r^2,
-// 1 / sqrt(y) = r (1 + e / 2 + 3 e^2 / 8 + ...).  The series cut after e^2 leaves less than 2^-57, so
-// the result carries one or two roundings.  Three and five FP64 operations in place of the eight to
+// 1 / y and 1 / sqrt(y) in FP64 from the hardware's estimate r: with e = 1 - y r, 1 / y = r (1 + e + e^2 + ...),
+// and with e = 1 - y r^2, 1 / sqrt(y) = r (1 + e / 2 + 3 e^2 / 8 + ...).  The estimate is of y with its low
+// word cleared (up to 2^-20 of it) and is itself a few 2^-21 off, so |e| stays below 2^-18.6 and 2^-18, and
+// what the series cut after e^2 leaves below 2^-55.  The quotient then carries one rounding and the root one
+// and a half (that of y r enters halved): within 2^-53 + 2^-55 and 1.5 2^-53 + 2^-55.  Three and five FP64 operations in place of the eight to
 // twelve of a correctly rounded quotient or root, on a GPU whose FP64 pipe sets these kernels' time.
 // y positive and within 2^+-900 (no zero, subnormal, infinity or NaN: the caller sees to it).
 __device__ __forceinline__ double fast_rcp(double y) {
