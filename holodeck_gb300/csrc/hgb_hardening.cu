@@ -1101,7 +1101,7 @@ __global__ void __launch_bounds__(GW_ROWS) k_dbn_gw(CyConst cc, const double *__
         s_isco[t] = cc.kfreq * sqrt(mt) / pow(3.0 * HGB_CY_SCHW * mt, 1.5);
     }
     // the row's redshift terms: A without the cell's constant
-    double rzp = -1.0, zp1 = 0.0, part = 0.0, z_third = 0.0;
+    double rzp = -1.0, zp1 = 0.0, part = 0.0, z_third = 0.0, scale = 1.0;
     const int cell = (z0 + t) / nz;
     if (t < nrb) {
         rzp = redz_prime[row0 + t];
@@ -1111,7 +1111,11 @@ __global__ void __launch_bounds__(GW_ROWS) k_dbn_gw(CyConst cc, const double *__
             const double dcom = hgb::interp_between(rzp, zgrid[zi], zgrid[zi + 1], dgrid[zi], dgrid[zi + 1]);
             const double dcm = dcom / HGB_CY_MPC;
             zp1 = 1.0 + rzp;
-            part = nden[row0 + t] * (cc.fourpi * zp1 * (dcm * dcm));
+            // densities near the least double (a mass function's cutoff) are carried up, so that a small
+            // factor before a large one takes none of their bits
+            const double nd = nden[row0 + t];
+            scale = ((unsigned)__double2hiint(nd) >> 20 & 0x7FFu) < 323u ? 0x1.0p-200 : 1.0;
+            part = (scale < 1.0 ? nd * 0x1.0p200 : nd) * (cc.fourpi * zp1 * (dcm * dcm));
             z_third = cbrt(zp1);
         }
     }
@@ -1136,7 +1140,7 @@ __global__ void __launch_bounds__(GW_ROWS) k_dbn_gw(CyConst cc, const double *__
             int cut = 0;
             if (!(rzp <= 0.0)) {
                 // (1 + z)^(-8/3) = cbrt(1 + z) / (1 + z)^3
-                amp = part * (s_k[cell] * z_third / (zp1 * zp1 * zp1));
+                amp = part * (s_k[cell] * z_third / (zp1 * zp1 * zp1)) * scale;
                 const double isco = s_isco[cell];
                 int hi = nfb;   // first f with ftop[f] (1 + z) > isco
                 while (cut < hi) {

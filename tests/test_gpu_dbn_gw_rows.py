@@ -56,3 +56,19 @@ def test_few_redshifts_cost_what_many_do(built_lib):
             times.append(begin.elapsed_time(end))
         best.append(min(times))
     assert best[0] < 4.0 * best[1], best
+
+
+@pytest.mark.parametrize("dens", [1e-300, 1e-305, 1e-310, 5e-324])
+def test_least_densities(built_lib, dens):
+    """Densities down to the least double keep their bits: RTOL of the value and a step of the subnormals."""
+    import torch
+    from holodeck_gb300.sams import sam_cyutils
+    fobs, like, mtot, mrat, zp = _inputs(7, 5, 1, 9)
+    full = np.full(like.shape, dens)
+    rf, dn = O.dbn_gw(fobs, full, mtot, mrat, zp)
+    dev = [torch.as_tensor(x, device="cuda") for x in (fobs, full, mtot, mrat, zp)]
+    grf, gdn = (x.cpu().numpy() for x in sam_cyutils.dbn_gw_device(*dev))
+    assert np.array_equal(grf, rf) and dn.max() > 0.0
+    # the reference rounds to a subnormal once or twice on its way, each half a step of what follows
+    slack = 5e-324 * (2.0 + dn / dens)
+    assert np.all(np.abs(gdn - dn) <= RTOL * dn + slack)
