@@ -5,8 +5,8 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-SIZES = [("float64", 1), ("float64", 125), ("float64", 126), ("float64", 4000), ("float64", 4001), ("float32", 100),
-         ("float32", 8000), ("int32", 7), ("float64", 0)]   # around one launch and its two argument sizes
+SIZES = [("float64", 1), ("float64", 125), ("float64", 126), ("float64", 500), ("float64", 501), ("float64", 4000), ("float64", 4001), ("float32", 100),
+         ("float32", 8000), ("int32", 7), ("float64", 0)]   # around one launch and its argument sizes
 
 
 @pytest.mark.parametrize("dtype,n", SIZES)
