@@ -1,19 +1,21 @@
 // Binary hardening on the GPU:
 //  * hgb_find_2pwl_hardening_norm: Brent root of the two-power-law lifetime per (mtot, mrat) cell
-//    (holodeck/sams/sam_cyutils.pyx:289-398); one warp per cell.
-//  * hgb_dbn_2pwl: differential binary number for Fixed_Time_2PL_SAM (sam_cyutils.pyx:510-781) in
-//    two phases: k_dbn_2pwl walks the separation steps (one block per (mtot, mrat) cell, one thread
-//    per starting redshift, step tables in shared memory) and records, per target frequency, the
-//    interpolated time of the bracketing step; k_dbn_2pwl_eval then evaluates redshift, distance,
-//    residence time and number for every bracketed (redz, frequency) element in parallel, with the
-//    model's (half-)integer exponents taken as products and square roots instead of pow().  The
-//    age -> redshift / distance interpolations use per-interval slopes computed once per block
-//    (a multiply instead of a divide per lookup; results differ from the reference's divide by an ulp).
+//    (holodeck/sams/sam_cyutils.pyx:289-398).  k_hardening_norm_sub: two or four cells a warp, the nodes of a
+//    total mass shared by a block; k_hardening_norm, a warp per cell, beyond its 320 steps.
+//  * hgb_dbn_2pwl: differential binary number for Fixed_Time_2PL_SAM (sam_cyutils.pyx:510-781) in two phases.
+//    The first records, per starting redshift and target frequency, the interpolated time of the separation
+//    step that brackets the target: k_dbn_2pwl_walk for ascending targets (several mrat cells of one mtot a
+//    block; steps found in FP32, brackets evaluated in FP64), k_dbn_2pwl for targets in any order, or tables
+//    beyond the first's limits.  k_dbn_2pwl_eval then evaluates redshift, distance, residence time and number
+//    of every bracketed (redz, frequency) element, the model's (half-)integer exponents as products and
+//    roots instead of pow().  The age -> redshift / distance interpolations use per-interval slopes computed
+//    once per block (a multiply instead of a divide per lookup; an ulp from the reference's divide).
 //  * hgb_dbn_gw: differential binary number for Hard_GW (sam_cyutils.pyx:788-899); one block per
 //    run of up to 256 (mtot, mrat, redz) points.
 // FP64 throughout (the hardening integral and the lookback-time -> redshift inversion are the
-// FP64 islands of the path).  Built with -fmad=false so operation order and rounding follow the
-// reference loops; the remaining differences are the last-ulp behaviour of pow/log10.
+// FP64 islands of the path).  Built with -fmad=false: k_hardening_norm, k_dbn_2pwl and the walk's nodes and
+// running times keep the reference loops' order and rounding, to the last-ulp behaviour of pow/log10.  The
+// other kernels regroup: explicit multiply-adds, fast_rcp / fast_rsqrt for quotients and roots, shared powers.
 #include <math.h>
 
 #include <algorithm>
@@ -443,8 +445,8 @@ __device__ __forceinline__ double shape_outer(double y, double p, PowPlan plan) 
 //      time is one.  (At the end, so that the rows' walk and search keep their registers.)
 // FP64 bounds both forms, but the walk in FP64 spent some 25 operations a step on 80 steps a row,
 // comparisons among them, with lanes idle where their neighbours walk longer, and wrote its outputs
-// eight bytes to a line.  91 x 81 x 101 points, 40 targets: 3130 us before, 1002 us now (FP64 pipe 75% busy); 30^3 points
-// with 20: 443 and 147 us.
+// eight bytes to a line.  91 x 81 x 101 points, 40 targets: 3130 us before, 930 us now (FP64 pipe 72% busy); 30^3 points
+// with 20: 443 and 141 us.
 constexpr int WK_THREADS = 256;
 constexpr unsigned WK_NONE = 0xFFFFFFFFu, WK_LATER = 0xFFFFFFFEu;   // no bracket; a row of C
 constexpr double WK_SCALE = 0x1.0p40;   // of the FP64 frequencies, some 1e-10 Hz: keeps the bracket's products in range

@@ -102,8 +102,9 @@ __global__ void k_gradients(hgb_scatter_plan P, const double *__restrict__ dens,
 // Two lanes per point, one per component, 16 points per warp, or four, a component's neighbours halved.  A point with more than HGB_SCATTER_DEG
 // neighbours (the hull's fans, up to 82) takes a warp: 16 lane pairs share its neighbours.  The static
 // entries of a warp's points in the next phase are loaded while the current phase computes.
-// FP64 bounds a phase: 90 points of about 6 neighbours are 6 warps of 13 to 15 FP64 instructions on
-// four sub-partitions, 1900 of its 2400 cycles.  91 x 81 points, 101 slices: 4283 us one level at a
+// A phase is bound by its fullest sub-partitions: 90 points of about 6 neighbours are 6 warps of 13 to 15
+// FP64 instructions, two warps on two of the four, 1900 cycles in a row, then the reduction and the barrier
+// (ncu: the FP64 pipes of the multiprocessors that hold a slice are 39% busy).  91 x 81 points, 101 slices: 4283 us one level at a
 // time, 1896 us with sweeps in flight (and 69 us for c); 181 x 161, 201 slices, where the slice exceeds
 // shared memory and its gradients stay in L2: 78.5 and 13.0 ms.  There the loads are the longer chain
 // and the second wave of blocks costs as much as the first, so with more slices than multiprocessors

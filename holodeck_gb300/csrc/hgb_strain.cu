@@ -8,6 +8,7 @@
 // (see bin_strain), which moves it by a few ulp.
 #include <limits.h>
 #include <math.h>
+#include <stdlib.h>
 
 #include <algorithm>
 
@@ -84,7 +85,8 @@ __device__ __forceinline__ double bin_strain(const StrainArgs &s, double z, doub
 // product.  9 and 26 FP64 operations an element where 16 and some 55 were, and FP64 bounds it.
 // 67 x 59 x 83 edges, 37 frequencies: number 305 us before, 263 us now, strain 1593 and 504 us;
 // both together (gwb), 41 x 31 x 37, 20 frequencies: 148 and 72 us.
-constexpr int CELL_THREADS = 512;   // of a block, at most
+constexpr int CELL_THREADS = 512;       // of a block, at most
+constexpr int CELL_F32_THREADS = 288;   // of an FP32 block: more leave an SM fewer warps (51 registers)
 constexpr int CELL_FREQS = 256;     // frequencies side by side, at most
 constexpr int STRAIN_MAX_FREQ = 3072;   // that the strain's entry points take
 
@@ -96,23 +98,29 @@ struct CellSplit {
 
 // A warp's instruction costs the FP64 pipe the same with one live lane as with 32, and a run pays for the
 // plane below its first bin (a third of a bin's work), so the runs of a block minimise warps times steps;
-// of splits within 2% the widest, for the shorter chain.  With 256 threads whatever the counts, 129 to 255
+// of splits within 1% the one nearest to 128 threads.  With 256 threads whatever the counts, 129 to 255
 // frequencies left up to half of them idle and 257 took a second walk for one; number and strain together in
 // FP64 and in FP32, us before and now: 30^3 edges, 129 frequencies 318 and 270, 164 and 126; 181x161x20, 30
 // 1660 and 1261, 754 and 597; 91x81x101, 40 2180 and 2008, 943 and 881 (redshifts in every bin).
 // Cells that leave multiprocessors short of 16 warps are shared by several blocks, down to runs of 8 (3x3
 // cells of 299 redshift bins, 129 frequencies, the whole call in FP64: 739 and 126).
-CellSplit cell_split(int nf, int nzb, long cells) {
+CellSplit cell_split(int nf, int nzb, long cells, int threads) {
     CellSplit c;
     const int passes = (nf + CELL_FREQS - 1) / CELL_FREQS;
     c.fb = (nf + passes - 1) / passes;
-    const int most = std::min(CELL_THREADS / c.fb, nzb);
+    const int most = std::min(threads / c.fb, nzb);
     auto cost = [&](int runs) { return (c.fb * runs + 31) / 32 * ((nzb + runs - 1) / runs + 0.33); };
     const int step = std::max(1, most / 32);   // (a short search)
     double best = cost(1);
     for (int r = most; r > 1; r -= step) best = std::min(best, cost(r));
-    int runs = most;
-    while (runs > 1 && cost(runs) > 1.02 * best) runs = std::max(1, runs - step);
+    int runs = 1, off = INT_MAX;
+    for (int r = most; r >= 1; r = r == 1 ? 0 : std::max(1, r - step)) {
+        const int d = std::abs((c.fb * r + 31) / 32 * 32 - 128);
+        if (cost(r) <= 1.01 * best && d < off) {
+            runs = r;
+            off = d;
+        }
+    }
     c.zlen = (nzb + runs - 1) / runs;
     runs = (nzb + c.zlen - 1) / c.zlen;
     c.threads = (c.fb * runs + 31) / 32 * 32;
@@ -243,7 +251,7 @@ __device__ __forceinline__ float dc_over_dh_f32(const StrainArgs32 &s, float z) 
 constexpr int F32_MAX_FREQ = 256;   // per-frequency terms staged in shared memory, a thread for each
 static_assert(F32_MAX_FREQ <= CELL_FREQS, "every frequency has a thread");
 
-__global__ void __launch_bounds__(CELL_THREADS) k_cells_f32(BinGeom g, CellSplit sp, StrainArgs32 s, double amp_scale, const double *__restrict__ mtot,
+__global__ void __launch_bounds__(CELL_F32_THREADS) k_cells_f32(BinGeom g, CellSplit sp, StrainArgs32 s, double amp_scale, const double *__restrict__ mtot,
                             const double *__restrict__ log10_mtot, const double *__restrict__ mrat,
                             const double *__restrict__ redz, const double *__restrict__ fedges,
                             const double *__restrict__ dln_freq, const double *__restrict__ dnum,
@@ -484,7 +492,7 @@ int hgb_integrate_3dx1d(const double *log10_mtot, int n_mtot, const double *mrat
     BinGeom g{n_mtot, n_mrat, n_redz, n_freq};
     const StrainArgs s{0.0, nullptr, nullptr, nullptr, 0, -1, 0.0};
     const long cells = (long)(n_mtot - 1) * (n_mrat - 1);
-    const CellSplit sp = cell_split(n_freq, n_redz - 1, cells);
+    const CellSplit sp = cell_split(n_freq, n_redz - 1, cells, CELL_THREADS);
     const dim3 grid((unsigned)cells, (unsigned)sp.parts);
     k_cells<true, false><<<grid, sp.threads, 0, (cudaStream_t)stream>>>(g, sp, s, nullptr, log10_mtot, mrat, redz, nullptr,
                                                                   dln_freq, dnum, nullptr, number, nullptr, nullptr);
@@ -501,7 +509,7 @@ int hgb_char_strain_sq(const double *mtot, int n_mtot, const double *mrat, int n
     HGB_CHECK_ARG(n_freq <= STRAIN_MAX_FREQ);
     const StrainArgs s = strain_args(gw_src_const, cosmo);
     const long cells = (long)(n_mtot - 1) * (n_mrat - 1);
-    const CellSplit sp = cell_split(n_freq, n_redz - 1, cells);
+    const CellSplit sp = cell_split(n_freq, n_redz - 1, cells, CELL_THREADS);
     const dim3 grid((unsigned)cells, (unsigned)sp.parts);
     k_cells<false, true><<<grid, sp.threads, 0, (cudaStream_t)stream>>>(g, sp, s, mtot, nullptr, mrat, nullptr, fobs_orb_edges,
                                                                      nullptr, nullptr, redz_final, nullptr, h2fdf,
@@ -522,7 +530,7 @@ int hgb_number_and_strain_f32(const double *mtot, const double *log10_mtot, int 
     BinGeom g{n_mtot, n_mrat, n_redz, n_freq};
     StrainArgs32 s{cosmo->dcg_val, cosmo->dcg_der, cosmo->dc_n, 1.0f / (float)cosmo->dc_n};
     const long cells = (long)(n_mtot - 1) * (n_mrat - 1);
-    const CellSplit sp = cell_split(n_freq, n_redz - 1, cells);
+    const CellSplit sp = cell_split(n_freq, n_redz - 1, cells, CELL_F32_THREADS);
     const dim3 grid((unsigned)cells, (unsigned)sp.parts);
     size_t smem = sizeof(float) * (size_t)(n_redz - 1);
     HGB_CHECK_ARG(smem <= 32 * 1024);
@@ -544,7 +552,7 @@ int hgb_number_and_strain(const double *mtot, const double *log10_mtot, int n_mt
     HGB_CHECK_ARG(n_freq <= STRAIN_MAX_FREQ);
     const StrainArgs s = strain_args(gw_src_const, cosmo);
     const long cells = (long)(n_mtot - 1) * (n_mrat - 1);
-    const CellSplit sp = cell_split(n_freq, n_redz - 1, cells);
+    const CellSplit sp = cell_split(n_freq, n_redz - 1, cells, CELL_THREADS);
     const dim3 grid((unsigned)cells, (unsigned)sp.parts);
     k_cells<true, true><<<grid, sp.threads, 0, (cudaStream_t)stream>>>(g, sp, s, mtot, log10_mtot, mrat, redz, fobs_orb_edges,
                                                                     dln_freq, dnum, redz_final, number, h2fdf, d_status);
