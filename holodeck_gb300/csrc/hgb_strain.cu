@@ -3,7 +3,7 @@
 //  * STRAIN: char_strain_sq_from_bin_edges_redz (holodeck/gravwaves.py:694-724)
 //  * both in one pass for gwb() (sam.py:930-935): each vertex of dnum and redz_final is read by the four
 //    (mtot, mrat) cells that share it, and number / h2fdf are written once.
-// One block per (mtot, mrat) cell, the frequency fastest over its threads.  Built with -fmad=false: the
+// One block, or a few, per (mtot, mrat) cell, the frequency fastest over its threads.  Built with -fmad=false: the
 // eight-vertex sum and the midpoints round like the Cython/numpy code; the strain product is regrouped
 // (see bin_strain), which moves it by a few ulp.
 #include <limits.h>
@@ -75,7 +75,7 @@ __device__ __forceinline__ double bin_strain(const StrainArgs &s, double z, doub
     return (hs * hs) * fc_df;
 }
 
-// One block per (mtot, mrat) bin cell.  A thread keeps one frequency (the threads' fastest index, so a
+// One block, or a few, per (mtot, mrat) bin cell (cell_split).  A thread keeps one frequency (the threads' fastest index, so a
 // warp's loads and stores are contiguous) and walks a run of redshifts, taking each vertex plane's values
 // from memory once:
 //   * the eight-vertex sum of the number keeps the reference's order, bit for bit;
@@ -84,7 +84,7 @@ __device__ __forceinline__ double bin_strain(const StrainArgs &s, double z, doub
 // The sentinel and sign tests read the values' bits: an FP64 comparison holds the pipe as long as a
 // product.  9 and 26 FP64 operations an element where 16 and some 55 were, and FP64 bounds it.
 // 67 x 59 x 83 edges, 37 frequencies: number 305 us before, 263 us now, strain 1593 and 504 us;
-// both together (gwb), 41 x 31 x 37, 20 frequencies: 148 and 72 us.
+// both together (gwb), 41 x 31 x 37, 20 frequencies: 148 and 67 us.
 constexpr int CELL_THREADS = 512;       // of a block, at most
 constexpr int CELL_F32_THREADS = 288;   // of an FP32 block: more leave an SM fewer warps (51 registers)
 constexpr int CELL_FREQS = 256;     // frequencies side by side, at most
@@ -100,8 +100,9 @@ struct CellSplit {
 // plane below its first bin (a third of a bin's work), so the runs of a block minimise warps times steps;
 // of splits within 1% the one nearest to 128 threads.  With 256 threads whatever the counts, 129 to 255
 // frequencies left up to half of them idle and 257 took a second walk for one; number and strain together in
-// FP64 and in FP32, us before and now: 30^3 edges, 129 frequencies 318 and 270, 164 and 126; 181x161x20, 30
-// 1660 and 1261, 754 and 597; 91x81x101, 40 2180 and 2008, 943 and 881 (redshifts in every bin).
+// FP64 and in FP32, us before and now, redshifts in three bins of four: 91x81x101 edges, 129 frequencies 6892
+// and 6199, 1704 and 1408; 40 frequencies 2033 and 1854, 497 and 425; 5 frequencies 358 and 323, 112 and 82;
+// 60^3, 200 2760 and 2748, 703 and 626; 181x161x201, 100 38982 and 35723, 8976 and 8725.
 // Cells that leave multiprocessors short of 16 warps are shared by several blocks, down to runs of 8 (3x3
 // cells of 299 redshift bins, 129 frequencies, the whole call in FP64: 739 and 126).
 CellSplit cell_split(int nf, int nzb, long cells, int threads) {
@@ -218,7 +219,7 @@ __global__ void __launch_bounds__(CELL_THREADS) k_cells(BinGeom g, CellSplit sp,
 //   from the FP32 table of hgb_cosmo; h2fdf = (hs_s^2 fc/df) 2^(2 (ka + kf)), hs_s the product of the
 //   mantissas.
 // A thread walks a run of redshifts at one frequency as in k_cells: half the loads and conversions of a
-// thread per element, the same sums.  91x81x101 edges, 40 frequencies: 627 us before, 483 us now;
+// thread per element, the same sums.  91x81x101 edges, 40 frequencies: 627 us before, 425 us now;
 // 181x161x201, 100 frequencies: 11.4 and 8.2 ms (issue bounds it, some 60% of it conversions and tests).
 struct StrainArgs32 {
     const float *g_val, *g_der;
