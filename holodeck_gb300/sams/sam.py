@@ -150,8 +150,9 @@ class Semi_Analytic_Model:
 
     def _scatter_finish(self, dens, gmt_time, redz_prime, pending=None):
         """Scatter and stalled-bin zeroing in place; caches the final density on the instance.  With a
-        list as ``pending`` the scatter's check is left to the caller (see add_scatter_to_masses_device);
-        one that raises drops the cached density."""
+        list as ``pending`` the scatter's check is left to the caller (see add_scatter_to_masses_device), and
+        the density is cached once that has passed: until then its kernels may be in flight, and another
+        thread that finds it would read it on a stream of its own."""
         scatter = self._mmbulge._scatter_dex
         checks = None if pending is None else []
         if scatter > 0.0:
@@ -159,15 +160,15 @@ class Semi_Analytic_Model:
             _scatter.add_scatter_to_masses_device(self.mtot, self.mrat, dens, scatter, pending=checks)
         if redz_prime is not None:
             N.call("hgb_zero_stalled", N.ptr(dens), N.ptr(redz_prime), int(dens.numel()), N.stream_handle())
-        self._density_t, self._gmt_time_t, self._redz_prime_t = dens, gmt_time, redz_prime
+
+        def keep():
+            self._gmt_time_t, self._redz_prime_t = gmt_time, redz_prime
+            self._density_t = dens   # the one that readers look for, last
+
         if checks:
-            def check():
-                try:
-                    _settle(checks)
-                except BaseException:
-                    self._density_t = self._gmt_time_t = self._redz_prime_t = None
-                    raise
-            pending.append(check)
+            pending.extend(checks + [keep])   # run in order: a check that raises keeps nothing
+        else:
+            keep()
         return dens
 
     @property
