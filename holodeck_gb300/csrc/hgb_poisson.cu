@@ -76,7 +76,7 @@ namespace {
 constexpr int RB = 128;                  // threads per block == bins per staged tile
 constexpr int NWARP = RB / 32;
 constexpr int RPT = 8;                   // realizations per thread, at most (see with_slots)
-constexpr int BULK_HELP_BLOCKS = 6;      // blocks per SM up to which a k_bulk block has helping threads
+constexpr int BULK_HELP_QUARTERS = 17;   // quarter blocks per SM up to which a k_bulk block has helping threads
 template <bool PARAMS, int NS>
 constexpr bool BULK_HELP = !PARAMS && NS < RPT;   // blocks may have RB more threads (see bulk_threads)
 constexpr int bulk_residency(bool params, int ns) {   // blocks per SM that registers are kept to
@@ -1749,14 +1749,16 @@ int n_rgroups(int nr) { return (int)hgb::ceil_div(nr, (long)RB * RPT); }
 
 // Threads of a k_bulk block.  On small grids the blocks of the lowest frequencies, with the longest
 // tables, run on after the others: RB more threads build tables and walk sparse runs with them.  Where
-// there are more blocks than an SM holds at once they only take their room (us without and with, 100
-// realizations: 30^3 bins with 20 frequencies, 3.5 blocks per SM, 630 and 557; 40x30x36 with 20, 5.7 per
-// SM, 673 and 623; 50x45x50 with 30, 20 per SM, 1186 and 1454).  Eight realizations a thread leave no
+// an SM has more blocks they take one another's room (us without and with at blocks per SM, of model grids:
+// 100 realizations, 30^3 edges with 20 frequencies 611 and 532 at 3.2, 26^3 with 40 632 and 562 at 4.2,
+// 34x32x34 with 20 624 and 609 at 4.3, 36x32x35 with 20 620 and 661 at 4.9, 60x50x55 with 5 607 and 766 at
+// 5.0, 50x45x50 with 30 1321 and 1622 at 20; 200 realizations, 24^3 with 40 854 and 784 at 3.2, 50x40x45
+// with 8 768 and 809 at 4.4).  Eight realizations a thread leave no
 // registers for them, nor do the parameter sums.
 template <int NS>
 unsigned bulk_threads(const dim3 &grid) {
     const long blocks = (long)grid.x * grid.y * grid.z;
-    return BULK_HELP<false, NS> && blocks <= (long)hgb::sm_count() * BULK_HELP_BLOCKS ? 2 * RB : RB;
+    return BULK_HELP<false, NS> && 4 * blocks <= (long)hgb::sm_count() * BULK_HELP_QUARTERS ? 2 * RB : RB;
 }
 
 // Launches with the fewest realizations per thread (1, 2, 4 or RPT) that hold all of them in one block:

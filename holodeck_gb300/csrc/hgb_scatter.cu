@@ -589,7 +589,8 @@ int hgb_add_scatter_to_masses(const hgb_scatter_plan *plan, double *dens, int n_
         const bool ahead = in_smem || n_redz <= hgb::sm_count();
         // Four lanes a point instead of two halve the chain of a phase and add some work: the faster form
         // while a phase leaves FP64 units idle (us with two and with four lanes: 30x30 points, 30 to a
-        // phase, 538 and 445; 50x45 878 and 822; 61x57 1111 and 1124; 91x81 1899 and 2032) and outside
+        // phase, 538 and 445; 50x45 878 and 822; 61x57 1111 and 1124; 91x81 1899 and 2032; the line lies between
+        // phases of 56 points, 1801 and 1721 on other values, and of 58, 1869 and 1885) and outside
         // shared memory, where loads make the chain (181x161 points, 152 slices: 9.3 and 8.6 ms), unless
         // two blocks fill the FP64 units, which the walk beside them needs (201 slices: 13.0 and 12.8,
         // but the whole call is 0.4% longer)
