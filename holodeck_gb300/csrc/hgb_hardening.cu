@@ -881,7 +881,7 @@ __global__ void __launch_bounds__(32 * EV_WARPS) k_dbn_2pwl_eval(CyConst cc, Dbn
     for (int i = threadIdx.x; i < NI; i += blockDim.x) {
         zg[i] = zgrid_g[i];
         ag[i] = agrid_g[i];
-        dg[i] = dgrid_g[i] * (1.0 / HGB_CY_MPC);
+        dg[i] = dgrid_g[i] * (1.0 / HGB_CY_MPC) * 0x1.0p-50;   // (exact; `unit` carries the square's 2^100)
     }
     for (int i = threadIdx.x; i < NF; i += blockDim.x) ft[i] = fobs[i];
     __syncthreads();
@@ -901,7 +901,9 @@ __global__ void __launch_bounds__(32 * EV_WARPS) k_dbn_2pwl_eval(CyConst cc, Dbn
     const double k13r = s_k13r, gw = s_g;
     const double pout = -a.go + a.gi, pin = 1.0 - a.gi;
     const PowPlan inner{a.p_inner.kind, a.p_inner.n, !a.p_inner.neg};
-    const double unit = cc.fourpi * (2.0 / 3.0) * a.rchar;
+    // 2^100: a density near the least double (a mass function's cutoff) keeps its bits through the residence
+    // time's factors, small in these units, until the distance takes the power out again
+    const double unit = cc.fourpi * (2.0 / 3.0) * a.rchar * 0x1.0p100;
     const int nzf = a.n_redz * NF;
     const long base = (long)cell * nzf;
 

@@ -58,3 +58,26 @@ def test_rows_without_ascending_times(built_lib, case):
     # as in test_gpu_walk_edges: times to a few ulp, and what a difference near z = 0 makes of them
     np.testing.assert_allclose(rf, want_rf, rtol=1e-10, atol=1e-13)
     np.testing.assert_allclose(dn, want_dn, rtol=1e-8, atol=0)
+
+
+@pytest.mark.parametrize("dens", [1e-290, 1e-303, 1e-308, 1e-312])
+def test_least_densities(built_lib, dens):
+    """A number is its density times a factor that does not depend on it, down to the subnormals."""
+    import types
+    import torch
+    from holodeck_gb300 import constants as C
+    from holodeck_gb300.sams import sam_cyutils
+    a = _inputs("plain")
+    dev = {k: torch.as_tensor(v, device="cuda") for k, v in a.items() if k != "init"}
+    hard = types.SimpleNamespace(_sepa_init=a["init"], _num_steps=STEPS, _rchar=100.0 * C.PC, _gamma_inner=-1.0,
+                                 _gamma_outer=2.5, _norm_device=lambda: dev["norm"])
+
+    def number(value):
+        nden = torch.full((NM, NQ, NZ), value, dtype=torch.float64, device="cuda")
+        return sam_cyutils.dbn_2pwl_device(dev["fobs"], hard, nden, dev["mtot"], dev["mrat"], dev["redz"],
+                                           dev["gmt"])[1].cpu().numpy()
+
+    one, got = number(1.0), number(dens)
+    assert (one > 0.0).sum() > 100
+    # the density times a factor of one and a half ulp, in two roundings, and a step of the subnormals
+    assert np.all(np.abs(got - dens * one) <= 8e-16 * (dens * one) + 1e-323)
